@@ -1,0 +1,95 @@
+"""Ragged lists and unaligned buffers through the stage kernels: entries of one
+list do not influence each other, whatever block they share, and the wide
+loads' fallbacks give the same bits as the wide loads (exact comparisons)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def frame(native):
+    import gpu_runner as R
+    from cases import Case
+    fr = R.Frame(Case(128, 96, seed=31, border_mode=1))
+    R.convert(fr)
+    return fr
+
+
+def _at_offset(tensors, floats):
+    """copies whose first element lies `floats` floats past a 256-byte boundary"""
+    import torch
+    out = []
+    for t in tensors:
+        x = torch.zeros(t.numel() + 64, dtype=t.dtype, device=t.device)
+        y = x[floats:floats + t.numel()]
+        y.copy_(t.reshape(-1))
+        out.append(y)
+    return out
+
+
+@pytest.mark.parametrize("colors", [1, 3])
+@pytest.mark.parametrize("count", [1, 2, 3, 4, 5, 9])
+def test_texture_entries_are_independent(frame, colors, count):
+    """A list of `count` entries, every third one invalid (no texture bit, or a
+    tile outside the frame), gives each entry what a list of it alone gives."""
+    import gpu_runner as R
+    c = frame.case
+    rng = np.random.default_rng(count)
+    tiles = rng.choice(c.TX * c.TY, count, replace=False)
+    idx = ((tiles << 8) | 0x8F).astype(np.int32)
+    idx[2::6] &= ~0x80
+    idx[5::6] = ((c.TX * c.TY + 3) << 8) | 0x8F
+    got = R.textures_tiles(frame, idx, keep_weights=1, colors=colors)
+    for i in range(count):
+        assert np.array_equal(got[i], R.textures_tiles(frame, idx[i:i + 1], keep_weights=1, colors=colors)[0]), i
+    assert np.all(got[2::6] == -7.0) and np.all(got[5::6] == -7.0)
+
+
+@pytest.mark.parametrize("colors", [1, 3])
+@pytest.mark.parametrize("floats", [1, 4])
+def test_textures_of_unaligned_clt(frame, colors, floats):
+    import gpu_runner as R
+    from tile_processor_gpu_b200 import api
+    c = frame.case
+    want = R.textures_tiles(frame, c.tex_idx, keep_weights=1, colors=colors)
+    moved, saved = _at_offset(frame.clt, floats), frame.p_clt
+    frame.p_clt = api.PointerArray(moved)
+    try:
+        got = R.textures_tiles(frame, c.tex_idx, keep_weights=1, colors=colors)
+    finally:
+        frame.p_clt = saved
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("impl", ["rgba", "process"])
+@pytest.mark.parametrize("rows,cols", [(1, 12), (12, 1), (3, 3)])
+def test_rgba_with_empty_parities(native, oracle, impl, rows, cols):
+    """Task lists that leave some of the four tile parities without a tile: the
+    image of the passes that have tiles is complete when the call's last
+    launch is, and equals the oracle's."""
+    import torch
+    import gpu_runner as R
+    from cases import Case, rel_err
+    from tile_processor_gpu_b200 import api
+    m = np.zeros((12, 16), dtype=bool)
+    m[4:4 + rows, 2:2 + cols] = True
+    c = Case(128, 96, seed=32, border_mode=1, mask=m)
+    fr = R.Frame(c)
+    clt = R.convert(fr)
+    if impl == "rgba":
+        out, woi, stride, used = R.rgba(fr)
+    else:
+        stride, used = (c.TX + 1) * 8 + 40, (c.TY + 1) * 8 * 4
+        rgba = torch.full((used + 8, stride), 3.0, device="cuda")
+        ints = [torch.zeros(n, dtype=torch.int32, device="cuda") for n in (c.TX * c.TYA + 256, 8, 4)]
+        corrs = torch.zeros((c.num_tiles * 6, 225), device="cuda")
+        api.process_frame(fr.g, fr.p_extra, fr.p_kernels, fr.p_images, c.dstride, fr.tasks, c.num_tiles, corrs, 225,
+                          fr.port_offsets, *ints, stride, rgba)
+        torch.cuda.synchronize()
+        out, woi = rgba.cpu().numpy(), ints[2].cpu().numpy()
+    want, _, _, _, woi_o = oracle.generate_RBGA(c.geom, c.tasks, c.TX, c.TY, [x.astype(np.float64) for x in clt],
+                                                c.port_offsets, stride, used)
+    assert np.array_equal(woi, woi_o)
+    h, w = (woi[3] + 1) * 8 * 4, (woi[2] + 1) * 8
+    assert rel_err(out[:h, :w], want[:h, :w]) < 1e-4

@@ -377,6 +377,29 @@ static int texture_params(int colors, float min_shot, float scale_shot, float di
     return TP_OK;
 }
 
+/* one launch of a texture kernel per 2^30 entries of the caller's list (the
+ * kernel counts entries in 32 bits) */
+extern "C++" {
+template <typename Kernel>
+static int launch_textures(Kernel kernel, const tp::Geom &gd, const int *woi, float *const *clt, size_t count,
+                           const int *indices, const float *port_offsets, const tp::TextureParams &p,
+                           size_t rbg_stride, float *rbg, size_t tile_stride, float *tiles, int sms,
+                           tp_stream_t stream)
+{
+    constexpr size_t kChunk = (size_t)1 << 30;
+    for (size_t n0 = 0; n0 < count; n0 += kChunk) {
+        const int n = (int)(count - n0 < kChunk ? count - n0 : kChunk);
+        const unsigned grid = grid_for(n, tp::tex_tiles(p.colors), sms, shape_per_sm(TP_SHAPE_TEXTURES));
+        kernel<<<grid, tp::kTexThreads, tp::kTexSmemBytes, (cudaStream_t)stream>>>(
+            gd, woi, clt, n, indices + n0, nullptr, 0, 0, 0, port_offsets, p, rbg_stride, rbg, tile_stride,
+            tiles ? tiles + n0 * tile_stride : nullptr);
+        const int rc = cuda_status(cudaGetLastError(), "textures_accumulate launch");
+        if (rc) return rc;
+    }
+    return TP_OK;
+}
+} /* extern "C++" */
+
 int tp_textures_accumulate(const tp_geometry *g, const int *woi, float *const *clt, size_t num_texture_tiles,
                            const int *texture_indices, const float *port_offsets, int colors, int is_lwir,
                            float min_shot, float scale_shot, float diff_sigma, float diff_threshold,
@@ -403,12 +426,9 @@ int tp_textures_accumulate(const tp_geometry *g, const int *woi, float *const *c
     int sms;
     if ((rc = sm_count(&sms))) return rc;
     if ((rc = texture_smem_setup())) return rc;
-    unsigned grid = grid_for((long long)num_texture_tiles, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES));
-    tex_kernel<false, true>(colors)<<<grid, tp::kTexThreads, tp::kTexSmemBytes, (cudaStream_t)stream>>>(
-        gd, woi, clt, (long long)num_texture_tiles, texture_indices, nullptr, 0, 0, 0, port_offsets, p,
-        want_rbg ? texture_rbg_stride : 0, want_rbg ? texture_rbg : nullptr, want_tiles ? texture_stride : 0,
-        want_tiles ? texture_tiles : nullptr);
-    return cuda_status(cudaGetLastError(), "textures_accumulate launch");
+    return launch_textures(tex_kernel<false, true>(colors), gd, woi, clt, num_texture_tiles, texture_indices,
+                           port_offsets, p, want_rbg ? texture_rbg_stride : 0, want_rbg ? texture_rbg : nullptr,
+                           want_tiles ? texture_stride : 0, want_tiles ? texture_tiles : nullptr, sms, stream);
 }
 
 int tp_imclt_rbg(const tp_geometry *g, const float *clt_one_cam, float *rbg, int color, int v_offset,
@@ -587,7 +607,7 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
         src = tile_scratch;
     }
     const int quarter = gd.TX * (gd.TYA >> 2);
-    const unsigned grid = grid_for(quarter, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES));
+    const unsigned grid = grid_for(quarter, tp::tex_tiles(colors), sms, shape_per_sm(TP_SHAPE_TEXTURES));
     /* one pass per tile parity: its inner sub-list, then its border one (the
      * reference runs the four inner passes, then the four border passes;
      * tiles of one parity never overlap, so a pass needs no ordering) */
@@ -595,7 +615,7 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
     for (int parity = 0; parity < 4; parity++) {
         const int *base = texture_indices + parity * quarter;
         const cudaError_t err =
-            launch_chained(true, grid, tp::kTexThreads, tp::kTexSmemBytes, s, tex, gd, (const int *)woi, src, 0LL,
+            launch_chained(true, grid, tp::kTexThreads, tp::kTexSmemBytes, s, tex, gd, (const int *)woi, src, 0,
                            (const int *)base, (const int *)num_texture_tiles, parity << 1, quarter, -quarter,
                            port_offsets, p, texture_rbga_stride, texture_tiles, (size_t)0, (float *)nullptr);
         if (err != cudaSuccess) return cuda_status(err, "generate_RBGA texture pass launch");
@@ -1238,12 +1258,9 @@ int tp_textures_accumulate_tc(const tp_geometry *g, const int *woi, float *const
     int sms;
     if ((rc = sm_count(&sms))) return rc;
     if ((rc = texture_smem_setup())) return rc;
-    unsigned grid = grid_for((long long)num_texture_tiles, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES));
-    tex_kernel<true, true>(colors)<<<grid, tp::kTexThreads, tp::kTexSmemBytes, (cudaStream_t)stream>>>(
-        gd, woi, tile_scratch, (long long)num_texture_tiles, texture_indices, nullptr, 0, 0, 0, port_offsets, p,
-        want_rbg ? texture_rbg_stride : 0, want_rbg ? texture_rbg : nullptr, want_tiles ? texture_stride : 0,
-        want_tiles ? texture_tiles : nullptr);
-    return cuda_status(cudaGetLastError(), "textures_accumulate_tc launch");
+    return launch_textures(tex_kernel<true, true>(colors), gd, woi, tile_scratch, num_texture_tiles, texture_indices,
+                           port_offsets, p, want_rbg ? texture_rbg_stride : 0, want_rbg ? texture_rbg : nullptr,
+                           want_tiles ? texture_stride : 0, want_tiles ? texture_tiles : nullptr, sms, stream);
 }
 
 int tp_generate_RBGA_tc(const tp_geometry *g, tp_task *tasks, int num_tiles, int *texture_indices,

@@ -153,6 +153,68 @@ __host__ __device__ __forceinline__ void dct2_fast(const float xin[8], float y[8
     for (int k = 0; k < 8; k++) y[k] = SINE ? r[7 - k] : r[k];
 }
 
+/* Two independent FP32 values in one 64-bit register pair (add/mul/fma.f32x2:
+ * one issue slot for two operations, each rounded as its scalar form).  The
+ * stage kernels are bound by issue slots, not by the FP32 units, so their
+ * transforms, stencils and camera fusion run on pairs. */
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tsub.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+#if !defined(__CUDA_ARCH__) || __CUDA_ARCH__ >= 1000
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+/* dct4_fast on both halves of pairs: y[2p] = Re Y_p, y[7-2p] = Im Y_p.  A
+ * DST-IV half takes its input in reverse order (x[7-n] at n) and leaves the
+ * sign of its odd outputs to the caller, who carries it in a later factor;
+ * one sequence then serves cosine and sine halves alike.  Bit-identical to
+ * dct4_fast. */
+__device__ __forceinline__ void dct4_pair(const float2 x[8], float2 y[8])
+{
+    constexpr float pre[4][2] = TP_DCT4_PRE_INIT;
+    constexpr float post[4][2] = TP_DCT4_POST_INIT;
+    float2 zr[4], zi[4];
+    zr[0] = x[0];
+#pragma unroll
+    for (int m = 1; m < 4; m++) {
+        const float2 a = x[2 * m], b = x[7 - 2 * m];
+        zr[m] = fma2(a, dup2(pre[m][0]), mul2(b, dup2(pre[m][1])));
+        zi[m] = fma2(a, dup2(pre[m][1]), mul2(b, dup2(-pre[m][0])));
+    }
+    const float2 b0 = x[7]; /* zi[0] = -b0 */
+    const float2 s02r = add2(zr[0], zr[2]), d02r = sub2(zr[0], zr[2]);
+    const float2 s02i = sub2(zi[2], b0), n02i = add2(b0, zi[2]); /* n02i = -d02i */
+    const float2 s13r = add2(zr[1], zr[3]), d13r = sub2(zr[1], zr[3]);
+    const float2 s13i = add2(zi[1], zi[3]), d13i = sub2(zi[1], zi[3]);
+    const float2 Zr[4] = {add2(s02r, s13r), sub2(d02r, d13i), sub2(s02r, s13r), add2(d02r, d13i)};
+    const float2 Zi[3] = {add2(s02i, s13i), sub2(d13r, n02i), sub2(s02i, s13i)};
+    const float2 n3 = add2(n02i, d13r); /* -Z_3's imaginary part */
+#pragma unroll
+    for (int p = 0; p < 3; p++) {
+        y[2 * p] = fma2(Zr[p], dup2(post[p][0]), mul2(Zi[p], dup2(-post[p][1])));
+        y[7 - 2 * p] = fma2(Zr[p], dup2(post[p][1]), mul2(Zi[p], dup2(post[p][0])));
+    }
+    y[6] = fma2(Zr[3], dup2(post[3][0]), mul2(n3, dup2(post[3][1])));
+    y[1] = fma2(Zr[3], dup2(post[3][1]), mul2(n3, dup2(-post[3][0])));
+}
+#endif
+
+/* 8 consecutive floats of global memory (32-byte aligned): one 256-bit access */
+__device__ __forceinline__ void ld8_global(const float *p, float v[8])
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
 /* y[k] = sum_n M[k][n] x[n] for the four 8-point transforms of the tables:
  * DCT-IV / DST-IV (KIND 0 / 1) through dct4_fast, DCT-II / DST-II (KIND 2 /
  * 3) through dct2_fast */

@@ -10,9 +10,12 @@
  * arithmetic is the same device code as the drop-in kernels, so the CLT and
  * the correlations are bit-identical to theirs.
  *
- * One 96-thread block (12 groups of 8 lanes) per tile, grid-stride over the
- * task list, seven blocks per SM (27.6 KB of shared memory each, the same
- * budget as the texture kernel):
+ * One 128-thread block (12 groups of 8 lanes with jobs; the fourth warp joins
+ * for the fusion) per tile, grid-stride over the task list, five blocks per SM
+ * at 96 registers and 27.6 KB of shared memory each.  More blocks leave less
+ * of the SM's memory as L1 for the Bayer and kernel-tile reads and spill
+ * (2592x1936 frame: five 2.60 ms, six 2.67, seven 2.69; 96-thread blocks at
+ * seven 2.73, at eight 3.07):
  *   1. forward CLT: group = (colour, camera) job, CLT into shared memory;
  *   2. correlations: groups 0-5, one camera pair each, from shared memory;
  *   3. texture: group = (camera, colour) job, inverse CLT into the
@@ -46,13 +49,13 @@ struct FrameParams {
     TextureParams tex; /* colors == 3, keep_weights == 0 */
 };
 
-constexpr int kFrameThreads = 96;
-constexpr int kFrameBlocksPerSm = 7;
+constexpr int kFrameThreads = 128;
+constexpr int kFrameBlocksPerSm = 5;
 /* dynamic shared memory of k_frame, in floats: per job its CLT, then T in
  * place (kJob floats); per group the transpose buffer, the correlation
  * buffers of groups 0-5 (kCorrBuf each) and then the debayered tile D */
-constexpr int kFrameSmemFloats = 12 * kJob + 12 * kTB4;
-static_assert(6 * kCorrBuf <= 12 * kTB4, "correlation buffers overlay the transpose buffers");
+constexpr int kFrameSmemFloats = 12 * kJob + 12 * kXb;
+static_assert(6 * kCorrBuf <= 12 * kXb, "correlation buffers overlay the transpose buffers");
 static_assert(kJob >= 256 && kJob % 4 == 0, "a job holds its 256 CLT floats, 16-byte aligned");
 constexpr size_t kFrameSmemBytes = sizeof(float) * kFrameSmemFloats;
 
@@ -65,20 +68,20 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
     extern __shared__ __align__(16) float smem[];
     float *s_clt = smem;            /* job CLT, job = camera * 3 + colour, then T */
     float *s_x = s_clt + 12 * kJob; /* transposes, correlation buffers, then D    */
-    __shared__ float s_pd2r[6], s_chw[3], s_chws[3];
+    __shared__ float s_npd2r[6], s_chw[3], s_chws[3];
 
     const int tid = threadIdx.x;
     const int l = tid & 7, grp = tid >> 3;
     const unsigned gm = group_mask();
-    /* 1 / (2 sigma^2) times log2(e), as combine_pixel takes it */
-    const float ksigma = (float)(1.0 / (2.0 * (double)p.tex.diff_sigma * (double)p.tex.diff_sigma)) * kLog2e;
+    /* -1 / (2 sigma^2) times log2(e), as combine_pair takes it */
+    const float nksigma = -((float)(1.0 / (2.0 * (double)p.tex.diff_sigma * (double)p.tex.diff_sigma)) * kLog2e);
     if (tid == 0) {
         int k = 0;
         for (int i = 0; i < 4; i++)
             for (int j = i + 1; j < 4; j++) {
                 const float dx = port_offsets[2 * j] - port_offsets[2 * i];
                 const float dy = port_offsets[2 * j + 1] - port_offsets[2 * i + 1];
-                s_pd2r[k++] = ksigma / (dx * dx + dy * dy);
+                s_npd2r[k++] = nksigma / (dx * dx + dy * dy);
             }
         s_chw[0] = p.tex.w0; s_chw[1] = p.tex.w1; s_chw[2] = p.tex.w2;
         /* D without the window and the shot scale (debayer_job<false>): the
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
      * transform, the offsets (and the kernel tile itself into L2) after the
      * correlations, the window's Bayer rows into L2 before the fusion. */
     __shared__ __align__(16) float s_pf[12][8];
-    const int color_c = grp >> 2, cam_c = grp & 3;
+    const int color_c = min(grp >> 2, 2), cam_c = grp & 3;
     int pf_n = -1; /* the tile whose inputs s_pf holds */
     const float step_inv = __int_as_float((127 - g.ls) << 23);
     auto kernel_tile = [&](float cx, float cy) -> size_t {
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
     };
     auto fetch_offsets = [&]() {
         pf_sync();
-        if (pf_n < 0) return;
+        if (pf_n < 0 || grp >= 12) return;
         const size_t kidx = kernel_tile(s_pf[grp][6], s_pf[grp][7]);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(kernels[cam_c] + kidx * 256 + l * 32));
         if (l < 6) cp_async4(&s_pf[grp][l], kernel_offsets[cam_c] + kidx * 8 + (l < 2 ? l : l + 2));
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
      * inside the image) */
     auto prefetch_window = [&]() {
         pf_sync();
-        if (pf_n < 0) return;
+        if (pf_n < 0 || grp >= 12) return;
         const float px = s_pf[grp][6] - 8.0f - s_pf[grp][0], py = s_pf[grp][7] - 8.0f - s_pf[grp][1];
         const int x0 = min(max(__float2int_rd(px + 0.5f), 0), g.W - 16);
         const int y0 = min(max(__float2int_rd(py + 0.5f), 0), g.H - 16);
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
         const int tx = txy & 0xffff, ty = txy >> 16;
 
         /* ---- 1. forward CLT: warp = colour, group = camera ---- */
-        {
+        if (grp < 12) {
             float cx, cy, ex[6];
             if (pf_n == n) {
                 cx = s_pf[grp][6]; cy = s_pf[grp][7];
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
                 ex[3] = __ldg(e + 5); ex[4] = __ldg(e + 6); ex[5] = __ldg(e + 7);
             }
             convert_job(g, dstride, kernel_offsets[cam_c], kernels[cam_c], images[cam_c], cx, cy, color_c, p.lpf_mask,
-                        s_clt + (cam_c * 3 + color_c) * kJob, reinterpret_cast<float(*)[9]>(s_x + grp * kTB4), l,
+                        s_clt + (cam_c * 3 + color_c) * kJob, reinterpret_cast<float(*)[9]>(s_x + grp * kXb), l,
                         gm, ex);
         }
         /* the block's next tile in this pass: lane i of every warp tests the
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
             pf_n = m ? n + __ffs(m) * (int)gridDim.x : -1;
             /* every lane of the group has read s_pf (before the transposes'
              * first __syncwarp in convert_job) */
-            if (pf_n >= 0 && l >= 6) cp_async4(&s_pf[grp][l], &tasks[pf_n].xy[cam_c][l - 6]);
+            if (grp < 12 && pf_n >= 0 && l >= 6) cp_async4(&s_pf[grp][l], &tasks[pf_n].xy[cam_c][l - 6]);
             cp_async_commit();
         }
         __syncthreads();
@@ -205,11 +208,14 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
         if (nbr) {
             __syncthreads(); /* the correlations have read the CLT and freed s_x */
             /* ---- 3. inverse CLT to T (in place), debayer to D: group = job ---- */
-            {
+            if (grp < 12) {
                 const int color = grp % 3;
-                float *cj = s_clt + grp * kJob, *xj = s_x + grp * kTB4;
-                imclt_unfold_job<false>(cj, d_lpf[color], xj, cj, l, gm);
-                debayer_job<false>(cj, xj, color < 2, p.tex.min_shot, p.tex.scale_shot, l, gm);
+                float *cj = s_clt + grp * kJob, *xj = s_x + grp * kXb;
+                float2 t[2][8];
+                float raw[4][8];
+                load_clt_rows<false>(cj, raw, l);
+                imclt_unfold_job<false>(raw, d_lpf[color], xj, cj, t, l, gm);
+                debayer_job<false>(t, cj, xj, color < 2, p.tex.min_shot, p.tex.scale_shot, l, gm);
             }
             __syncthreads();
             prefetch_window();
@@ -223,32 +229,41 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
             }
             const int gy0 = (ty - wy0) * 8, gx0 = (tx - wx0) * 8;
 #pragma unroll 1
-            for (int px = tid; px < 256; px += kFrameThreads) {
-                const int r = px >> 4, c = px & 15;
-                const float wnd2 = __ldg(&d_tex_wnd2[px]), wi = __ldg(&d_tex_wi[px]);
-                /* the pixel's RGBA values, loaded before the fusion covers their latency */
+            for (int e = tid; e < 128; e += kFrameThreads) {
+                const int r = (e >> 4) * 2, c = e & 15, px = r * 16 + c;
+                const float2 wnd2 = make_float2(__ldg(&d_tex_wnd2[px]), __ldg(&d_tex_wnd2[px + 16]));
+                /* the pixels' RGBA values, loaded before the fusion covers their latency */
                 const int gy = gy0 + r, gx = gx0 + c;
                 float *b = (gy < 0 || gx < 0) ? nullptr : rgba + (size_t)gy * rgba_stride + (size_t)gx;
-                float old[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                float2 old[4];
                 if (b) {
 #pragma unroll
-                    for (int sl = 0; sl < 4; sl++) old[sl] = b[(size_t)sl * slice_stride];
+                    for (int sl = 0; sl < 4; sl++)
+                        old[sl] = make_float2(__ldcg(b + (size_t)sl * slice_stride),
+                                              __ldcg(b + (size_t)sl * slice_stride + rgba_stride));
                 }
-                float o[12];
-                combine_pixel<3, false>(s_x, kTB4, s_clt, kJob, wnd2, JTS(kJS, r, c), s_pd2r, ksigma, s_chw, s_chws, wnd2,
-                                        wi, p.tex.dust_remove, 0, o);
+                float2 o[12];
+                combine_pair<3, false>(reinterpret_cast<const float2 *>(s_x), kXb / 2,
+                                       reinterpret_cast<const float2 *>(s_clt), kJob / 2, wnd2, e, s_npd2r, nksigma,
+                                       s_chw, s_chws, wnd2, wnd2, p.tex.dust_remove, 0, o);
                 if (!b) continue;
-                const float f = (nbr != TP_TASK_TEXTURE_BITS) ? __ldg(&d_alpha_fade[nbr][px]) : 1.0f;
+                float2 f = dup2(1.0f);
+                if (nbr != TP_TASK_TEXTURE_BITS)
+                    f = make_float2(__ldg(&d_alpha_fade[nbr][px]), __ldg(&d_alpha_fade[nbr][px + 16]));
 #pragma unroll
                 for (int sl = 0; sl < 4; sl++) {
-                    const float v = (nbr != TP_TASK_TEXTURE_BITS) ? o[sl] * f : o[sl];
-                    b[(size_t)sl * slice_stride] = old[sl] + v;
+                    const float2 v = add2(old[sl], mul2(o[sl], f));
+                    b[(size_t)sl * slice_stride] = v.x;
+                    b[(size_t)sl * slice_stride + rgba_stride] = v.y;
                 }
             }
         }
         if (!nbr) prefetch_window();
         __syncthreads(); /* the tile's buffers free for the next one */
     }
+    /* a block without a textured tile waits too: a grid has completed only
+     * once the launches before it have */
+    if (!waited) grid_dependency_wait();
 }
 
 } /* namespace tp */

@@ -4,25 +4,32 @@
  * :3847-4017, debayer_shot / debayer :4019-4199 and tile_combine_rgba
  * :4202-4665).
  *
- * One 96-thread block (three warps) per listed tile (grid-stride), seven
- * blocks per SM (at most 80 registers, 27 KB of shared memory each: the
- * tiles T and D only).  The CLT is read straight from global memory by the inverse
+ * One 128-thread block per listed tile (mono: per four tiles), grid-stride.  The CLT is read straight from global memory by the inverse
  * transform; the next tile's CLT and the RGBA rows it will update are
  * prefetched into L2 while the block works on the current tile.  Per
- * (camera, color) job one 8-lane group, working only with __syncwarp on its
+ * (camera, colour) job one 8-lane group, working only with __syncwarp on its
  * own buffers:
- *   1. low-pass filter and invert the CLT tile (vertical DCT-IV/DST-IV on the
- *      held column, transpose, horizontal pass on the held row) and unfold it
- *      into the un-windowed tile T (colour) or the windowed tile M (mono);
- *   2. debayer T with the 3x3 stencil (a register window walked down each
- *      column), apply the shot-noise square root and re-window into D (lane l
- *      owns columns l and l + 8).
- * After one block barrier every thread fuses the four cameras at its pixels
- * (stage 3; the plain windowed tile is T times the squared window) and
+ *   1. low-pass filter and invert the CLT tile (horizontal DCT-IV/DST-IV on
+ *      the held rows, transpose, vertical pass on the held column) and unfold
+ *      it into the un-windowed tile T (colour) or the windowed tile M (mono);
+ *   2. debayer T with the 3x3 stencil (walked down each column), apply the
+ *      shot-noise square root and re-window into D (a lane owns two columns).
+ * After one block barrier every thread fuses the four cameras at its pixel
+ * pairs (stage 3; the plain windowed tile is T times the squared window) and
  * writes them out itself (stage 4): as non-overlapping 16x16 tiles and/or
  * faded by the neighbour mask and added into the overlapped RGBA image.
- * Per-job buffers are 280 floats apart (280 % 32 == 24) so the four groups
- * of a warp never share a bank.
+ *
+ * The kernel is bound by issue slots and by the latency of each tile's chain of
+ * steps (DRAM 16-27%), so all of it runs on packed pairs of FP32 values
+ * (add2 / mul2 / fma2): two quadrants per pair in the transforms, two rows of
+ * a column per pair from the unfold on.  The RGBA-only colour form takes 4776
+ * warp instructions a tile (7238 in scalar form); the four passes of a
+ * 2592x1936 frame with their list and clear went from 0.787 to 0.614 ms.
+ * Seven blocks of four warps share an SM; three-warp blocks (no idle warp
+ * in the transforms, but two turns of the fusion for one warp) took 0.671.  Tiles in shared memory hold pairs of
+ * rows: pair (rp, c) = rows 2 rp and 2 rp + 1 of column c at float2 16 rp + c,
+ * so a warp of the fusion reads two row pairs of 16 columns in 64-bit loads
+ * without a bank conflict and its RGBA accesses stay whole 64-byte rows.
  */
 #pragma once
 #include "tp_common.cuh"
@@ -37,19 +44,15 @@ struct TextureParams {
     int dust_remove, keep_weights;
 };
 
-constexpr int kJob = 280; /* floats per job tile (16 rows of at most 17), padded */
-/* Pixel (r, c) of a job tile with row stride S.  The camera fusion reads 32
- * consecutive pixels (two rows) per warp: at stride 16 they fall on 32
- * distinct banks, at 17 the second row's last pixel shares the first row's
- * first bank.  The column-wise passes (unfold, debayer: one column per lane,
- * the four groups' tiles 280 floats apart) are conflict-free at either
- * stride.  Tiles copied in row by row (one row per lane, the tensor-core
- * inverse's output) keep stride 17, where those stores spread over the
- * banks. */
-#define JTS(S, r, c) ((r) * (S) + (c))
-constexpr int kJS = 16; /* row stride of tiles the inverse transform writes */
-
-__device__ __forceinline__ int sym8(int i) { return (i & 8) ? (i ^ 15) : i; }
+/* floats per job tile (16 x 16), padded: 272 % 32 == 16 puts the two groups of
+ * a half-warp, whose 64-bit accesses cover 64 bytes each, on distinct banks */
+constexpr int kJob = 272;
+/* floats per group of transpose buffer: 8 rows of 9 quadruples, one per
+ * quadrant (16-byte accesses along rows and columns are conflict-free);
+ * 304 % 32 == 16 where job tiles overlay it */
+constexpr int kXb = 304;
+/* float2 index of the pair (rows 2 rp, 2 rp + 1) of column c in a job tile */
+#define JT2(rp, c) ((rp) * 16 + (c))
 
 /* Per-pixel factors of the unfold, [16][17]:
  *   tfac[r][c] = (0.25 / w[c]) / w[r]     un-windowed tile T = d * tfac
@@ -64,80 +67,131 @@ __device__ float d_tex_mfac[kFac] = TP_TEX_MFAC_INIT;
 __device__ float d_tex_wnd2[256] = TP_TEX_WND2_INIT;
 __device__ float d_tex_wi[256] = TP_TEX_WI_INIT;
 
-/* Windowed inverse CLT of one job (imclt8threads, :3847-4017) into the
- * [16][kJS] tile M = w * d (w the product of the two half-sine windows, no
- * accumulation), and, for the debayer, the same tile with the squared window
- * removed, T = M / (sin^2 r sin^2 c) = d / (4 sin r sin c), formed directly
- * from the signed sum d.  Lane l loads coefficient row l of each quadrant (two
- * 16-byte loads per row where the source allows); per quadrant it applies
- * the low-pass filter, runs
- * the horizontal DCT-IV/DST-IV on it, and after a transpose the vertical one
- * on column l: it ends holding pixel-domain column l of all four quadrants.
- * The unfold (fold column RIND[c] = l for exactly two output columns c) then
- * writes those two columns whole, the quadrant signs of idct_signs
- * (:399-420) factored into a horizontal sign pair per column (per lane) and
- * a vertical sign per row (compile-time); the window factors are a per-lane
- * column factor, carried by the horizontal sign pair, times a compile-time
- * row factor.  MONO: M (mono) instead of T (colour).  The first column a lane
- * writes is 11 - l: with job buffers 280 floats apart the four groups of a
- * warp then store to 32 distinct banks in both columns.  src: the job's
- * 4x64 coefficients (row stride 8), shared or global memory; tb: the
- * group's transpose buffer; out: the job's [16][kJS] output tile. */
-template <bool MONO>
-__device__ __forceinline__ void imclt_unfold_job(const float *src, const float *lpf, float *tb, float *out, int l,
-                                                 unsigned gm)
+/* 8 consecutive floats of a CLT tile: one 256-bit load from global memory
+ * where the tile allows it, else 16-byte or scalar loads (GLOBAL false:
+ * shared memory) */
+template <bool GLOBAL>
+__device__ __forceinline__ void load_clt_row(const float *p, float v[8])
 {
-    constexpr float kHwin[16] = TP_HWIN_INIT;
-    float a[4][8]; /* pixel-domain column l of each quadrant */
-    float f[8];    /* row l of the low-pass filter, shared by the quadrants */
-    if (lpf)
+    if (GLOBAL && !(reinterpret_cast<uintptr_t>(p) & 31))
+        ld8_global(p, v);
+    else
+        load_row8(p, !(reinterpret_cast<uintptr_t>(p) & 15), v);
+}
+
+/* Lane l's rows of a job's CLT tile: row l of quadrants 0 and 1, row 7 - l of 2
+ * and 3 (see imclt_pairs) */
+template <bool GLOBAL>
+__device__ __forceinline__ void load_clt_rows(const float *src, float raw[4][8], int l)
+{
+#pragma unroll
+    for (int q = 0; q < 4; q++) load_clt_row<GLOBAL>(src + q * 64 + (q < 2 ? l : 7 - l) * 8, raw[q]);
+}
+
+/* The four quadrants of one CLT tile to the pixel domain on an 8-lane group
+ * (imclt8threads, :3847-4017).  Lane l holds coefficient row l of quadrants 0
+ * and 1 and row 7 - l of 2 and 3 (load_clt_rows), times the low-pass filter
+ * (NULL: none); the horizontal pass runs on the pairs (q0, q2) (DCT-IV) and
+ * (q1, q3) (DST-IV), one 16-byte transpose per coefficient moves both pairs,
+ * and the vertical pass runs on the same pairs, whose second halves (DST-IV)
+ * arrive in the reverse row order the sine transform wants.  Lane l ends with
+ * pixel-domain column l, a02[u] = (q0, q2), a13[u] = (q1, q3), except for the
+ * signs dct4_pair leaves out: a02[u].y and a13[u].y are negated for odd u, and
+ * a13 is negated as a whole for odd l. */
+__device__ __forceinline__ void imclt_pairs(const float raw[4][8], const float *lpf, float4 *tb, float2 a02[8],
+                                            float2 a13[8], int l, unsigned gm)
+{
+    float2 x[8], y02[8], y13[8];
+    float f[8], g[8]; /* rows l and 7 - l of the low-pass filter */
+    if (lpf) {
         load_row8(lpf + l * 8, true, f);
-    const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
-    /* all four rows in flight before the first transform needs one */
-    float raw[4][8];
+        load_row8(lpf + (7 - l) * 8, true, g);
+    } else {
 #pragma unroll
-    for (int q = 0; q < 4; q++) load_row8(src + q * 64 + l * 8, al16, raw[q]);
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        float row[8], v[8], col[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) row[k] = raw[q][k];
-        if (lpf) {
-#pragma unroll
-            for (int k = 0; k < 8; k++) row[k] *= f[k];
-        }
-        if (q & 1) dtt8<1>(row, v); else dtt8<0>(row, v);
-#pragma unroll
-        for (int k = 0; k < 8; k++) tb[TBI(q, l, k)] = v[k];
-        __syncwarp(gm);
-#pragma unroll
-        for (int k = 0; k < 8; k++) col[k] = tb[TBI(q, k, l)];
-        if (q >> 1) dtt8<1>(col, a[q]); else dtt8<0>(col, a[q]);
+        for (int k = 0; k < 8; k++) f[k] = g[k] = 1.0f;
     }
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        /* the output column and its quarter (columns 0-3: (+,+); 4-11:
-         * (-,+); 12-15: (-,-) on the (even, odd) quadrant of each pair) */
-        const int c = h ? ((l < 4) ? l + 12 : l - 4) : 11 - l;
-        const int cq = c >> 2;
-        const float wc = __ldg(&d_hwin[c]);
-        /* the column's window factor: 0.5 w[c] (M) or 0.25 / w[c] (T) */
-        const float cf = MONO ? 0.5f * wc : 0.25f / wc;
-        const float s0 = (cq == 0) ? cf : -cf, s1 = (cq == 3) ? -cf : cf;
-        float e0[8], e1[8];
+    for (int k = 0; k < 8; k++) x[k] = make_float2(raw[0][k] * f[k], raw[2][k] * g[k]);
+    dct4_pair(x, y02);
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            e0[u] = __fmaf_rn(s0, a[0][u], s1 * a[1][u]);
-            e1[u] = __fmaf_rn(s0, a[2][u], s1 * a[3][u]);
-        }
+    for (int k = 0; k < 8; k++) x[k] = make_float2(raw[1][7 - k] * f[7 - k], raw[3][7 - k] * g[7 - k]);
+    dct4_pair(x, y13);
 #pragma unroll
-        for (int r = 0; r < 16; r++) {
+    for (int k = 0; k < 8; k++) tb[l * 9 + k] = make_float4(y02[k].x, y02[k].y, y13[k].x, y13[k].y);
+    __syncwarp(gm);
+    float2 z[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        const float4 t = tb[r * 9 + l];
+        x[r] = make_float2(t.x, t.y);
+        z[r] = make_float2(t.z, t.w);
+    }
+    dct4_pair(x, a02);
+    dct4_pair(z, a13);
+}
+
+/* output column h (0, 1) of a lane: the two window columns that fold onto l */
+__device__ __forceinline__ int unfold_col(int l, int h) { return h ? ((l < 4) ? l + 12 : l - 4) : 11 - l; }
+
+/* Unfold of output column c of lane l into row pairs t[8], from the pairs of
+ * imclt_pairs: the quadrant signs of idct_signs (:399-420) are a sign pair
+ * per column (columns 0-3: (+,+); 4-11: (-,+); 12-15: (-,-) on the (even,
+ * odd) quadrants) and compile-time signs per row; cf, the column's window
+ * factor, rides on the column's signs, as do the signs imclt_pairs left out;
+ * kr[r] is the row's factor. */
+__device__ __forceinline__ void unfold_column(const float2 a02[8], const float2 a13[8], int l, int c, float cf,
+                                              const float (&kr)[16], float2 t[8])
+{
+    const int cq = c >> 2;
+    const float s0 = (cq == 0) ? cf : -cf, s1 = ((cq == 3) != ((l & 1) != 0)) ? -cf : cf;
+    const float2 s0e = dup2(s0), s0o = make_float2(s0, -s0), s1e = dup2(s1), s1o = make_float2(s1, -s1);
+    float2 e[8]; /* the even and odd vertical quadrants' sums */
+#pragma unroll
+    for (int u = 0; u < 8; u++) e[u] = fma2((u & 1) ? s0o : s0e, a02[u], mul2((u & 1) ? s1o : s1e, a13[u]));
+#pragma unroll
+    for (int rp = 0; rp < 8; rp++) {
+        float d[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int r = 2 * rp + i, rq = r >> 2;
             const int u = (r < 4) ? r + 4 : (r < 12) ? 11 - r : r - 12;
-            const int rq = r >> 2;
             /* vertical signs: rows 0-3 (+,+); 4-11 (-,+); 12-15 (-,-) */
-            const float d = ((rq != 0) ? -e0[u] : e0[u]) + ((rq == 3) ? -e1[u] : e1[u]);
-            out[JTS(kJS, r, c)] = d * (MONO ? 0.5f * kHwin[r] : 1.0f / kHwin[r]);
+            d[i] = ((rq != 0) ? -e[u].x : e[u].x) + ((rq == 3) ? -e[u].y : e[u].y);
         }
+        t[rp] = mul2(make_float2(d[0], d[1]), make_float2(kr[2 * rp], kr[2 * rp + 1]));
+    }
+}
+
+/* Inverse CLT of one job (raw: load_clt_rows), unfolded into the job tile `out` (row pairs): the
+ * un-windowed tile T = d / (4 sin r sin c) (the windowed one with the squared
+ * window removed, formed directly from the signed sum d) or, MONO, the
+ * windowed M = (w_r / 2) (w_c / 2) d.  t: the lane's two columns, for the
+ * debayer.  out may be the memory of tb, or the one raw was loaded from. */
+template <bool MONO>
+__device__ __forceinline__ void imclt_unfold_job(const float raw[4][8], const float *lpf, float *tb, float *out,
+                                                 float2 t[2][8], int l, unsigned gm)
+{
+    constexpr float kHwin[16] = TP_HWIN_INIT;
+    constexpr float kRow[16] = {
+        MONO ? 0.5f * kHwin[0] : 1.0f / kHwin[0],   MONO ? 0.5f * kHwin[1] : 1.0f / kHwin[1],
+        MONO ? 0.5f * kHwin[2] : 1.0f / kHwin[2],   MONO ? 0.5f * kHwin[3] : 1.0f / kHwin[3],
+        MONO ? 0.5f * kHwin[4] : 1.0f / kHwin[4],   MONO ? 0.5f * kHwin[5] : 1.0f / kHwin[5],
+        MONO ? 0.5f * kHwin[6] : 1.0f / kHwin[6],   MONO ? 0.5f * kHwin[7] : 1.0f / kHwin[7],
+        MONO ? 0.5f * kHwin[8] : 1.0f / kHwin[8],   MONO ? 0.5f * kHwin[9] : 1.0f / kHwin[9],
+        MONO ? 0.5f * kHwin[10] : 1.0f / kHwin[10], MONO ? 0.5f * kHwin[11] : 1.0f / kHwin[11],
+        MONO ? 0.5f * kHwin[12] : 1.0f / kHwin[12], MONO ? 0.5f * kHwin[13] : 1.0f / kHwin[13],
+        MONO ? 0.5f * kHwin[14] : 1.0f / kHwin[14], MONO ? 0.5f * kHwin[15] : 1.0f / kHwin[15]};
+    float2 a02[8], a13[8]; /* pixel-domain column l of the quadrants */
+    imclt_pairs(raw, lpf, reinterpret_cast<float4 *>(tb), a02, a13, l, gm);
+    __syncwarp(gm);
+    float2 *o2 = reinterpret_cast<float2 *>(out);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int c = unfold_col(l, h);
+        const float wc = __ldg(&d_hwin[c]);
+        unfold_column(a02, a13, l, c, MONO ? 0.5f * wc : 0.25f / wc, kRow, t[h]);
+#pragma unroll
+        for (int rp = 0; rp < 8; rp++) o2[JT2(rp, c)] = t[h][rp];
     }
 }
 
@@ -161,60 +215,62 @@ __device__ __forceinline__ float rcp_hw(float x)
 
 /* 3x3 debayer of the un-windowed tile T (interior 14x14; border copied),
  * shot-noise square root, squared window re-applied: T -> D
- * (debayer_shot / debayer, :4019-4199).  Lane l: columns l and l + 8, each
- * walked down with a 3x3 register window.  The stencil's horizontal pair
- * t[r][c-1] + t[r][c+1] is summed once per row and shared by the three rows
- * that use it; red/blue (rb_mode) and green take one branch-free form (the
- * diagonal term's weight is 0 for green), so the groups of a warp, which
- * hold different colours, do not diverge; the border columns (copied
- * unchanged) take the same form with stencil weights 0, 0 and 1.  The
- * shot-noise scale and the two window factors are one product per pixel.
- * WINDOWED = false stores D without them (the camera fusion of the RGBA-only
- * path measures distances in D wi sqrt(w) scale_shot, where the squared
- * window cancels against wi = 1 / wnd2: it takes scale_shot with its colour
- * factors instead).  SHOT: scale_shot > 0, the shot-noise step applies.
- * S: the tiles' row stride. */
-template <bool WINDOWED, bool SHOT, int S>
-__device__ __forceinline__ void debayer_tile(const float *t, float *d, int rb_mode, float min_shot,
-                                             float scale_shot, int l, unsigned gm)
+ * (debayer_shot / debayer, :4019-4199).  Lane l owns the two columns it
+ * unfolded (in t), as row pairs; the neighbouring columns come from the job
+ * tile.  The stencil's horizontal sum t[r][c-1] + t[r][c+1] is formed once
+ * per row and shared by the three rows that use it; red/blue (rb_mode) and
+ * green take one branch-free form (the diagonal term's weight is 0 for
+ * green), so the groups of a warp, which hold different colours, do not
+ * diverge; the border columns (copied unchanged) take the same form with
+ * stencil weights 0, 0 and 1.
+ * WINDOWED = false stores D without the shot scale and the window factors
+ * (the camera fusion of the RGBA-only path measures distances in D wi sqrt(w)
+ * scale_shot, where the squared window cancels against wi = 1 / wnd2: it
+ * takes scale_shot with its colour factors instead).  SHOT: scale_shot > 0,
+ * the shot-noise step applies. */
+template <bool WINDOWED, bool SHOT>
+__device__ __forceinline__ void debayer_tile(const float2 t[2][8], const float *tile, float *d, int rb_mode,
+                                             float min_shot, float scale_shot, int l, unsigned gm)
 {
-    /* the window as compile-time constants (the values of c_hwin): the
-     * squared window of an unrolled row folds into an immediate operand */
+    /* the window as compile-time constants (the values of c_hwin) */
     constexpr float kHwin[16] = TP_HWIN_INIT;
+    const float2 *t2 = reinterpret_cast<const float2 *>(tile);
+    float2 *d2 = reinterpret_cast<float2 *>(d);
     __syncwarp(gm);
     const float kdiag = rb_mode ? 0.0625f : 0.0f, kcenter = rb_mode ? 0.25f : 0.5f;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const int c = l + 8 * h;
-        const bool cborder = (c == 0) || (c == 15);
+        const int c = unfold_col(l, h);
+        const bool cborder = h && ((c == 0) || (c == 15)); /* columns 4..11 for h = 0 */
         const int cm = cborder ? c : c - 1, cp = cborder ? c : c + 1;
         /* per-lane stencil weights: diagonal, orthogonal, centre */
-        const float kd = cborder ? 0.0f : kdiag, ko = cborder ? 0.0f : 0.125f, kc = cborder ? 1.0f : kcenter;
+        const float2 kd = dup2(cborder ? 0.0f : kdiag), ko = dup2(cborder ? 0.0f : 0.125f);
+        const float2 kc = dup2(cborder ? 1.0f : kcenter);
         const float hcc = __ldg(&d_hwin[c]);
         const float swx = (SHOT ? scale_shot : 1.0f) * (hcc * hcc);
-        float a1 = t[JTS(S, 0, c)], ha = t[JTS(S, 0, cm)] + t[JTS(S, 0, cp)];
-        float b1 = t[JTS(S, 1, c)], hb = t[JTS(S, 1, cm)] + t[JTS(S, 1, cp)];
+        float2 hp = make_float2(0.0f, 0.0f), hs = add2(t2[JT2(0, cm)], t2[JT2(0, cp)]);
 #pragma unroll
-        for (int r = 0; r < 16; r++) {
-            float v;
-            if (r == 0) {
-                v = a1;
-            } else if (r == 15) {
-                v = b1;
-            } else {
-                const float e1 = t[JTS(S, r + 1, c)], he = t[JTS(S, r + 1, cm)] + t[JTS(S, r + 1, cp)];
-                const float orth = (a1 + e1) + hb;
-                const float diag = ha + he;
-                v = __fmaf_rn(kd, diag, __fmaf_rn(ko, orth, kc * b1));
-                a1 = b1; ha = hb;
-                b1 = e1; hb = he;
-            }
+        for (int rp = 0; rp < 8; rp++) {
+            float2 hn = make_float2(0.0f, 0.0f);
+            if (rp < 7) hn = add2(t2[JT2(rp + 1, cm)], t2[JT2(rp + 1, cp)]);
+            const float up = rp > 0 ? t[h][rp - 1].y : 0.0f, dn = rp < 7 ? t[h][rp + 1].x : 0.0f;
+            const float2 me = t[h][rp];
+            const float2 orth = add2(make_float2(up + me.y, me.x + dn), hs);
+            const float2 diag = make_float2(hp.y + hs.y, hs.x + hn.x);
+            float2 v = fma2(kd, diag, fma2(ko, orth, mul2(kc, me)));
+            if (rp == 0) v.x = me.x;
+            if (rp == 7) v.y = me.y;
+            hp = hs;
+            hs = hn;
             /* shot-noise square root above min_shot, v / sqrt(min_shot) at or
              * below it: both are v * rsqrt(max(v, min_shot)) (min_shot is a
              * normal float > 0 whenever the transform applies), from the
              * hardware reciprocal square root (within 3e-7 of sqrtf) */
-            if (SHOT) v = v * rsqrt_hw(fmaxf(v, min_shot));
-            d[JTS(S, r, c)] = WINDOWED ? v * (swx * (kHwin[r] * kHwin[r])) : v;
+            if (SHOT) v = mul2(v, make_float2(rsqrt_hw(fmaxf(v.x, min_shot)), rsqrt_hw(fmaxf(v.y, min_shot))));
+            if (WINDOWED)
+                v = mul2(v, mul2(dup2(swx), make_float2(kHwin[2 * rp] * kHwin[2 * rp],
+                                                        kHwin[2 * rp + 1] * kHwin[2 * rp + 1])));
+            d2[JT2(rp, c)] = v;
         }
     }
     __syncwarp(gm);
@@ -222,14 +278,14 @@ __device__ __forceinline__ void debayer_tile(const float *t, float *d, int rb_mo
 
 /* debayer_tile with the shot-noise step compiled in (scale_shot > 0) or out:
  * one switch per job, outside the unrolled stencil */
-template <bool WINDOWED, int S = kJS>
-__device__ __forceinline__ void debayer_job(const float *t, float *d, int rb_mode, float min_shot,
-                                            float scale_shot, int l, unsigned gm)
+template <bool WINDOWED>
+__device__ __forceinline__ void debayer_job(const float2 t[2][8], const float *tile, float *d, int rb_mode,
+                                            float min_shot, float scale_shot, int l, unsigned gm)
 {
     if (scale_shot > 0.0f)
-        debayer_tile<WINDOWED, true, S>(t, d, rb_mode, min_shot, scale_shot, l, gm);
+        debayer_tile<WINDOWED, true>(t, tile, d, rb_mode, min_shot, scale_shot, l, gm);
     else
-        debayer_tile<WINDOWED, false, S>(t, d, rb_mode, min_shot, scale_shot, l, gm);
+        debayer_tile<WINDOWED, false>(t, tile, d, rb_mode, min_shot, scale_shot, l, gm);
 }
 
 /* log2(e): e^x = 2^(x log2 e) */
@@ -244,55 +300,70 @@ __device__ __forceinline__ float exp2_hw(float x)
     return y;
 }
 
-/* Fuse the four cameras at one pixel (tile_combine_rgba, one pixel).
+/* a >= b as 1.0 / 0.0, on both halves of pairs */
+__device__ __forceinline__ float2 ge2(float2 a, float2 b)
+{
+    float2 r;
+    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r.x) : "f"(a.x), "f"(b.x));
+    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r.y) : "f"(a.y), "f"(b.y));
+    return r;
+}
+
+/* exp2 plus the 1e-4 weight floor, added in double and rounded once to float
+ * (see combine_pair) */
+__device__ __forceinline__ float weight_hw(float x) { return __double2float_rn((double)exp2_hw(x) + 1e-4); }
+
+/* Fuse the four cameras at a pair of pixels, rows 2 rp and 2 rp + 1 of one
+ * column (tile_combine_rgba, two pixels).
  * sd: debayered tiles D; sm: the plain (not debayered) tiles, scaled by
  * m_scale (the plain tile is the un-windowed one times the squared window);
- * both [job = cam * colors + color] with the given strides, pixel offset e.
+ * both [job = cam * colors + color] with the given strides in float2, pair
+ * index e.
  * chw: the colour weights; chws: their square roots, times scale_shot when
  * the D tiles come without the window and the shot scale (D_WINDOWED false;
- * wi is then not applied to them).  pd2r (the six pairs'
- * 1 / (2 sigma^2 |offset|^2)) and ksigma (1 / (2 sigma^2)) come multiplied by
- * log2(e): each weight exp(-k d) is evaluated as 2^(-(k log2 e) d).
+ * wi is then not applied to them).  npd2r (the six pairs'
+ * -1 / (2 sigma^2 |offset|^2)) and nksigma (-1 / (2 sigma^2)) come multiplied
+ * by log2(e): each weight exp(-k d) is evaluated as 2^(-(k log2 e) d).
  * o: colours, alpha, 4 port weights and (keep_weights) colors + 1 rms.
  * The colour distances sum_col chw[col] ((X[col] - Y[col]) wi)^2 are formed
  * as sum_col (X'[col] - Y'[col])^2 in the scaled space X' = X wi sqrt(chw),
  * the same quantity with fewer operations per camera pair. */
 template <int COLORS, bool D_WINDOWED = true>
-__device__ __forceinline__ void combine_pixel(const float *sd, int sd_stride, const float *sm, int sm_stride,
-                                              float m_scale, int e, const float *pd2r, float ksigma,
-                                              const float *chw, const float *chws, float wnd2, float wi,
-                                              int dust_remove, int keep_weights, float *o)
+__device__ __forceinline__ void combine_pair(const float2 *sd, int sd_stride, const float2 *sm, int sm_stride,
+                                             float2 m_scale, int e, const float *npd2r, float nksigma,
+                                             const float *chw, const float *chws, float2 wnd2, float2 wi,
+                                             int dust_remove, int keep_weights, float2 *o)
 {
-    float D[4][COLORS];
+    float2 D[4][COLORS];
 #pragma unroll
     for (int cam = 0; cam < 4; cam++)
 #pragma unroll
         for (int col = 0; col < COLORS; col++) D[cam][col] = sd[(cam * COLORS + col) * sd_stride + e];
     if (keep_weights) {
-        float sw = 0.0f;
+        float2 sw = make_float2(0.0f, 0.0f);
 #pragma unroll
         for (int col = 0; col < COLORS; col++) {
             /* variance of the four cameras, two-pass (the one-pass form of
              * the reference loses digits where the cameras agree) */
-            const float mean = ((D[0][col] + D[1][col]) + (D[2][col] + D[3][col])) * 0.25f;
-            float ss = 0.0f;
+            const float2 mean = mul2(add2(add2(D[0][col], D[1][col]), add2(D[2][col], D[3][col])), dup2(0.25f));
+            float2 ss = make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int cam = 0; cam < 4; cam++) {
-                const float dv = D[cam][col] - mean;
-                ss = __fmaf_rn(dv, dv, ss);
+                const float2 dv = sub2(D[cam][col], mean);
+                ss = fma2(dv, dv, ss);
             }
-            const float mse = ss * 0.25f;
-            o[COLORS + 5 + col] = sqrtf(mse);
-            sw = __fmaf_rn(chw[col], mse, sw);
+            const float2 mse = mul2(ss, dup2(0.25f));
+            o[COLORS + 5 + col] = make_float2(sqrtf(mse.x), sqrtf(mse.y));
+            sw = fma2(dup2(chw[col]), mse, sw);
         }
-        o[COLORS + 5 + COLORS] = sqrtf(sw);
+        o[COLORS + 5 + COLORS] = make_float2(sqrtf(sw.x), sqrtf(sw.y));
     }
     /* D in the scaled space */
 #pragma unroll
     for (int col = 0; col < COLORS; col++) {
-        const float sc = D_WINDOWED ? wi * chws[col] : chws[col];
+        const float2 sc = D_WINDOWED ? mul2(wi, dup2(chws[col])) : dup2(chws[col]);
 #pragma unroll
-        for (int cam = 0; cam < 4; cam++) D[cam][col] *= sc;
+        for (int cam = 0; cam < 4; cam++) D[cam][col] = mul2(D[cam][col], sc);
     }
     /* wi = 1 / wnd2 correctly rounded (the reference forms it in double).
      * A weight is exp(...) plus the 1e-4 floor added in double and rounded
@@ -302,105 +373,125 @@ __device__ __forceinline__ void combine_pixel(const float *sd, int sd_stride, co
      * with 1e-4f can land one ulp lower and break such ties the other way
      * (splitting the floor into two floats still rounds 1 in 2e6 tiny sums
      * differently).  The exponential is the hardware's base-2 one with the
-     * log2(e) factor folded into pd2r and ksigma: its relative error (about
+     * log2(e) factor folded into npd2r and nksigma: its relative error (about
      * 2^-22) is under what float32 inputs already move a weight by, and a
      * flushed subnormal weight is lost in the 1e-4 floor. */
-    float pw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float2 pw[4];
     {
         int k = 0;
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
             for (int j = i + 1; j < 4; j++) {
-                float d = 0.0f;
+                float2 d;
 #pragma unroll
                 for (int col = 0; col < COLORS; col++) {
-                    const float dc = D[i][col] - D[j][col];
-                    d = __fmaf_rn(dc, dc, d);
+                    const float2 dc = sub2(D[i][col], D[j][col]);
+                    d = col ? fma2(dc, dc, d) : mul2(dc, dc);
                 }
-                const float x = __double2float_rn((double)exp2_hw(-pd2r[k] * d) + 1e-4);
-                pw[i] += x;
-                pw[j] += x;
+                d = mul2(d, dup2(npd2r[k]));
+                const float2 x = make_float2(weight_hw(d.x), weight_hw(d.y));
+                pw[i] = (i == 0 && j == 1) ? x : add2(pw[i], x);
+                pw[j] = (i == 0) ? x : add2(pw[j], x);
                 k++;
             }
     }
-    /* the best two cameras (first of equals), their weights carried beside
-     * the indices: an array indexed by a run-time camera would live in local
-     * memory */
-    int b1 = 0;
-    float p1 = pw[0];
+    /* the average of the best two cameras (first of equals) in proportion to
+     * their weights.  Camera i beats a later camera j when w_i >= w_j; the two
+     * best are those that beat at least two of the others, whichever of them
+     * is first.  Six comparisons as 1.0 / 0.0 and a saturated sum of each
+     * camera's wins (1 where there are two or three) choose them without a
+     * branch or a select */
+    {
+        const float2 c01 = ge2(pw[0], pw[1]), c02 = ge2(pw[0], pw[2]), c03 = ge2(pw[0], pw[3]);
+        const float2 c12 = ge2(pw[1], pw[2]), c13 = ge2(pw[1], pw[3]), c23 = ge2(pw[2], pw[3]);
+        const float2 one = dup2(1.0f);
+        /* wins - 1: camera 1 loses c01, 2 loses c02 and c12, 3 loses c03, c13 and c23 */
+        const float2 n0 = sub2(add2(c01, c02), one), n1 = sub2(c12, c01), n2 = sub2(sub2(one, c02), c12);
+        const float2 n3 = sub2(sub2(dup2(2.0f), c03), c13);
+        pw[0] = mul2(pw[0], make_float2(__saturatef(n0.x + c03.x), __saturatef(n0.y + c03.y)));
+        pw[1] = mul2(pw[1], make_float2(__saturatef(n1.x + c13.x), __saturatef(n1.y + c13.y)));
+        pw[2] = mul2(pw[2], make_float2(__saturatef(n2.x + c23.x), __saturatef(n2.y + c23.y)));
+        pw[3] = mul2(pw[3], make_float2(__saturatef(n3.x - c23.x), __saturatef(n3.y - c23.y)));
+    }
+    const float2 best = add2(add2(pw[0], pw[1]), add2(pw[2], pw[3])); /* two of the four are 0 */
+    const float2 binv = make_float2(rcp_hw(best.x), rcp_hw(best.y));
+    float2 avg[COLORS];
 #pragma unroll
-    for (int cam = 1; cam < 4; cam++)
-        if (pw[cam] > p1) { b1 = cam; p1 = pw[cam]; }
-    int b2 = (b1 == 0) ? 1 : 0;
-    float p2 = (b1 == 0) ? pw[1] : pw[0];
+    for (int cam = 0; cam < 4; cam++) {
+        const float2 sh = mul2(pw[cam], binv);
 #pragma unroll
-    for (int cam = 1; cam < 4; cam++)
-        if (cam > b2 && cam != b1 && pw[cam] > p2) { b2 = cam; p2 = pw[cam]; }
-    const float w1 = __fdividef(p1, p1 + p2);
-    const float w2 = 1.0f - w1;
-    float avg[COLORS];
-#pragma unroll
-    for (int col = 0; col < COLORS; col++) {
-        float a = 0.0f, b = 0.0f;
-#pragma unroll
-        for (int cam = 0; cam < 4; cam++) {
-            if (cam == b1) a = D[cam][col];
-            if (cam == b2) b = D[cam][col];
-        }
-        avg[col] = w1 * a + w2 * b;
+        for (int col = 0; col < COLORS; col++)
+            avg[col] = cam ? fma2(sh, D[cam][col], avg[col]) : mul2(sh, D[cam][col]);
     }
 #pragma unroll
     for (int cam = 0; cam < 4; cam++) {
-        float d2 = 0.0f;
+        float2 d;
 #pragma unroll
         for (int col = 0; col < COLORS; col++) {
-            const float dc = D[cam][col] - avg[col];
-            d2 = __fmaf_rn(dc, dc, d2);
+            const float2 dc = sub2(D[cam][col], avg[col]);
+            d = col ? fma2(dc, dc, d) : mul2(dc, dc);
         }
-        pw[cam] = __double2float_rn((double)exp2_hw(-ksigma * d2) + 1e-4);
+        d = mul2(d, dup2(nksigma));
+        pw[cam] = make_float2(weight_hw(d.x), weight_hw(d.y));
     }
     if (dust_remove) {
-        int worst = 0;
-        float wv = pw[0];
+        const float2 wv = make_float2(fminf(fminf(pw[0].x, pw[1].x), fminf(pw[2].x, pw[3].x)),
+                                      fminf(fminf(pw[0].y, pw[1].y), fminf(pw[2].y, pw[3].y)));
+        float2 a = sub2(pw[0], wv);
 #pragma unroll
-        for (int cam = 1; cam < 4; cam++)
-            if (pw[cam] < wv) { worst = cam; wv = pw[cam]; }
-        float a = -wv;
+        for (int cam = 1; cam < 4; cam++) a = add2(a, pw[cam]);
+        a = mul2(a, dup2(1.0f / 3.0f));
+        const float2 ra = make_float2(rcp_hw(a.x), rcp_hw(a.y));
+        const float2 scale =
+            fma2(mul2(mul2(wv, sub2(a, wv)), mul2(ra, ra)), dup2(1.0f / 3.0f), dup2(1.0f));
+        const float2 fw = mul2(wv, ra);
+        /* the worst camera (first of equals) */
+        bool fx = true, fy = true;
 #pragma unroll
-        for (int cam = 0; cam < 4; cam++) a += pw[cam];
-        a *= (1.0f / 3.0f);
-        const float ra = rcp_hw(a);
-        const float scale = 1.0f + (wv * (a - wv)) * (ra * ra) * (1.0f / 3.0f);
-        const float fw = wv * ra;
-#pragma unroll
-        for (int cam = 0; cam < 4; cam++) pw[cam] *= (cam == worst) ? fw : scale;
+        for (int cam = 0; cam < 4; cam++) {
+            const bool ex = fx && pw[cam].x == wv.x, ey = fy && pw[cam].y == wv.y;
+            pw[cam] = mul2(pw[cam], make_float2(ex ? fw.x : scale.x, ey ? fw.y : scale.y));
+            fx = fx && !ex;
+            fy = fy && !ey;
+        }
     }
-    float ksum = 0.0f;
+    float2 ksum = pw[0];
 #pragma unroll
-    for (int cam = 0; cam < 4; cam++) ksum += pw[cam];
-    const float kinv = rcp_hw(ksum);
-    float kw[4];
+    for (int cam = 1; cam < 4; cam++) ksum = add2(ksum, pw[cam]);
+    const float2 kinv = make_float2(rcp_hw(ksum.x), rcp_hw(ksum.y));
+    float2 kw[4];
 #pragma unroll
-    for (int cam = 0; cam < 4; cam++) kw[cam] = kinv * pw[cam];
+    for (int cam = 0; cam < 4; cam++) kw[cam] = mul2(kinv, pw[cam]);
 #pragma unroll
     for (int col = 0; col < COLORS; col++) {
-        float v = 0.0f;
+        float2 v;
 #pragma unroll
-        for (int cam = 0; cam < 4; cam++) v = __fmaf_rn(kw[cam], sm[(cam * COLORS + col) * sm_stride + e], v);
-        o[col] = v * m_scale;
+        for (int cam = 0; cam < 4; cam++) {
+            const float2 m = sm[(cam * COLORS + col) * sm_stride + e];
+            v = cam ? fma2(kw[cam], m, v) : mul2(kw[cam], m);
+        }
+        o[col] = mul2(v, m_scale);
     }
-    o[COLORS] = wnd2 * ksum / 4.0f;
+    o[COLORS] = mul2(mul2(wnd2, ksum), dup2(0.25f));
 #pragma unroll
     for (int cam = 0; cam < 4; cam++) o[COLORS + 1 + cam] = pw[cam];
 }
 
-/* k_textures block: three warps, one 8-lane group per (camera, colour) job */
-constexpr int kTexThreads = 96;
-/* dynamic shared memory of k_textures, in floats: T (un-windowed tiles),
- * transposes then D (debayered tiles) */
-constexpr int kTexSmemFloats = 12 * kJob + 12 * kTB4;
-constexpr size_t kTexSmemBytes = sizeof(float) * kTexSmemFloats;
+/* k_textures block: four warps, so that the fusion of a tile's 128 pixel pairs
+ * takes each of them one turn; one 8-lane group per (camera, colour) job of
+ * the block's tiles (colour: one tile of 12 jobs on three warps, the fourth
+ * prefetches; mono: four tiles of four jobs) */
+constexpr int kTexThreads = 128;
+__host__ __device__ constexpr int tex_tiles(int colors) { return colors == 1 ? kTexThreads / 32 : 1; }
+/* dynamic shared memory of k_textures: per job its un-windowed tile T, then its
+ * debayered tile D (mono: the windowed tile M alone); the transposes of the
+ * inverse run over both.  26.3 KB a block: seven blocks, 28 warps, share an SM */
+__host__ __device__ constexpr int tex_job(int colors) { return colors == 1 ? kXb : 560; } /* floats; % 32 == 16 as kJob */
+constexpr int kTexD = kJob; /* D's offset in a job */
+static_assert(kTexD + 256 <= tex_job(3) && 8 * 9 * 4 <= tex_job(1), "a job's tiles and its transposes");
+constexpr size_t kTexSmemBytes = sizeof(float) * 12 * tex_job(3);
+static_assert(sizeof(float) * 16 * tex_job(1) <= kTexSmemBytes, "mono fits the same block");
 
 /* FROM_T: `clt` holds the jobs' pixel tiles instead of their CLT, as
  * k_tc_stage<InvTcStage> writes them (the un-windowed T for colour, the
@@ -411,29 +502,26 @@ constexpr size_t kTexSmemBytes = sizeof(float) * kTexSmemFloats;
  * a compile-time count lets each form keep only its own colour path). */
 template <bool FROM_T, bool ALL, int COLORS>
 __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
-    Geom g, const int *__restrict__ woi, float *const *clt, long long num_texture_tiles,
+    Geom g, const int *__restrict__ woi, float *const *clt, int num_texture_tiles,
     const int *__restrict__ list, const int *__restrict__ dev_counts, int count_slot, int list_cap,
     int border_quarter, const float *__restrict__ port_offsets, TextureParams p,
     size_t texture_rbg_stride, float *__restrict__ texture_rbg, size_t texture_stride,
     float *__restrict__ texture_tiles)
 {
     extern __shared__ __align__(16) float smem[];
-    float *s_t = smem;                 /* un-windowed tiles T (colour) or windowed M (mono) */
-    float *s_x = s_t + 12 * kJob;      /* transposes, then the debayered tiles D            */
     __shared__ float *s_cp[4];
-    __shared__ float s_pd2r[6], s_chw[3], s_chws[3];
+    __shared__ float s_npd2r[6], s_chw[3], s_chws[3];
 
     const int tid = threadIdx.x;
     const int l = tid & 7, grp = tid >> 3;
     const unsigned gm = group_mask();
     static_assert(COLORS == 1 || COLORS == 3, "colour count");
-    constexpr int colors = COLORS;
-    /* row stride of the T and D tiles: 17 where stage 1 copies T in row by
-     * row (FROM_T), else that of the inverse transform's output */
-    constexpr int kS = FROM_T ? 17 : kJS;
-    const int njobs = 4 * colors;
-    /* 1 / (2 sigma^2) times log2(e): the fusion's weights are powers of two */
-    const float ksigma = (float)(1.0 / (2.0 * (double)p.diff_sigma * (double)p.diff_sigma)) * kLog2e;
+    constexpr int colors = COLORS, kTiles = tex_tiles(COLORS), kJobs = 4 * COLORS, kTexJob = tex_job(COLORS);
+    /* this group's job: tile `sub` of the block's (kTiles: none), camera, colour */
+    const int sub = grp / kJobs, job = grp - sub * kJobs;
+    const int cam = job / colors, color = job - cam * colors;
+    /* -1 / (2 sigma^2) times log2(e): the fusion's weights are powers of two */
+    const float nksigma = -((float)(1.0 / (2.0 * (double)p.diff_sigma * (double)p.diff_sigma)) * kLog2e);
     if (tid < 4) s_cp[tid] = clt[tid];
     if (tid == 0) {
         int k = 0;
@@ -441,7 +529,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             for (int j = i + 1; j < 4; j++) {
                 const float dx = port_offsets[2 * j] - port_offsets[2 * i];
                 const float dy = port_offsets[2 * j + 1] - port_offsets[2 * i + 1];
-                s_pd2r[k++] = ksigma / (dx * dx + dy * dy);
+                s_npd2r[k++] = nksigma / (dx * dx + dy * dy);
             }
         s_chw[0] = p.w0; s_chw[1] = p.w1; s_chw[2] = p.w2;
         /* the RGBA-only colour path debayers without the window (see
@@ -453,7 +541,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * for mono (the keep-weights statistics and mono need them as the
      * reference forms them); the RGBA-only colour form debayers without them */
 
-    long long count = num_texture_tiles;
+    int count = num_texture_tiles;
     const int *lst = list;
     /* entries at or past `split` sit `gap` further on in the list */
     int split = 0x7fffffff, gap = 0;
@@ -468,7 +556,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             /* inner (count_slot) then border (count_slot + 1) sub-lists of one
              * quarter of -border_quarter entries in one pass: tiles of one
              * parity never overlap, so their RGBA updates need no ordering */
-            const int q = -border_quarter, ci = (int)count;
+            const int q = -border_quarter, ci = count;
             int cb = dev_counts[count_slot + 1];
             cb = cb < 0 ? 0 : (cb > q - ci ? q - ci : cb);
             split = ci;
@@ -476,8 +564,6 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             count += cb;
         }
     }
-    /* list entry n of this pass */
-    auto code_at = [&](long long n) -> int { return lst[n + (n >= split ? gap : 0)]; };
     const bool want_rbg = texture_rbg && texture_rbg_stride;
     const bool want_tiles = ALL && texture_tiles && texture_stride;
     const int keep_weights = ALL ? p.keep_weights : 0;
@@ -487,161 +573,213 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
     const size_t slice_stride = texture_rbg_stride * (size_t)(wh + 1) * 8;
     __syncthreads();
     const int ntiles = g.TX * g.TY;
-    /* list entry -> tile index, or -1 when the entry is not a texture tile */
-    auto tile_of = [&](long long n) -> int {
-        if (n >= count) return -1;
-        const int code = code_at(n);
-        const int tile = code >> 8;
-        return ((code & (1 << 7)) && tile >= 0 && tile < ntiles) ? tile : -1;
+    /* entry n of this pass: its code, or 0 when there is none or it is not a
+     * texture tile */
+    auto entry = [&](int n) -> int {
+        if (n >= count) return 0;
+        const int code = lst[n + (n >= split ? gap : 0)], tile = code >> 8;
+        return ((code & (1 << 7)) && tile >= 0 && tile < ntiles) ? code : 0;
     };
-    /* window position of a tile's top-left pixel (once per tile) */
+    /* window position of a tile's top-left pixel.  The row comes from a float
+     * quotient (tiles < 2^24 are exact, the quotient within one of the row)
+     * and one correction either way. */
+    const float tx_inv = 1.0f / (float)g.TX;
     auto rgba_origin = [&](int tile, int *gy0, int *gx0) {
-        const int ty = tile / g.TX, tx = tile - ty * g.TX;
+        int ty = (int)((float)tile * tx_inv), tx = tile - ty * g.TX;
+        if (tx < 0) { ty--; tx += g.TX; }
+        if (tx >= g.TX) { ty++; tx -= g.TX; }
         *gy0 = (ty - wy0) * 8;
         *gx0 = (tx - wx0) * 8;
     };
-    /* RGBA address of pixel px (slice 0) of the tile at (gy0, gx0), or NULL
-     * when it lies left of / above the window */
-    auto rgba_at = [&](int gy0, int gx0, int px) -> float * {
-        const int gy = gy0 + (px >> 4), gx = gx0 + (px & 15);
+    /* RGBA address of pixel (r, c) (slice 0) of the tile at (gy0, gx0), or
+     * NULL when it lies left of / above the window (gy0 and gx0 are multiples
+     * of 8, so both rows of a pair lie on the same side) */
+    auto rgba_at = [&](int gy0, int gx0, int r, int c) -> float * {
+        const int gy = gy0 + r, gx = gx0 + c;
         if (gy < 0 || gx < 0) return nullptr;
         return texture_rbg + (size_t)gy * texture_rbg_stride + (size_t)gx;
     };
-    /* The next tile's inputs are prefetched into L2 while the block works on
-     * the current one: its CLT (one 128-byte line per thread: 24 lines of 768
-     * floats per camera) and the RGBA rows its pixels update (both ends of
-     * each 16-pixel row of each slice).  The RGBA prefetch comes after the
-     * wait for the previous pass, which writes those rows. */
-    auto prefetch_clt = [&](int tile) {
-        const int cam = tid / 24, line = tid - cam * 24;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(s_cp[cam] + (size_t)tile * 768 + line * 32));
+    /* The next tiles' inputs are prefetched into L2 while the block works on
+     * the current ones: their CLT (one 128-byte line per thread: 24 lines of
+     * 768 floats per camera, mono 8 lines of 256) and, after the fusion, the
+     * RGBA rows their pixels update (both ends of each 16-pixel row of each
+     * slice; the previous pass, which writes them, has completed by then). */
+    constexpr int kLines = colors == 3 ? 24 : 8;
+    auto prefetch_clt = [&](const int *codes) {
+        const int t = colors == 3 ? 0 : tid >> 5, k = colors == 3 ? tid : tid & 31;
+        if (k >= 4 * kLines) return;
+        int code = 0;
+#pragma unroll
+        for (int i = 0; i < kTiles; i++)
+            if (t == i) code = codes[i];
+        if (!code) return;
+        const int pcam = k / kLines, line = k - pcam * kLines;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(s_cp[pcam] + (size_t)(code >> 8) * 768 + line * 32));
     };
-    auto prefetch_rgba = [&](long long n) {
-        if (!want_rbg || n >= count) return;
-        const int code = code_at(n);
-        const int tile = code >> 8;
-        if (!(code & (1 << 7)) || tile < 0 || tile >= ntiles || !(code & TP_TASK_TEXTURE_BITS)) return;
-        int gy0, gx0;
-        rgba_origin(tile, &gy0, &gx0);
-        const int r = tid & 15, sl = tid >> 4; /* row r of slice sl */
-        if (sl <= colors) {
-            const float *b = rgba_at(gy0, gx0, r * 16);
-            if (b) {
-                b += (size_t)sl * slice_stride;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(b));
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(b + 15));
-            }
+    auto prefetch_rgba = [&](int code, int gy0, int gx0) {
+        /* row r of slice sl */
+        const int r = tid & 15, sl = colors == 3 ? tid >> 4 : (tid >> 4) & 1;
+        if (!want_rbg || !(code & TP_TASK_TEXTURE_BITS) || sl > colors) return;
+        const float *b = rgba_at(gy0, gx0, r, 0);
+        if (b) {
+            b += (size_t)sl * slice_stride;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(b));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(b + 15));
         }
+    };
+    /* this group's entry of a block's codes (0: none) */
+    auto pick = [&](const int *codes) -> int {
+        int code = 0;
+#pragma unroll
+        for (int i = 0; i < kTiles; i++)
+            if (sub == i) code = codes[i];
+        return code;
+    };
+    auto job_clt = [&](int code) -> const float * {
+        return s_cp[cam] + ((size_t)(code >> 8) * 3 + color) * 256;
     };
 
     /* the next tile-parity pass may be scheduled on the SM slots this grid
      * frees as its blocks finish */
     grid_dependents_launch();
-    {
-        const long long n0 = blockIdx.x;
-        const int t0 = tile_of(n0);
-        if (t0 >= 0) prefetch_clt(t0);
-        /* A pass launched as a programmatic dependent of the launch before it
-         * (the RGBA clear, or the previous tile-parity pass) waits here for
-         * it: that launch writes the RGBA image.  Everything read above (the
-         * list and its counts, the window, the CLT, the port offsets) was
-         * complete before that launch let this one start. */
-        grid_dependency_wait();
-        if (t0 >= 0) prefetch_rgba(n0);
-    }
-
-    for (long long n = blockIdx.x; n < count; n += gridDim.x) {
-        const int code = code_at(n);
-        const int tile = tile_of(n);
-        const long long n_next = n + gridDim.x;
-        __syncthreads(); /* the previous tile's buffers free */
-        if (tile < 0) {
-            const int tn = tile_of(n_next);
-            if (tn >= 0) {
-                prefetch_clt(tn);
-                prefetch_rgba(n_next);
-            }
-            continue;
-        }
-
-        /* ---- stages 1-2: per (camera, color) group ---- */
-        if (grp < njobs && FROM_T) {
-            const int cam = grp / colors, color = grp - cam * colors;
-            float *tj = s_t + grp * kJob, *xj = s_x + grp * kTB4;
-            const float *src = s_cp[cam] + ((size_t)tile * 3 + color) * 256 + l * 32;
-            const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
-            /* lane l: rows 2 l and 2 l + 1 */
+    /* A pass launched as a programmatic dependent of the launch before it (the
+     * RGBA clear, or the previous tile-parity pass) waits for it before its
+     * first access to the RGBA image, which that launch writes; the inverse
+     * transform and debayer of its first tiles run before that wait.
+     * Everything they read (the list and its counts, the window, the CLT, the
+     * port offsets) was complete before that launch let this one start. */
+    bool waited = false;
+    int codes[kTiles], gy0 = 0, gx0 = 0;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[16];
-                load_row8(src + 16 * h, al16, v);
-                load_row8(src + 16 * h + 8, al16, v + 8);
+    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x * kTiles + i);
+    int mine = pick(codes);
+    if (colors == 3 && want_rbg) rgba_origin(codes[0] >> 8, &gy0, &gx0);
+
+    for (int n = (int)blockIdx.x * kTiles; n < count; n += (int)gridDim.x * kTiles) {
+        int next[kTiles];
 #pragma unroll
-                for (int c = 0; c < 16; c++) tj[JTS(kS, 2 * l + h, c)] = v[c];
-            }
-            if (colors > 1) debayer_job<ALL, kS>(tj, xj, color < 2, p.min_shot, p.scale_shot, l, gm);
-        } else if (grp < njobs) {
-            const int cam = grp / colors, color = grp - cam * colors;
-            float *tj = s_t + grp * kJob, *xj = s_x + grp * kTB4;
-            if (colors > 1) {
-                /* T -> s_t, then the debayered D -> s_x (the transpose
-                 * buffer, free once the unfold has read it) */
-                imclt_unfold_job<false>(s_cp[cam] + ((size_t)tile * 3 + color) * 256, d_lpf[color], xj, tj, l, gm);
-                debayer_job<ALL>(tj, xj, color < 2, p.min_shot, p.scale_shot, l, gm);
+        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * kTiles + i);
+
+        /* ---- stages 1-2: per (tile, camera, color) group ---- */
+        if (mine) {
+            /* T (mono: M), then D; the transposes use the whole job */
+            float *tj = smem + grp * kTexJob, *dj = tj + kTexD;
+            float2 t[2][8];
+            if (FROM_T) {
+                /* lane l: rows 2 l and 2 l + 1, one row pair */
+                const float *src = job_clt(mine);
+                const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
+                float2 *t2 = reinterpret_cast<float2 *>(tj);
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+                    float v[8], w[8];
+                    load_row8(src + l * 32 + half * 8, al16, v);
+                    load_row8(src + l * 32 + 16 + half * 8, al16, w);
+#pragma unroll
+                    for (int c = 0; c < 8; c++) t2[JT2(l, half * 8 + c)] = make_float2(v[c], w[c]);
+                }
+                if (colors > 1) {
+                    __syncwarp(gm);
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int rp = 0; rp < 8; rp++) t[h][rp] = t2[JT2(rp, unfold_col(l, h))];
+                }
             } else {
-                imclt_unfold_job<true>(s_cp[cam] + ((size_t)tile * 3 + color) * 256, d_lpf[3], xj, tj, l, gm);
+                float raw[4][8];
+                load_clt_rows<true>(job_clt(mine), raw, l);
+                imclt_unfold_job<COLORS == 1>(raw, d_lpf[colors > 1 ? color : 3], tj, tj, t, l, gm);
             }
+            if (colors > 1) debayer_job<ALL>(t, tj, dj, color < 2, p.min_shot, p.scale_shot, l, gm);
         }
         __syncthreads();
-        {
-            const int tn = tile_of(n_next);
-            if (tn >= 0) prefetch_clt(tn);
+        prefetch_clt(next);
+        if (!waited) {
+            grid_dependency_wait();
+            waited = true;
         }
 
-        /* ---- stages 3-4: fuse the four cameras at the thread's pixels and
-         * write them out ---- */
-        const int nbr = code & TP_TASK_TEXTURE_BITS;
-        int gy0 = 0, gx0 = 0;
-        if (want_rbg && nbr) rgba_origin(tile, &gy0, &gx0);
+        /* ---- stages 3-4: fuse the four cameras at the thread's pixel pairs
+         * and write them out ---- */
 #pragma unroll 1
-        for (int px = tid; px < 256; px += kTexThreads) {
-            const int r = px >> 4, c = px & 15;
-            const int e = JTS(kS, r, c);
-            const float wnd2 = __ldg(&d_tex_wnd2[px]), wi = __ldg(&d_tex_wi[px]);
-            /* the pixel's RGBA values are loaded before the fusion, whose
+        for (int i = tid; i < 128 * kTiles; i += kTexThreads) {
+            const int k = kTiles > 1 ? i >> 7 : 0; /* uniform in a warp */
+            int code = codes[0];
+#pragma unroll
+            for (int j = 1; j < kTiles; j++)
+                if (k == j) code = codes[j];
+            if (!code) continue;
+            const int e = i & 127, r = (e >> 4) * 2, c = e & 15;
+            const int px = r * 16 + c;
+            const int nbr = code & TP_TASK_TEXTURE_BITS;
+            const float2 wnd2 = make_float2(__ldg(&d_tex_wnd2[px]), __ldg(&d_tex_wnd2[px + 16]));
+            float2 wi = wnd2;
+            if (ALL || colors == 1) wi = make_float2(__ldg(&d_tex_wi[px]), __ldg(&d_tex_wi[px + 16]));
+            /* the pixels' RGBA values are loaded before the fusion, whose
              * arithmetic then covers their latency */
-            float old[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            float *b = (want_rbg && nbr) ? rgba_at(gy0, gx0, px) : nullptr;
+            float2 old[4];
+            float *b = nullptr;
+            if (want_rbg && nbr) {
+                if (colors == 1) rgba_origin(code >> 8, &gy0, &gx0);
+                b = rgba_at(gy0, gx0, r, c);
+            }
             if (b) {
 #pragma unroll
-                for (int sl = 0; sl < 4; sl++)
-                    if (sl <= colors) old[sl] = b[(size_t)sl * slice_stride];
+                for (int sl = 0; sl <= colors; sl++)
+                    old[sl] = make_float2(__ldcg(b + (size_t)sl * slice_stride),
+                                          __ldcg(b + (size_t)sl * slice_stride + texture_rbg_stride));
             }
-            float o[12];
+            float2 o[12];
+            const float2 *t2 = reinterpret_cast<const float2 *>(smem + k * kJobs * kTexJob);
             if (colors == 3)
-                combine_pixel<3, ALL>(s_x, kTB4, s_t, kJob, wnd2, e, s_pd2r, ksigma, s_chw, s_chws, wnd2, wi,
-                                      p.dust_remove, keep_weights, o);
+                combine_pair<3, ALL>(t2 + kTexD / 2, kTexJob / 2, t2, kTexJob / 2, wnd2, e, s_npd2r, nksigma, s_chw,
+                                     s_chws, wnd2, wi, p.dust_remove, keep_weights, o);
             else
-                combine_pixel<1>(s_t, kJob, s_t, kJob, 1.0f, e, s_pd2r, ksigma, s_chw, s_chws, wnd2, wi,
-                                 p.dust_remove, keep_weights, o);
+                combine_pair<1>(t2, kTexJob / 2, t2, kTexJob / 2, dup2(1.0f), e, s_npd2r, nksigma, s_chw, s_chws,
+                                wnd2, wi, p.dust_remove, keep_weights, o);
             if (want_tiles) {
-                float *dst = texture_tiles + (size_t)n * texture_stride + px;
+                float *dst = texture_tiles + (size_t)(n + k) * texture_stride + px;
 #pragma unroll
                 for (int sl = 0; sl < 12; sl++)
-                    if (sl < ns_tiles) dst[sl * 256] = o[sl];
+                    if (sl < ns_tiles) {
+                        dst[sl * 256] = o[sl].x;
+                        dst[sl * 256 + 16] = o[sl].y;
+                    }
             }
             if (b) {
-                const float f = (nbr != TP_TASK_TEXTURE_BITS) ? __ldg(&d_alpha_fade[nbr][px]) : 1.0f;
+                float2 f = dup2(1.0f);
+                if (nbr != TP_TASK_TEXTURE_BITS)
+                    f = make_float2(__ldg(&d_alpha_fade[nbr][px]), __ldg(&d_alpha_fade[nbr][px + 16]));
 #pragma unroll
-                for (int sl = 0; sl < 4; sl++) {
-                    if (sl > colors) break;
-                    const float v = (nbr != TP_TASK_TEXTURE_BITS) ? o[sl] * f : o[sl];
-                    b[(size_t)sl * slice_stride] = old[sl] + v;
+                for (int sl = 0; sl <= colors; sl++) {
+                    const float2 v = add2(old[sl], mul2(o[sl], f));
+                    b[(size_t)sl * slice_stride] = v.x;
+                    b[(size_t)sl * slice_stride + texture_rbg_stride] = v.y;
                 }
             }
         }
-        prefetch_rgba(n_next);
+#pragma unroll
+        for (int i = 0; i < kTiles; i++) codes[i] = next[i];
+        mine = pick(codes);
+        if (want_rbg) {
+            if (colors == 3) {
+                rgba_origin(codes[0] >> 8, &gy0, &gx0);
+                prefetch_rgba(codes[0], gy0, gx0);
+            } else {
+                int code = 0;
+#pragma unroll
+                for (int i = 0; i < kTiles; i++)
+                    if ((tid >> 5) == i) code = codes[i];
+                int y, x;
+                rgba_origin(code >> 8, &y, &x);
+                prefetch_rgba(code, y, x);
+            }
+        }
+        __syncthreads(); /* the tiles' buffers free */
     }
+    /* a block without a tile waits too: a grid has completed only once the
+     * launches before it have */
+    if (!waited) grid_dependency_wait();
 }
 
 } /* namespace tp */
