@@ -93,3 +93,38 @@ def test_rgba_with_empty_parities(native, oracle, impl, rows, cols):
     assert np.array_equal(woi, woi_o)
     h, w = (woi[3] + 1) * 8 * 4, (woi[2] + 1) * 8
     assert rel_err(out[:h, :w], want[:h, :w]) < 1e-4
+
+
+@pytest.mark.parametrize("count", [1, 3, 4, 5, 739, 741, 768])
+@pytest.mark.parametrize("floats", [0, 1, 4])
+def test_convert_counts_and_alignment(native, oracle, count, floats):
+    """Task counts on both sides of the one-colour / three-colour item rule, not
+    multiples of the four tasks of an item among them, with the kernel tables,
+    images and the CLT on and off 32-byte boundaries: the same bits as the
+    one-colour items on aligned buffers give tile by tile, and within 1e-5 of
+    the oracle."""
+    import torch
+    import gpu_runner as R
+    from cases import Case, rel_err
+    from tile_processor_gpu_b200 import api
+    c = Case(256, 192, seed=33, border_mode=0)
+    fr = R.Frame(c)
+    want = R.convert(fr, num_tiles=count)
+    o = oracle.convert_correct_tiles(c.geom, c.extra, c.kernels, c.pitched, c.dstride, c.tasks[:count])
+    assert max(rel_err(want[k], o[k]) for k in range(4)) < 1e-5
+    for name in ("images", "kernels", "extra", "clt"):
+        moved = _at_offset(getattr(fr, name), floats)
+        setattr(fr, name, moved)
+        setattr(fr, "p_" + name, api.PointerArray(moved))
+    got = R.convert(fr, num_tiles=count)
+    for k in range(4):
+        assert np.array_equal(got[k], want[k]), k
+    # the last four tasks alone, as items of one colour
+    n = min(4, count)
+    saved = fr.tasks
+    fr.tasks = saved[count - n:count].contiguous()
+    alone = R.convert(fr, num_tiles=n)
+    fr.tasks = saved
+    for k in range(4):
+        assert np.array_equal(alone[k][(count - n) * 768:count * 768], want[k][(count - n) * 768:count * 768]), k
+    torch.cuda.synchronize()

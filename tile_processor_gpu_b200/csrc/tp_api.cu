@@ -268,7 +268,7 @@ int tp_resident_ctas(int kernel)
     int n = 0, rc;
     cudaError_t e;
     if (kernel == TP_SHAPE_CONVERT) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_convert_correct_tiles, 256, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_convert_correct_tiles<3>, tp::kConvertThreads, 0);
     } else if (kernel == TP_SHAPE_CORRELATE) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_correlate2D, 128, 0);
     } else {
@@ -325,10 +325,15 @@ int tp_convert_correct_tiles(const tp_geometry *g, float *const *kernel_offsets,
     if (num_tiles == 0) return TP_OK;
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    const long long warps = (long long)((num_tiles + 3) / 4) * 12;
-    unsigned grid = grid_for(warps, 8, sms, shape_per_sm(TP_SHAPE_CONVERT));
-    tp::k_convert_correct_tiles<<<grid, 256, 0, (cudaStream_t)stream>>>(
-        gd, dstride, kernel_offsets, kernels, images, tasks, clt, num_tiles, lpf_mask);
+    /* one colour per warp item while those items fit the resident warps (3 CTAs
+     * per SM) in one turn, else all three (see the kernel) */
+    const long long chunks = ((long long)num_tiles + 3) / 4;
+    const bool small = chunks * 12 <= (long long)sms * 3 * (tp::kConvertThreads / 32);
+    unsigned grid = grid_for(chunks * (small ? 12 : 4), tp::kConvertThreads / 32, sms, shape_per_sm(TP_SHAPE_CONVERT));
+    if (!small) grid = (grid + 3) & ~3u; /* a warp keeps its camera */
+    const auto kernel = small ? tp::k_convert_correct_tiles<1> : tp::k_convert_correct_tiles<3>;
+    kernel<<<grid, tp::kConvertThreads, 0, (cudaStream_t)stream>>>(gd, dstride, kernel_offsets, kernels, images, tasks, clt,
+                                                   num_tiles, lpf_mask);
     return cuda_status(cudaGetLastError(), "convert_correct_tiles launch");
 }
 

@@ -28,7 +28,7 @@ __device__ __constant__ float c_hwinc[16] = TP_HWINC_INIT;
  * fetch distinct words in one pass, where the constant cache would serialise
  * them.  Runtime-settable low-pass filters: lpf_data[0..3], lpf_rb_corr,
  * lpf_corr. */
-__device__ __align__(16) float d_lpf[6][64] = TP_LPF_DEFAULT_INIT;
+__device__ __align__(32) float d_lpf[6][64] = TP_LPF_DEFAULT_INIT;
 __device__ float d_alpha_fade[16][256] = TP_ALPHA_FADE_INIT;
 __device__ float d_hwin[16] = TP_HWIN_INIT;
 __device__ float d_hwinc[16] = TP_HWINC_INIT;
@@ -206,6 +206,13 @@ __device__ __forceinline__ void dct4_pair(const float2 x[8], float2 y[8])
     y[1] = fma2(Zr[3], dup2(post[3][1]), mul2(n3, dup2(-post[3][0])));
 }
 #endif
+
+/* 8 consecutive floats of shared memory (16-byte aligned) */
+__device__ __forceinline__ void load_row8s(const float *p, float v[8])
+{
+    const float4 x = *reinterpret_cast<const float4 *>(p), y = *reinterpret_cast<const float4 *>(p + 4);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+}
 
 /* 8 consecutive floats of global memory (32-byte aligned): one 256-bit access */
 __device__ __forceinline__ void ld8_global(const float *p, float v[8])

@@ -7,14 +7,26 @@
  * same camera and color for four consecutive tasks, so the green jobs (two
  * Bayer phases and a DST pass) never share a warp with the cheaper red/blue
  * ones.  Per job:
- *   lane u gathers DTT row u of the folded, windowed Bayer samples (one image
- *   row, 8 same-color pixels), applies the row DCT-IV (green: also the row
- *   DST-IV of the sine-windowed fold), transposes through shared memory and
- *   applies the column DCT-IV, ending with column u of CC (and SC);
- *   the remaining quadrants come from the Bayer mirror symmetries by lane
- *   shuffles; the CLT-domain kernel, the two residual-shift rotations and the
- *   optional LPF are per-coefficient and run in registers; the 256
- *   coefficients are stored as 32-byte row segments.
+ *   lane v gathers DTT column v of the folded, windowed Bayer samples (8
+ *   same-color pixels of one image column; the group's 8 loads of one row are
+ *   one 64-byte run), applies the column DCT-IV, transposes through shared
+ *   memory and applies the row DCT-IV (green: also the row DST-IV of the
+ *   sine-windowed fold), ending with row v of CC (and SC);
+ *   the remaining quadrants come from the Bayer mirror symmetries, within the
+ *   row or from the opposite row; the CLT-domain kernel, the two
+ *   residual-shift rotations and the optional LPF are per coefficient, run on
+ *   pairs of coefficients (mul2 / fma2) and end in rows of 32 bytes, the width
+ *   of one load of the kernel tile and one store of the result.
+ *
+ * Lanes that hold rows make every access of the kernel tile and the CLT a
+ * whole 32-byte sector; holding columns (the transposed order of the two
+ * passes) took eight times as many load and store instructions and kept the L1
+ * busy 79% of the time at 55% issue.  815 warp instructions a job (1232
+ * before); a 2592x1936 frame went from 0.454 to 0.351 ms (2.87 to 3.71 TB/s of
+ * its 1.30 GB).  What bounds it now is the latency of a job's steps at 15 warps
+ * per SM: the samples, the kernel rows and the result of a job are 48 to 80
+ * registers, and more warps spill them (256 threads at 80 registers 0.448 ms,
+ * 192 at 96 0.451, 128 at 158 0.358).
  */
 #pragma once
 #include "tp_common.cuh"
@@ -42,10 +54,6 @@ __device__ __forceinline__ int pair_clamp(int idx, int n)
     return idx;
 }
 
-struct ConvertJob {
-    int cam, color;
-};
-
 /* Where a job's window sits and how its kernel tile and shifts follow from
  * the task's tile centre (float32, as the reference computes them:
  * src/TileProcessor.cuh:3129-3255). */
@@ -53,7 +61,6 @@ struct JobGeometry {
     size_t kidx;    /* kernel tile (x, y, colour) index into the table   */
     int itlx, itly; /* integer corner of the 16x16 window                */
     float shx, shy; /* residual shifts                                   */
-    float hc, hs, vc, vs; /* (cos, sin)(pi s / 16) of the shifted windows */
 };
 
 __device__ __forceinline__ JobGeometry job_geometry(const Geom &g, const float *__restrict__ extra_tab, float cx,
@@ -79,10 +86,6 @@ __device__ __forceinline__ JobGeometry job_geometry(const Geom &g, const float *
     j.itly = corner_clamp(__float2int_rd(py + 0.5f), g.H, false, g.border_mode);
     j.shx = (float)j.itlx - px;
     j.shy = (float)j.itly - py;
-    /* (cos, sin)(pi s / 16) for the shifted windows */
-    const float xh = j.shx * (1.0f / 16.0f), xv = j.shy * (1.0f / 16.0f);
-    sincospif(xh, &j.hs, &j.hc);
-    sincospif(xv, &j.vs, &j.vc);
     return j;
 }
 
@@ -90,14 +93,14 @@ __device__ __forceinline__ JobGeometry job_geometry(const Geom &g, const float *
  * rows of 20 floats from the 16-byte boundary at or left of the corner */
 constexpr int kCvWinW = 20, kCvWinH = 16;
 
-/* The fold: lane l builds DTT row l of the folded, windowed Bayer samples of
- * the job's colour (P: the cosine fold; Q: the sine-windowed fold of green,
- * zeros for red and blue), both Bayer phases of green summed
- * (src/TileProcessor.cuh:3257-3416).  win (may be NULL): the job's window in
- * shared memory, used for windows inside the image (the same samples). */
+/* The fold by rows, as the tensor-core form wants it: lane l builds DTT row l
+ * of the folded, windowed Bayer samples of the job's colour (P: the cosine
+ * fold; Q: the sine-windowed fold of green, zeros for red and blue), both
+ * Bayer phases of green summed (src/TileProcessor.cuh:3257-3416).  (hc, hs)
+ * and (vc, vs): (cos, sin)(pi s / 16) of the job's residual shifts. */
 __device__ __forceinline__ void fold_rows(const Geom &g, size_t dstride, const float *__restrict__ img,
-                                          const JobGeometry &j, int color, int l, float P[8], float Q[8],
-                                          const float *win = nullptr, int win_dx = 0)
+                                          const JobGeometry &j, int color, int l, float hc, float hs, float vc,
+                                          float vs, float P[8], float Q[8])
 {
     const int itlx = j.itlx, itly = j.itly;
     const int c0 = color & 1, c1 = (color >> 1) & 1;
@@ -111,7 +114,7 @@ __device__ __forceinline__ void fold_rows(const Geom &g, size_t dstride, const f
         const int colp = (itlx & 1) ^ (1 ^ c0 ^ c1 ^ gp);
         const int rowp = (itly & 1) ^ (c0 ^ gp);
         const int lr = fold_sample(l, rowp);
-        const float wv = fold_sign_c(lr) * shifted_window_lane(lr, j.vc, j.vs);
+        const float wv = fold_sign_c(lr) * shifted_window_lane(lr, vc, vs);
         long long rowbase;
         int eff_col = 0;
         if (fast) {
@@ -137,13 +140,9 @@ __device__ __forceinline__ void fold_rows(const Geom &g, size_t dstride, const f
             const int lc0 = fold_sample(v, 0), lc1 = fold_sample(v, 1);
             const int lc = colp ? lc1 : lc0;
             const float ww = colp ? kW[lc1] : kW[lc0], wwc = colp ? kWc[lc1] : kWc[lc0];
-            const float whs_raw = __fmaf_rn(ww, j.hc, wwc * j.hs);
+            const float whs_raw = __fmaf_rn(ww, hc, wwc * hs);
             float pix;
-            if (fast && win) {
-                /* the window staged in shared memory: rows of kCvWinW floats from
-                 * column itlx - win_dx */
-                pix = win[lr * kCvWinW + win_dx + lc];
-            } else if (fast) {
+            if (fast) {
                 pix = __ldg(img + rowbase + lc);
             } else if (g.border_mode == TP_BORDER_CLAMP) {
                 pix = __ldg(img + rowbase + pair_clamp(itlx + lc, g.W));
@@ -161,15 +160,302 @@ __device__ __forceinline__ void fold_rows(const Geom &g, size_t dstride, const f
     }
 }
 
-/* STREAM: out is global memory and takes evict-first stores.  The kernel
- * writes 963 MB of CLT for a full quad frame, far more than L2 holds, and
- * later kernels read it back; retaining the stores in L2 would only evict the
- * kernel tiles and Bayer rows that neighbouring jobs of this kernel still
- * read. */
-template <bool STREAM = false>
-__device__ __forceinline__ void convert_finish(const float *__restrict__ kern_tab, const JobGeometry &jg, int color,
-                                               int lpf_mask, float *__restrict__ out, float (*tb)[9], int l,
-                                               unsigned gm, float P[8], float Q[8]);
+/* (cos, sin) of a lane's residual-shift rotations: column l horizontally, row
+ * l vertically, pi s (2l + 1) / 16.  Lane 0's are the rotations of the shifted
+ * windows. */
+struct JobAngles {
+    float ch, sh, cv, sv;
+};
+
+__device__ __forceinline__ JobAngles job_angles(const JobGeometry &j, int l)
+{
+    JobAngles a;
+    sincospif((j.shx * (float)(2 * l + 1)) * 0.0625f, &a.sh, &a.ch);
+    sincospif((j.shy * (float)(2 * l + 1)) * 0.0625f, &a.sv, &a.cv);
+    return a;
+}
+
+/* Floats of a group's shared buffer: the shifted windows (vertical, horizontal
+ * cosine and sine fold: [2 parities][8 DTT indices] each), the horizontal
+ * rotations (8 cosines, 8 sines), then two 8x8 transposes with rows of 12
+ * (16-byte reads along rows and 4-byte writes down columns are conflict-free)
+ * or the mirror exchange with rows of 20.  264 % 32 == 8 keeps the four groups
+ * of a warp on distinct banks. */
+constexpr int kCvRot = 48, kCvTr = 64, kCvTrRow = 12, kCvMirRow = 20;
+constexpr int kCvBuf = 264;
+static_assert(kCvTr + 2 * 8 * kCvTrRow <= kCvBuf && kCvTr + 8 * kCvMirRow <= kCvBuf, "group buffer");
+
+/* 8 consecutive floats (16-byte aligned) as pairs */
+__device__ __forceinline__ void lds_row(const float *p, float2 v[4])
+{
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    v[0] = make_float2(a.x, a.y);
+    v[1] = make_float2(a.z, a.w);
+    v[2] = make_float2(b.x, b.y);
+    v[3] = make_float2(b.z, b.w);
+}
+
+/* The job's Bayer samples of DTT column l: pix[gp][u] = the sample of Bayer
+ * phase gp (green has two) that folds onto DTT row u, from image addresses as
+ * src/TileProcessor.cuh:3257-3416.  win (may be NULL): the job's window in
+ * shared memory, used for windows inside the image (the same samples). */
+__device__ __forceinline__ void load_pixels(const Geom &g, size_t dstride, const float *__restrict__ img,
+                                            const JobGeometry &j, int color, int l, float pix[2][8],
+                                            const float *win = nullptr, int win_dx = 0)
+{
+    const int itlx = j.itlx, itly = j.itly;
+    const int c0 = color & 1, c1 = (color >> 1) & 1;
+    const bool fast = (itlx >= 0) && (itlx < g.W - 16) && (itly >= 0) && (itly < g.H - 16);
+    const long long last = (long long)g.image_rows * (long long)dstride - 1;
+#pragma unroll
+    for (int gp = 0; gp < 2; gp++) {
+        if (gp > c1) break;
+        const int colp = (itlx & 1) ^ (1 ^ c0 ^ c1 ^ gp);
+        const int rowp = (itly & 1) ^ (c0 ^ gp);
+        const int lc = fold_sample(l, colp);
+        /* row i of the phase (rowp + 2i) at pix[u(i)]: the DTT rows of i at rowp
+         * 0; at rowp 1 neighbours 2k and 2k + 1 change places (fold_phase) */
+        constexpr int kI[8] = {6, 5, 7, 4, 0, 3, 1, 2};
+        if (fast && win) {
+            /* the window staged in shared memory: rows of kCvWinW floats from
+             * column itlx - win_dx */
+            const float *w = win + rowp * kCvWinW + win_dx + lc;
+#pragma unroll
+            for (int u = 0; u < 8; u++) pix[gp][u] = w[2 * kI[u] * kCvWinW];
+        } else if (fast) {
+            const float *w = img + (size_t)(itly + rowp) * dstride + (itlx + lc);
+#pragma unroll
+            for (int u = 0; u < 8; u++) pix[gp][u] = __ldg(w + kI[u] * (2 * dstride));
+        } else if (g.border_mode == TP_BORDER_CLAMP) {
+            const float *w = img + pair_clamp(itlx + lc, g.W);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                pix[gp][u] = __ldg(w + (size_t)pair_clamp(itly + rowp + 2 * kI[u], g.H) * dstride);
+        } else {
+            /* src/TileProcessor.cuh:3328-3361: columns clamped by IMG_HEIGHT/2,
+             * rows by IMG_WIDTH/2, row offset `rowp` added once */
+            const int cp = min(g.H / 2 - 1, max(0, itlx >> 1));
+            const int col = (cp << 1) + (itlx & 1) + lc;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int rp = min(g.W / 2 - 1, max(0, (itly >> 1) + kI[u]));
+                long long a = (long long)(rowp + (rp << 1) + (itly & 1)) * (long long)dstride + col;
+                a = a > last ? last : (a < 0 ? 0 : a);
+                pix[gp][u] = __ldg(img + a);
+            }
+        }
+    }
+}
+
+/* The fold by columns: lane l builds DTT column l (P[k] = rows 2k, 2k + 1; Q
+ * for green) of the folded, windowed Bayer samples of load_pixels, both Bayer
+ * phases of green summed.  Leaves the group's rotations in buf. */
+__device__ __forceinline__ void fold_cols(const JobGeometry &j, const JobAngles &ang, int color, int l, unsigned gm,
+                                          float *buf, const float pix[2][8], float2 P[4], float2 Q[4])
+{
+    const int itlx = j.itlx, itly = j.itly;
+    const int c0 = color & 1, c1 = (color >> 1) & 1;
+    const float hc = __shfl_sync(gm, ang.ch, 0, 8), hs = __shfl_sync(gm, ang.sh, 0, 8);
+    const float vc = __shfl_sync(gm, ang.cv, 0, 8), vs = __shfl_sync(gm, ang.sv, 0, 8);
+    /* the lane's two of the 16 window samples, n = l and l + 8, at their
+     * parity and DTT index, with the signs of the fold branches (cosine: + for
+     * n < 4; sine: + for n < 12) */
+    {
+        const float s0 = l < 4 ? 1.0f : -1.0f;
+        const int i0 = (l & 1) * 8 + (l < 4 ? l + 4 : 11 - l), i1 = (l & 1) * 8 + (l < 4 ? 3 - l : l - 4);
+        const float h0 = shifted_window_lane(l, hc, hs), h1 = shifted_window_lane(l + 8, hc, hs);
+        buf[i0] = s0 * shifted_window_lane(l, vc, vs);
+        buf[i1] = -shifted_window_lane(l + 8, vc, vs);
+        buf[16 + i0] = s0 * h0;
+        buf[16 + i1] = -h1;
+        buf[32 + i0] = h0;
+        buf[32 + i1] = s0 * h1;
+        buf[kCvRot + l] = ang.ch;
+        buf[kCvRot + 8 + l] = ang.sh;
+    }
+    __syncwarp(gm);
+#pragma unroll
+    for (int gp = 0; gp < 2; gp++) {
+        if (gp > c1) break;
+        const int colp = (itlx & 1) ^ (1 ^ c0 ^ c1 ^ gp);
+        const int rowp = (itly & 1) ^ (c0 ^ gp);
+        float2 wv[4];
+        lds_row(buf + rowp * 8, wv);
+        const float2 whc = dup2(buf[16 + colp * 8 + l]);
+        const float2 whs = c1 ? dup2(buf[32 + colp * 8 + l]) : whc;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float x = pix[gp][2 * k], y = pix[gp][2 * k + 1];
+            const float2 d = mul2(make_float2(rowp ? y : x, rowp ? x : y), wv[k]);
+            P[k] = gp ? fma2(d, whc, P[k]) : mul2(d, whc);
+            if (c1) Q[k] = gp ? fma2(d, whs, Q[k]) : mul2(d, whs);
+        }
+    }
+}
+
+/* Row l of the four quadrants of a kernel tile (p: row l of the first),
+ * read-only for the whole launch: one 256-bit load each where the tile lies on
+ * a 32-byte boundary */
+__device__ __forceinline__ void load_kernel_rows(const float *p, float2 v[4][4])
+{
+    if (!(reinterpret_cast<uintptr_t>(p) & 31)) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                         : "=f"(v[q][0].x), "=f"(v[q][0].y), "=f"(v[q][1].x), "=f"(v[q][1].y), "=f"(v[q][2].x),
+                           "=f"(v[q][2].y), "=f"(v[q][3].x), "=f"(v[q][3].y)
+                         : "l"(p + q * 64));
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[q][k] = make_float2(__ldg(p + q * 64 + 2 * k), __ldg(p + q * 64 + 2 * k + 1));
+    }
+}
+
+/* Row l of the four quadrants of a result (p: row l of the first).  STREAM:
+ * global memory, evict-first (the kernel writes 963 MB of CLT for a full quad
+ * frame, far more than L2 holds, and later kernels read it back; retaining the
+ * stores in L2 would only evict the kernel tiles and Bayer rows that
+ * neighbouring jobs of this kernel still read); else shared memory, 16-byte
+ * aligned */
+template <bool STREAM>
+__device__ __forceinline__ void store_rows(float *p, const float2 v[4][4])
+{
+    if (!STREAM) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+                reinterpret_cast<float4 *>(p + q * 64)[k] =
+                    make_float4(v[q][2 * k].x, v[q][2 * k].y, v[q][2 * k + 1].x, v[q][2 * k + 1].y);
+    } else if (!(reinterpret_cast<uintptr_t>(p) & 31)) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + q * 64),
+                         "f"(v[q][0].x), "f"(v[q][0].y), "f"(v[q][1].x), "f"(v[q][1].y), "f"(v[q][2].x),
+                         "f"(v[q][2].y), "f"(v[q][3].x), "f"(v[q][3].y)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                __stcs(p + q * 64 + 2 * k, v[q][k].x);
+                __stcs(p + q * 64 + 2 * k + 1, v[q][k].y);
+            }
+    }
+}
+
+/* The rest of a job after its fold (fold_cols: P, Q, the rotations in buf; kq:
+ * row l of its kernel tile): 2-D transform, CLT-domain convolution with the kernel tile, residual
+ * shifts, LPF, store. */
+template <bool STREAM>
+__device__ __forceinline__ void convert_finish(const JobGeometry &jg, const JobAngles &ang, int color, int lpf_mask, float *__restrict__ out,
+                                               float *buf, int l, unsigned gm, const float2 kq[4][4],
+                                               const float2 P[4], const float2 Q[4])
+{
+    const int itlx = jg.itlx, itly = jg.itly;
+    const int c1 = (color >> 1) & 1;
+    float *tr = buf + kCvTr;
+    /* ---- 2-D transform: columns (registers), transpose, rows; a[q]: row l
+     * of the four quadrants as pairs ---- */
+    float2 a[4][4];
+    {
+        float cc[8], row[8];
+        if (c1) {
+            /* the cosine and the sine-windowed fold side by side */
+            float2 x[8], y[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                x[2 * k] = make_float2(P[k].x, Q[k].x);
+                x[2 * k + 1] = make_float2(P[k].y, Q[k].y);
+            }
+            dct4_pair(x, y);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                tr[k * kCvTrRow + l] = y[k].x;
+                tr[(8 + k) * kCvTrRow + l] = y[k].y;
+            }
+        } else {
+            const float x[8] = {P[0].x, P[0].y, P[1].x, P[1].y, P[2].x, P[2].y, P[3].x, P[3].y};
+            float y[8];
+            dtt8<0>(x, y);
+#pragma unroll
+            for (int k = 0; k < 8; k++) tr[k * kCvTrRow + l] = y[k];
+        }
+        __syncwarp(gm);
+        load_row8s(tr + l * kCvTrRow, row);
+        dtt8<0>(row, cc); /* row l of CC */
+        float sc[8];
+        if (c1) {
+            load_row8s(tr + (8 + l) * kCvTrRow, row);
+            dtt8<1>(row, sc); /* row l of SC */
+        } else {
+            /* R, B: SC[i][7-j] = +-CC[i][j] (src/TileProcessor.cuh:3459-3475) */
+            const float neg1 = 1.0f - 2.0f * (float)((itlx & 1) ^ (1 ^ color));
+#pragma unroll
+            for (int m = 0; m < 8; m++) sc[m] = neg1 * cc[7 - m];
+        }
+        __syncwarp(gm); /* the transposes read */
+        /* SS[7-i][7-j] = +-CC[i][j], CS[7-i][7-j] = +-SC[i][j] (:3486-3504):
+         * from the opposite row, reversed */
+        float *mir = tr + l * kCvMirRow;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            reinterpret_cast<float4 *>(mir)[k] =
+                make_float4(cc[7 - 4 * k], cc[6 - 4 * k], cc[5 - 4 * k], cc[4 - 4 * k]);
+            reinterpret_cast<float4 *>(mir + 8)[k] =
+                make_float4(sc[7 - 4 * k], sc[6 - 4 * k], sc[5 - 4 * k], sc[4 - 4 * k]);
+        }
+        __syncwarp(gm);
+        const float2 neg2 = dup2(1.0f - 2.0f * (float)((itlx & 1) ^ (itly & 1) ^ 1 ^ c1));
+        lds_row(tr + (7 - l) * kCvMirRow, a[3]);
+        lds_row(tr + (7 - l) * kCvMirRow + 8, a[2]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            a[0][k] = make_float2(cc[2 * k], cc[2 * k + 1]);
+            a[1][k] = make_float2(sc[2 * k], sc[2 * k + 1]);
+            a[2][k] = mul2(neg2, a[2][k]);
+            a[3][k] = mul2(neg2, a[3][k]);
+        }
+    }
+
+    /* ---- CLT-domain convolution (src/TileProcessor.cuh:2778-2827), then the
+     * residual shift: horizontal (per column, shared across the group), then
+     * vertical (this lane's row) (:2715-2776) ---- */
+    float2 ch[4], sh[4];
+    lds_row(buf + kCvRot, ch);
+    lds_row(buf + kCvRot + 8, sh);
+    const float2 cv = dup2(ang.cv), sv = dup2(ang.sv), nsv = dup2(-ang.sv);
+    float2 o[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 a0 = a[0][k], a1 = a[1][k], a2 = a[2][k], a3 = a[3][k];
+        const float2 k0 = kq[0][k], k1 = kq[1][k], k2 = kq[2][k], k3 = kq[3][k];
+        const float2 x0 = sub2(fma2(a3, k3, mul2(a0, k0)), fma2(a2, k2, mul2(a1, k1)));
+        const float2 x1 = sub2(fma2(a0, k1, mul2(a1, k0)), fma2(a3, k2, mul2(a2, k3)));
+        const float2 x2 = sub2(fma2(a0, k2, mul2(a2, k0)), fma2(a3, k1, mul2(a1, k3)));
+        const float2 x3 = fma2(a0, k3, fma2(a1, k2, fma2(a2, k1, mul2(a3, k0))));
+        const float2 nsh = make_float2(-sh[k].x, -sh[k].y);
+        const float2 y0 = fma2(x0, ch[k], mul2(x1, nsh)), y1 = fma2(x0, sh[k], mul2(x1, ch[k]));
+        const float2 y2 = fma2(x2, ch[k], mul2(x3, nsh)), y3 = fma2(x2, sh[k], mul2(x3, ch[k]));
+        o[0][k] = fma2(y0, cv, mul2(y2, nsv));
+        o[2][k] = fma2(y0, sv, mul2(y2, cv));
+        o[1][k] = fma2(y1, cv, mul2(y3, nsv));
+        o[3][k] = fma2(y1, sv, mul2(y3, cv));
+    }
+    if ((lpf_mask >> color) & 1) { /* optional LPF (:3572-3593) */
+        float2 f[4];
+        lds_row(&d_lpf[color][l * 8], f);
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) o[q][k] = mul2(o[q][k], f[k]);
+    }
+    store_rows<STREAM>(out + l * 8, o);
+    __syncwarp(gm); /* buf free for the group's next job */
+}
 
 template <bool STREAM = false>
 __device__ __forceinline__ void convert_job(const Geom &g, size_t dstride,
@@ -177,182 +463,123 @@ __device__ __forceinline__ void convert_job(const Geom &g, size_t dstride,
                                             const float *__restrict__ kern_tab,
                                             const float *__restrict__ img, float cx, float cy,
                                             int color, int lpf_mask, float *__restrict__ out,
-                                            float (*tb)[9], int l, unsigned gm, const float *pre_ex = nullptr)
+                                            float *buf, int l, unsigned gm, const float *pre_ex = nullptr)
 {
     const JobGeometry jg = job_geometry(g, extra_tab, cx, cy, color, pre_ex);
-    /* ---- fold: lane l builds DTT row l ---- */
-    float P[8], Q[8];
-    fold_rows(g, dstride, img, jg, color, l, P, Q);
-    convert_finish<STREAM>(kern_tab, jg, color, lpf_mask, out, tb, l, gm, P, Q);
+    /* the samples and the kernel tile's rows in flight together, while the
+     * angles and windows are computed */
+    float pix[2][8];
+    load_pixels(g, dstride, img, jg, color, l, pix);
+    float2 kq[4][4];
+    load_kernel_rows(kern_tab + jg.kidx * 256 + l * 8, kq);
+    const JobAngles ang = job_angles(jg, l);
+    float2 P[4], Q[4];
+    fold_cols(jg, ang, color, l, gm, buf, pix, P, Q);
+    convert_finish<STREAM>(jg, ang, color, lpf_mask, out, buf, l, gm, kq, P, Q);
 }
 
-/* The rest of a job after its fold: 2-D transform, CLT-domain convolution
- * with the kernel tile, residual shifts, LPF, store. */
-template <bool STREAM>
-__device__ __forceinline__ void convert_finish(const float *__restrict__ kern_tab, const JobGeometry &jg, int color,
-                                               int lpf_mask, float *__restrict__ out, float (*tb)[9], int l,
-                                               unsigned gm, float P[8], float Q[8])
-{
-    const size_t kidx = jg.kidx;
-    const int itlx = jg.itlx, itly = jg.itly;
-    const float shx = jg.shx, shy = jg.shy;
-    const int c1 = (color >> 1) & 1;
-
-    /* ---- 2-D transform: rows (registers), transpose, columns ---- */
-    float cc[8], sc[8], cs[8], ss[8], t[8];
-    dtt8<0>(P, t);
-    group_transpose(tb, t, P, l, gm);
-    dtt8<0>(P, cc); /* lane l: column l of CC */
-    if (c1) {
-        dtt8<1>(Q, t);
-        group_transpose(tb, t, Q, l, gm);
-        dtt8<0>(Q, sc); /* column l of SC */
-    } else {
-        /* R, B: SC[i][7-j] = +-CC[i][j] (src/TileProcessor.cuh:3459-3475) */
-        const float neg1 = 1.0f - 2.0f * (float)((itlx & 1) ^ (1 ^ color));
-#pragma unroll
-        for (int m = 0; m < 8; m++) sc[m] = neg1 * __shfl_xor_sync(gm, cc[m], 7);
-    }
-    /* SS[7-i][7-j] = +-CC[i][j], CS[7-i][7-j] = +-SC[i][j] (:3486-3504) */
-    const float neg2 = 1.0f - 2.0f * (float)((itlx & 1) ^ (itly & 1) ^ 1 ^ c1);
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        ss[m] = neg2 * __shfl_xor_sync(gm, cc[7 - m], 7);
-        cs[m] = neg2 * __shfl_xor_sync(gm, sc[7 - m], 7);
-    }
-
-    /* ---- CLT-domain convolution (src/TileProcessor.cuh:2778-2827) ---- */
-    const float *kr = kern_tab + kidx * 256 + l;
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        const float k0 = __ldg(kr + m * 8), k1 = __ldg(kr + 64 + m * 8);
-        const float k2 = __ldg(kr + 128 + m * 8), k3 = __ldg(kr + 192 + m * 8);
-        const float a0 = cc[m], a1 = sc[m], a2 = cs[m], a3 = ss[m];
-        cc[m] = __fmaf_rn(a3, k3, __fmaf_rn(-a2, k2, __fmaf_rn(-a1, k1, a0 * k0)));
-        sc[m] = __fmaf_rn(-a2, k3, __fmaf_rn(-a3, k2, __fmaf_rn(a0, k1, a1 * k0)));
-        cs[m] = __fmaf_rn(-a1, k3, __fmaf_rn(a0, k2, __fmaf_rn(-a3, k1, a2 * k0)));
-        ss[m] = __fmaf_rn(a0, k3, __fmaf_rn(a1, k2, __fmaf_rn(a2, k1, a3 * k0)));
-    }
-
-    /* ---- residual shift: horizontal (this lane's column), then vertical
-     * (per row, angles shared across the group) (:2715-2776) ---- */
-    {
-        const float a = (shx * (float)(2 * l + 1)) * 0.0625f;
-        float ch, sh;
-        sincospif(a, &sh, &ch);
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const float x0 = cc[m], x1 = sc[m], x2 = cs[m], x3 = ss[m];
-            cc[m] = x0 * ch - x1 * sh;
-            sc[m] = x0 * sh + x1 * ch;
-            cs[m] = x2 * ch - x3 * sh;
-            ss[m] = x2 * sh + x3 * ch;
-        }
-    }
-    {
-        const float a = (shy * (float)(2 * l + 1)) * 0.0625f;
-        float cvl, svl;
-        sincospif(a, &svl, &cvl);
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const float cv = __shfl_sync(gm, cvl, m, 8), sv = __shfl_sync(gm, svl, m, 8);
-            const float x0 = cc[m], x1 = sc[m], x2 = cs[m], x3 = ss[m];
-            cc[m] = x0 * cv - x2 * sv;
-            cs[m] = x0 * sv + x2 * cv;
-            sc[m] = x1 * cv - x3 * sv;
-            ss[m] = x1 * sv + x3 * cv;
-        }
-    }
-    if ((lpf_mask >> color) & 1) { /* optional LPF (:3572-3593) */
-#pragma unroll
-        for (int m = 0; m < 8; m++) {
-            const float f = __ldg(&d_lpf[color][m * 8 + l]);
-            cc[m] *= f; sc[m] *= f; cs[m] *= f; ss[m] *= f;
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-        if constexpr (STREAM) {
-            __stcs(out + m * 8 + l, cc[m]);
-            __stcs(out + 64 + m * 8 + l, sc[m]);
-            __stcs(out + 128 + m * 8 + l, cs[m]);
-            __stcs(out + 192 + m * 8 + l, ss[m]);
-        } else {
-            out[m * 8 + l] = cc[m];
-            out[64 + m * 8 + l] = sc[m];
-            out[128 + m * 8 + l] = cs[m];
-            out[192 + m * 8 + l] = ss[m];
-        }
-    }
-}
-
-/* Warp w of the grid-stride loop handles tasks 4*(w/12) .. +3 for camera
- * (w%12)%4 and color (w%12)/4. */
-__global__ void __launch_bounds__(256, 3) k_convert_correct_tiles(
+/* A warp's item of the grid-stride loop is four consecutive tasks of one camera
+ * with PER colours: 3, one job after another (the tasks' fields and kernel tile
+ * are then found once for three jobs, and the warp keeps its camera's tables),
+ * or 1 (item % 12 = colour * 4 + camera), which spreads a small list over
+ * three times as many warps.  The host takes PER 1 as long as its items fit
+ * the resident warps in one turn: past that the shared work is worth more
+ * (2592x1936 frame: 0.351 ms, 0.374 with PER 1).
+ * The fields of the next item's tasks are read an item ahead, the offsets of
+ * the next job's kernel tile a job ahead, and the kernel tile itself is
+ * prefetched into L2 an item ahead (lane l: bytes 128 l .. 128 l + 127 of the
+ * 1 KB tile). */
+constexpr int kConvertThreads = 160;
+template <int PER>
+__global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
     Geom g, size_t dstride, float *const *kernel_offsets, float *const *kernels,
     float *const *images, const tp_task *__restrict__ tasks, float *const *clt, int num_tiles,
     int lpf_mask)
 {
-    __shared__ float tbuf[256 / 8][8][9];
+    static_assert(PER == 1 || PER == 3, "colours per item");
+    __shared__ __align__(16) float cbuf[kConvertThreads / 8][kCvBuf];
     const int l = threadIdx.x & 7;
     const int grp = threadIdx.x >> 3;
     const unsigned gm = group_mask();
-    const int warps_total = gridDim.x * (blockDim.x >> 5);
-    const int chunks = (num_tiles + 3) >> 2;
-    /* the task fields of this group's job, read two jobs ahead so that the
-     * loads overlap the jobs before it */
-    auto fetch = [&](int w, int *task, int *txy, float *cx, float *cy) {
-        *task = 0;
-        if (w >= chunks * 12) return;
-        const int chunk = w / 12, r = w - chunk * 12, cam = r & 3;
-        const int n = chunk * 4 + ((threadIdx.x >> 3) & 3);
-        if (n >= num_tiles) return;
-        const tp_task *t = tasks + n;
-        *task = __ldg(&t->task);
-        *txy = __ldg(&t->txy);
-        *cx = __ldg(&t->xy[cam][0]);
-        *cy = __ldg(&t->xy[cam][1]);
+    const int step = gridDim.x * (blockDim.x >> 5);
+    const int items = ((num_tiles + 3) >> 2) * (12 / PER);
+    /* a task of the list as this group sees it: its tile (-1: none) and centre */
+    struct Task {
+        int tile;
+        float cx, cy;
+        int ktile; /* kernel tile x + y * KH, times 3 */
     };
-    /* its kernel tile's offsets (the kernel-tile choice of convert_job),
-     * read one job ahead, and the kernel tile itself prefetched into L2
-     * (lane l: bytes 128 l .. 128 l + 127 of the 1 KB tile) */
-    auto fetch_extra = [&](int w, float cx, float cy, float ex[6]) {
-        const int r = w % 12, color = r >> 2, cam = r & 3;
+    auto fetch = [&](int w) -> Task {
+        Task t = {-1, 0.0f, 0.0f, 0};
+        if (w >= items) return t;
+        const int chunk = PER == 3 ? w >> 2 : w / 12, cam = PER == 3 ? w & 3 : (w - chunk * 12) & 3;
+        const int n = chunk * 4 + (grp & 3);
+        if (n >= num_tiles) return t;
+        const tp_task *p = tasks + n;
+        const int task = __ldg(&p->task), txy = __ldg(&p->txy);
+        const int tx = txy & 0xfff, ty = txy >> 16;
+        t.cx = __ldg(&p->xy[cam][0]);
+        t.cy = __ldg(&p->xy[cam][1]);
+        if (!task || tx >= g.TX || ty < 0 || ty >= g.TY) return t;
+        t.tile = ty * g.TX + tx;
+        /* the kernel tile (as job_geometry chooses it) */
         const float step_inv = __int_as_float((127 - g.ls) << 23);
-        const int ktx = min(g.KH - 1, max(0, __float2int_rn(__fmaf_rn(cx, step_inv, 1.0f))));
-        const int kty = min(g.KV - 1, max(0, __float2int_rn(__fmaf_rn(cy, step_inv, 1.0f))));
-        const size_t kidx = ((size_t)ktx + (size_t)kty * g.KH) * 3 + color;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(kernels[cam] + kidx * 256 + l * 32));
-        const float *e = kernel_offsets[cam] + kidx * 8;
+        const int ktx = min(g.KH - 1, max(0, __float2int_rn(__fmaf_rn(t.cx, step_inv, 1.0f))));
+        const int kty = min(g.KV - 1, max(0, __float2int_rn(__fmaf_rn(t.cy, step_inv, 1.0f))));
+        t.ktile = (ktx + kty * g.KH) * 3;
+        return t;
+    };
+    auto fetch_extra = [&](const float *extra, int ktile, int color, float ex[6]) {
+        const float *e = extra + (size_t)(ktile + color) * 8;
         ex[0] = __ldg(e + 0); ex[1] = __ldg(e + 1);
         ex[2] = __ldg(e + 4); ex[3] = __ldg(e + 5);
         ex[4] = __ldg(e + 6); ex[5] = __ldg(e + 7);
     };
     int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    int ntask = 0, ntxy = 0;
-    float ncx = 0.0f, ncy = 0.0f, nex[6];
-    fetch(w, &ntask, &ntxy, &ncx, &ncy);
-    if (ntask) fetch_extra(w, ncx, ncy, nex);
-    int n2task = 0, n2txy = 0;
-    float n2cx = 0.0f, n2cy = 0.0f;
-    fetch(w + warps_total, &n2task, &n2txy, &n2cx, &n2cy);
-    for (; w < chunks * 12; w += warps_total) {
-        const int chunk = w / 12, r = w - chunk * 12;
-        const int color = r >> 2, cam = r & 3;
-        const int task = ntask, txy = ntxy;
-        const float cx = ncx, cy = ncy;
-        float ex[6];
+    /* PER 3: the grid, and so the step, is a multiple of 4: a warp keeps its camera */
+    int cam = PER == 3 ? w & 3 : (w % 12) & 3;
+    const float *kern = kernels[cam], *extra = kernel_offsets[cam], *img = images[cam];
+    float *out = clt[cam];
+    Task next = fetch(w);
+    float nex[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (next.tile >= 0) fetch_extra(extra, next.ktile, PER == 3 ? 0 : (w % 12) >> 2, nex);
+    for (; w < items; w += step) {
+        const Task t = next;
+        const int color0 = PER == 3 ? 0 : (w % 12) >> 2;
+        next = fetch(w + step);
+        const float *kern_n = kern, *extra_n = extra, *img_n = img;
+        float *out_n = out;
+        const int color_n = PER == 3 ? 0 : ((w + step) % 12) >> 2;
+        if (PER == 1) {
+            const int c = ((w + step) % 12) & 3;
+            kern_n = kernels[c];
+            extra_n = kernel_offsets[c];
+            img_n = images[c];
+            out_n = clt[c];
+        }
+#pragma unroll 1
+        for (int i = 0; i < PER; i++) {
+            const int color = color0 + i;
+            float ex[6];
 #pragma unroll
-        for (int i = 0; i < 6; i++) ex[i] = nex[i];
-        ntask = n2task; ntxy = n2txy; ncx = n2cx; ncy = n2cy;
-        if (ntask) fetch_extra(w + warps_total, ncx, ncy, nex);
-        fetch(w + 2 * warps_total, &n2task, &n2txy, &n2cx, &n2cy);
-        if (!task) continue;
-        const int tx = txy & 0xfff, ty = txy >> 16;
-        if (tx >= g.TX || ty < 0 || ty >= g.TY) continue;
-        float *out = clt[cam] + (((size_t)ty * g.TX + tx) * 3 + color) * 256;
-        convert_job<true>(g, dstride, kernel_offsets[cam], kernels[cam], images[cam], cx, cy, color,
-                    lpf_mask, out, tbuf[grp], l, gm, ex);
+            for (int k = 0; k < 6; k++) ex[k] = nex[k];
+            if (i + 1 < PER) {
+                if (t.tile >= 0) fetch_extra(extra, t.ktile, color + 1, nex);
+            } else if (next.tile >= 0) {
+                fetch_extra(extra_n, next.ktile, color_n, nex);
+            }
+            if (next.tile >= 0)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(kern_n + (size_t)(next.ktile + color_n + i) * 256 + l * 32));
+            if (t.tile < 0) continue;
+            convert_job<true>(g, dstride, extra, kern, img, t.cx, t.cy, color, lpf_mask,
+                              out + ((size_t)t.tile * 3 + color) * 256, cbuf[grp], l, gm, ex);
+        }
+        if (PER == 1) {
+            kern = kern_n;
+            extra = extra_n;
+            img = img_n;
+            out = out_n;
+        }
     }
 }
 

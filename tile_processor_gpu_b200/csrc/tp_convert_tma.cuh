@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kCvThreads, 2) k_convert_tma(
 {
     extern __shared__ __align__(128) unsigned char cv_smem[];
     __shared__ __align__(8) uint64_t bars[2 * kCvSlots]; /* full[slot], then empty[slot] */
-    __shared__ float tbuf[kCvConsumers * 4][8][9];
+    __shared__ __align__(16) float cbuf[kCvConsumers * 4][kCvBuf];
     const uint32_t base_s = (uint32_t)__cvta_generic_to_shared(cv_smem);
     const uint32_t pad = (128 - (base_s & 127)) & 127;
     unsigned char *sm = cv_smem + pad;
@@ -169,11 +169,11 @@ __global__ void __launch_bounds__(kCvThreads, 2) k_convert_tma(
             const long long w = blockIdx.x + k * gridDim.x;
             const int chunk = (int)(w / 12), r = (int)(w - (long long)chunk * 12);
             const int color = r >> 2, cam = r & 3;
-            float P[8], Q[8];
+            float pix[2][8];
             if (m.task) {
                 const float *win =
                     m.fast ? reinterpret_cast<const float *>(sm + (size_t)(slot * 4 + grp) * kCvWinBytes) : nullptr;
-                fold_rows(g, dstride, images[cam], m.jg, color, l, P, Q, win, m.dx);
+                load_pixels(g, dstride, images[cam], m.jg, color, l, pix, win, m.dx);
             }
             /* the window and the metadata read: the slot may be refilled */
             __syncwarp();
@@ -181,7 +181,11 @@ __global__ void __launch_bounds__(kCvThreads, 2) k_convert_tma(
             if (m.task) {
                 const int tx = m.txy & 0xfff, ty = m.txy >> 16;
                 float *out = clt[cam] + (((size_t)ty * g.TX + tx) * 3 + color) * 256;
-                convert_finish<true>(kernels[cam], m.jg, color, lpf_mask, out, tbuf[warp * 4 + grp], l, gm, P, Q);
+                float2 kq[4][4], P[4], Q[4];
+                load_kernel_rows(kernels[cam] + m.jg.kidx * 256 + l * 8, kq);
+                const JobAngles ang = job_angles(m.jg, l);
+                fold_cols(m.jg, ang, color, l, gm, cbuf[warp * 4 + grp], pix, P, Q);
+                convert_finish<true>(m.jg, ang, color, lpf_mask, out, cbuf[warp * 4 + grp], l, gm, kq, P, Q);
             }
         }
     }

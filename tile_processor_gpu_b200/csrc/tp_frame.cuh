@@ -55,6 +55,7 @@ constexpr int kFrameBlocksPerSm = 5;
  * place (kJob floats); per group the transpose buffer, the correlation
  * buffers of groups 0-5 (kCorrBuf each) and then the debayered tile D */
 constexpr int kFrameSmemFloats = 12 * kJob + 12 * kXb;
+static_assert(kCvBuf <= kXb, "the convert buffers overlay the transpose buffers");
 static_assert(6 * kCorrBuf <= 12 * kXb, "correlation buffers overlay the transpose buffers");
 static_assert(kJob >= 256 && kJob % 4 == 0, "a job holds its 256 CLT floats, 16-byte aligned");
 constexpr size_t kFrameSmemBytes = sizeof(float) * kFrameSmemFloats;
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
                 ex[3] = __ldg(e + 5); ex[4] = __ldg(e + 6); ex[5] = __ldg(e + 7);
             }
             convert_job(g, dstride, kernel_offsets[cam_c], kernels[cam_c], images[cam_c], cx, cy, color_c, p.lpf_mask,
-                        s_clt + (cam_c * 3 + color_c) * kJob, reinterpret_cast<float(*)[9]>(s_x + grp * kXb), l,
+                        s_clt + (cam_c * 3 + color_c) * kJob, s_x + grp * kXb, l,
                         gm, ex);
         }
         /* the block's next tile in this pass: lane i of every warp tests the

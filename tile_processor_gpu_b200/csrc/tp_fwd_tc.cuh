@@ -83,10 +83,16 @@ struct FwdTcStage {
         jg.itlx = jg.itly = 0;
         if (tile >= 0) {
             jg = job_geometry(g, kernel_offsets[cam], cx, cy, color, nullptr);
-            fold_rows(g, dstride, images[cam], jg, color, l, P, Q);
-            /* the rotation angles of column l (horizontal) and row l (vertical) */
-            sincospif((jg.shx * (float)(2 * l + 1)) * 0.0625f, &rot[1], &rot[0]);
-            sincospif((jg.shy * (float)(2 * l + 1)) * 0.0625f, &rot[3], &rot[2]);
+            /* the rotation angles of column l (horizontal) and row l (vertical);
+             * lane 0's are the shifted windows' */
+            const JobAngles ang = job_angles(jg, l);
+            rot[0] = ang.ch;
+            rot[1] = ang.sh;
+            rot[2] = ang.cv;
+            rot[3] = ang.sv;
+            fold_rows(g, dstride, images[cam], jg, color, l, __shfl_sync(gm, rot[0], 0, 8),
+                      __shfl_sync(gm, rot[1], 0, 8), __shfl_sync(gm, rot[2], 0, 8), __shfl_sync(gm, rot[3], 0, 8), P,
+                      Q);
         } else {
 #pragma unroll
             for (int v = 0; v < 8; v++) {

@@ -67,25 +67,21 @@ __device__ float d_tex_mfac[kFac] = TP_TEX_MFAC_INIT;
 __device__ float d_tex_wnd2[256] = TP_TEX_WND2_INIT;
 __device__ float d_tex_wi[256] = TP_TEX_WI_INIT;
 
-/* 8 consecutive floats of a CLT tile: one 256-bit load from global memory
- * where the tile allows it, else 16-byte or scalar loads (GLOBAL false:
- * shared memory) */
-template <bool GLOBAL>
-__device__ __forceinline__ void load_clt_row(const float *p, float v[8])
-{
-    if (GLOBAL && !(reinterpret_cast<uintptr_t>(p) & 31))
-        ld8_global(p, v);
-    else
-        load_row8(p, !(reinterpret_cast<uintptr_t>(p) & 15), v);
-}
-
 /* Lane l's rows of a job's CLT tile: row l of quadrants 0 and 1, row 7 - l of 2
- * and 3 (see imclt_pairs) */
+ * and 3 (see imclt_pairs); one 256-bit load each from global memory where the
+ * tile lies on a 32-byte boundary, else 16-byte or scalar loads (GLOBAL false:
+ * shared memory) */
 template <bool GLOBAL>
 __device__ __forceinline__ void load_clt_rows(const float *src, float raw[4][8], int l)
 {
+    if (GLOBAL && !(reinterpret_cast<uintptr_t>(src) & 31)) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) load_clt_row<GLOBAL>(src + q * 64 + (q < 2 ? l : 7 - l) * 8, raw[q]);
+        for (int q = 0; q < 4; q++) ld8_global(src + q * 64 + (q < 2 ? l : 7 - l) * 8, raw[q]);
+    } else {
+        const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
+#pragma unroll
+        for (int q = 0; q < 4; q++) load_row8(src + q * 64 + (q < 2 ? l : 7 - l) * 8, al16, raw[q]);
+    }
 }
 
 /* The four quadrants of one CLT tile to the pixel domain on an 8-lane group
