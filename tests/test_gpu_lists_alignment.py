@@ -128,3 +128,22 @@ def test_convert_counts_and_alignment(native, oracle, count, floats):
     for k in range(4):
         assert np.array_equal(alone[k][(count - n) * 768:count * 768], want[k][(count - n) * 768:count * 768]), k
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("radius,colors", [(7, 3), (7, 1), (3, 3), (0, 3)])
+@pytest.mark.parametrize("floats", [1, 4])
+def test_correlate_of_unaligned_clt(frame, radius, colors, floats):
+    """The narrower loads of a CLT off 32-byte boundaries give the bits of the
+    wide ones, in single entries as in the whole list."""
+    import gpu_runner as R
+    from tile_processor_gpu_b200 import api
+    c = frame.case
+    want = R.correlate(frame, c.corr_idx, colors=colors, radius=radius)
+    moved, saved = _at_offset(frame.clt, floats), frame.p_clt
+    frame.p_clt = api.PointerArray(moved)
+    try:
+        got = R.correlate(frame, c.corr_idx, colors=colors, radius=radius)
+        one = R.correlate(frame, c.corr_idx[13:14], colors=colors, radius=radius)
+    finally:
+        frame.p_clt = saved
+    assert np.array_equal(got, want) and np.array_equal(one[0], want[13])

@@ -270,7 +270,7 @@ int tp_resident_ctas(int kernel)
     if (kernel == TP_SHAPE_CONVERT) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_convert_correct_tiles<3>, tp::kConvertThreads, 0);
     } else if (kernel == TP_SHAPE_CORRELATE) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_correlate2D, 128, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_correlate2D, tp::kCorrThreads, 0);
     } else {
         if ((rc = texture_smem_setup())) return rc;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_textures<false, false, 3>, tp::kTexThreads,
@@ -354,10 +354,11 @@ int tp_correlate2D(const tp_geometry *g, float *const *clt, int colors, float sc
     if (corr_stride < sz) return fail(TP_ERR_ARG, "corr_stride %zu < (2r+1)^2 = %zu", corr_stride, sz);
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    unsigned grid = grid_for((long long)num_corr_tiles, 16, sms, shape_per_sm(TP_SHAPE_CORRELATE));
-    tp::k_correlate2D<<<grid, 128, 0, (cudaStream_t)stream>>>(gd, clt, colors, scale0, scale1, scale2, fat_zero,
-                                                              (long long)num_corr_tiles, corr_indices,
-                                                              corr_stride, corr_radius, corrs);
+    const unsigned grid = grid_for((long long)num_corr_tiles, tp::kCorrThreads / 8, sms,
+                                   shape_per_sm(TP_SHAPE_CORRELATE));
+    tp::k_correlate2D<<<grid, tp::kCorrThreads, 0, (cudaStream_t)stream>>>(
+        gd, clt, colors, scale0, scale1, scale2, fat_zero, (long long)num_corr_tiles, corr_indices, corr_stride,
+        corr_radius, corrs);
     return cuda_status(cudaGetLastError(), "correlate2D launch");
 }
 

@@ -205,6 +205,28 @@ __device__ __forceinline__ void dct4_pair(const float2 x[8], float2 y[8])
     y[6] = fma2(Zr[3], dup2(post[3][0]), mul2(n3, dup2(post[3][1])));
     y[1] = fma2(Zr[3], dup2(post[3][1]), mul2(n3, dup2(-post[3][0])));
 }
+
+/* dct2_fast<false> on both halves of pairs.  A DST-II half takes its input
+ * with alternating signs ((-1)^n x[n]) and finds its outputs in reverse order
+ * (DST_k at 7-k).  Bit-identical to dct2_fast. */
+__device__ __forceinline__ void dct2_pair(const float2 x[8], float2 r[8])
+{
+    constexpr float K[8] = TP_DCT2_FAST_INIT;
+    const float2 u0 = add2(x[0], x[7]), u1 = add2(x[1], x[6]), u2 = add2(x[2], x[5]), u3 = add2(x[3], x[4]);
+    const float2 v0 = sub2(x[0], x[7]), v1 = sub2(x[1], x[6]), v2 = sub2(x[2], x[5]), v3 = sub2(x[3], x[4]);
+    const float2 w0 = add2(u0, u3), w1 = add2(u1, u2), d0 = sub2(u0, u3), d1 = sub2(u1, u2);
+    r[0] = mul2(dup2(0.5f), add2(w0, w1));
+    r[4] = mul2(dup2(K[0]), sub2(w0, w1));
+    r[2] = fma2(d0, dup2(K[1]), mul2(d1, dup2(K[2])));
+    r[6] = fma2(d0, dup2(K[2]), mul2(d1, dup2(-K[1])));
+    const float2 z1r = mul2(dup2(K[3]), add2(v2, v1)), z1i = mul2(dup2(K[3]), sub2(v2, v1));
+    const float2 p0r = add2(v0, z1r), p0i = sub2(z1i, v3);
+    const float2 p1r = sub2(v0, z1r), n1i = add2(v3, z1i); /* n1i = -p1i */
+    r[1] = fma2(p0r, dup2(K[4]), mul2(p0i, dup2(-K[5])));
+    r[7] = fma2(p0r, dup2(K[5]), mul2(p0i, dup2(K[4])));
+    r[5] = fma2(p1r, dup2(K[6]), mul2(n1i, dup2(K[7])));
+    r[3] = fma2(p1r, dup2(K[7]), mul2(n1i, dup2(-K[6])));
+}
 #endif
 
 /* 8 consecutive floats of shared memory (16-byte aligned) */

@@ -28,61 +28,6 @@
 
 namespace tp {
 
-/* The normalised, low-pass-filtered CLT-domain product of one (tile, pair)
- * entry, row l of the four quadrants in acc (k_correlate2D's first half). */
-__device__ __forceinline__ void corr_product_rows(const float *a, const float *b, int cstride, int colors,
-                                                  float scale0, float scale1, float scale2, float fat_zero,
-                                                  int l, float acc[4][8])
-{
-    const bool al16 = !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
-                         (uintptr_t)(cstride * sizeof(float))) & 15);
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-#pragma unroll
-        for (int k = 0; k < 8; k++) acc[q][k] = 0.0f;
-    for (int color = 0; color < colors; color++) {
-        const float s = color == 0 ? scale0 : color == 1 ? scale1 : scale2;
-        float A[4][8], B[4][8];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            load_row8(a + color * cstride + q * 64 + l * 8, al16, A[q]);
-            load_row8(b + color * cstride + q * 64 + l * 8, al16, B[q]);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float a0 = A[0][k], a1 = A[1][k], a2 = A[2][k], a3 = A[3][k];
-            const float b0 = B[0][k], b1 = B[1][k], b2 = B[2][k], b3 = B[3][k];
-            const float r0 = __fmaf_rn(a3, b3, __fmaf_rn(a2, b2, __fmaf_rn(a1, b1, a0 * b0)));
-            const float r1 = __fmaf_rn(a2, b3, __fmaf_rn(-a3, b2, __fmaf_rn(a0, b1, -a1 * b0)));
-            const float r2 = __fmaf_rn(a1, b3, __fmaf_rn(a0, b2, __fmaf_rn(-a3, b1, -a2 * b0)));
-            const float r3 = __fmaf_rn(a0, b3, __fmaf_rn(-a1, b2, __fmaf_rn(-a2, b1, a3 * b0)));
-            acc[0][k] = __fmaf_rn(s, r0, acc[0][k]);
-            acc[1][k] = __fmaf_rn(s, r1, acc[1][k]);
-            acc[2][k] = __fmaf_rn(s, r2, acc[2][k]);
-            acc[3][k] = __fmaf_rn(s, r3, acc[3][k]);
-        }
-        if (color == 1) {
-            float f[8];
-            load_row8(&d_lpf[4][l * 8], true, f);
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[q][k] *= f[k];
-        }
-    }
-    float f[8];
-    load_row8(&d_lpf[5][l * 8], true, f);
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        float s2 = fat_zero * fat_zero;
-#pragma unroll
-        for (int q = 0; q < 4; q++) s2 = __fmaf_rn(acc[q][k], acc[q][k], s2);
-        const float sc = rsqrtf(s2);
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[q][k] = (acc[q][k] * sc) * f[k];
-    }
-}
-
 /* The correlation as a tensor-core stage (k_tc_stage): rows are index
  * entries; twelve producer warps (the CLT products are the heavy part), four
  * epilogue warps (512 threads, at most 128 registers each). */
@@ -119,18 +64,29 @@ struct CorrTcStage {
         (void)gm;
         (void)meta;
         int tile, pair;
-        float acc[4][8];
+        float2 acc[4][4], scale[4];
         if (entry(n, &tile, &pair)) {
-            corr_product_rows(clt[c_pairs[pair][0]] + (size_t)tile * 768, clt[c_pairs[pair][1]] + (size_t)tile * 768,
-                              256, colors, scale0, scale1, scale2, fat_zero, l, acc);
+            corr_product<true>(clt[c_pairs[pair][0]] + (size_t)tile * 768, clt[c_pairs[pair][1]] + (size_t)tile * 768,
+                               256, colors, scale0, scale1, scale2, fat_zero, l, acc, scale);
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; q++)
+            for (int k = 0; k < 4; k++) {
+                scale[k] = make_float2(0.0f, 0.0f);
 #pragma unroll
-                for (int k = 0; k < 8; k++) acc[q][k] = 0.0f;
+                for (int q = 0; q < 4; q++) acc[q][k] = make_float2(0.0f, 0.0f);
+            }
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) A.template put8<FMT>(row, q, l * 8, acc[q], up);
+        for (int q = 0; q < 4; q++) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 x = mul2(acc[q][k], scale[k]);
+                v[2 * k] = x.x;
+                v[2 * k + 1] = x.y;
+            }
+            A.template put8<FMT>(row, q, l * 8, v, up);
+        }
     }
 
     /* corrUnfoldTile: R[+-i][+-j] from q0[i][j], q1[i][j-1], q2[i-1][j],

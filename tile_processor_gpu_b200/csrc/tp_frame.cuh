@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
 
         /* ---- 2. correlations: group = pair ---- */
         if (grp < 6 && ((pairs >> grp) & 1))
-            corr_job<4>(s_clt + c_pairs[grp][0] * 3 * kJob, s_clt + c_pairs[grp][1] * 3 * kJob, kJob, p.corr_colors,
+            corr_job<false>(s_clt + c_pairs[grp][0] * 3 * kJob, s_clt + c_pairs[grp][1] * 3 * kJob, kJob, p.corr_colors,
                         p.s0, p.s1, p.s2, p.fat_zero, p.corr_radius, s_x + grp * kCorrBuf,
                         corrs + ((size_t)n * 6 + grp) * p.corr_stride, l, gm);
         /* the convert above has read s_pf: its next contents may be copied in */
