@@ -147,3 +147,28 @@ def test_correlate_of_unaligned_clt(frame, radius, colors, floats):
     finally:
         frame.p_clt = saved
     assert np.array_equal(got, want) and np.array_equal(one[0], want[13])
+
+
+@pytest.mark.parametrize("width,height,marks,floats,pitch", [
+    (32, 32, 0, 0, 0), (40, 48, 1, 1, 3), (120, 128, 0, 4, 1), (248, 32, 1, 0, 8), (1304, 904, 1, 0, 5)])
+def test_imclt_all_is_the_twelve_passes(native, width, height, marks, floats, pitch):
+    """The one-launch image equals the twelve parity passes bit for bit: odd and
+    even tile counts, strips and segments of one cell, the debug marks, an
+    unaligned CLT, an odd pitch, and an image that held other values before
+    (cells that pass (0, 0) does not cover accumulate onto them)."""
+    import torch
+    from tile_processor_gpu_b200 import api
+    g = api.Geometry(width, height, debug_marks=marks)
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    clt = torch.randn(g.num_tiles * 768, generator=gen, device="cuda")
+    clt = _at_offset([clt], floats)[0]
+    stride = width + 8 + pitch
+    before = torch.randn((3 * (height + 8), stride), generator=gen, device="cuda")
+    want, got = before.clone(), before.clone()
+    for color in range(3):
+        for v in range(2):
+            for h in range(2):
+                api.imclt_rbg(g, clt, want, color, v, h, stride)
+    api.imclt_rbg_all(g, clt, got, stride)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

@@ -459,13 +459,23 @@ int tp_imclt_rbg(const tp_geometry *g, const float *clt_one_cam, float *rbg, int
 int tp_imclt_rbg_all(const tp_geometry *g, const float *clt_one_cam, float *rbg, size_t dstride,
                      tp_stream_t stream)
 {
-    for (int color = 0; color < 3; color++)
-        for (int v = 0; v < 2; v++)
-            for (int h = 0; h < 2; h++) {
-                int rc = tp_imclt_rbg(g, clt_one_cam, rbg, color, v, h, dstride, stream);
-                if (rc) return rc;
-            }
-    return TP_OK;
+    tp::Geom gd;
+    int rc = check_geometry(g, &gd);
+    if (rc) return rc;
+    if (!clt_one_cam || !rbg) return fail(TP_ERR_ARG, "NULL clt / rbg");
+    if (dstride < (size_t)g->img_width + 8) return fail(TP_ERR_ARG, "dstride %zu < width + 8", dstride);
+    int sms;
+    if ((rc = sm_count(&sms))) return rc;
+    /* as many row segments as keep the blocks in one resident wave; a segment
+     * inverts one tile row more than it writes, so none is shorter than 2 */
+    const int strips = (gd.TX + tp::kImclCells) / tp::kImclCells, rows = gd.TY + 1;
+    int segs = sms * tp::kImclBlocksPerSm / (3 * strips);
+    segs = segs < 1 ? 1 : segs;
+    int seg_rows = (rows + segs - 1) / segs;
+    seg_rows = seg_rows < 2 ? 2 : seg_rows;
+    const dim3 grid((unsigned)strips, (unsigned)((rows + seg_rows - 1) / seg_rows), 3);
+    tp::k_imclt_rbg_all<<<grid, tp::kImclThreads, 0, (cudaStream_t)stream>>>(gd, clt_one_cam, rbg, dstride, seg_rows);
+    return cuda_status(cudaGetLastError(), "imclt_rbg_all launch");
 }
 
 /* Launch kern on stream s; with `dependent` as a programmatic dependent of

@@ -134,7 +134,8 @@ __device__ __forceinline__ int unfold_col(int l, int h) { return h ? ((l < 4) ? 
  * per column (columns 0-3: (+,+); 4-11: (-,+); 12-15: (-,-) on the (even,
  * odd) quadrants) and compile-time signs per row; cf, the column's window
  * factor, rides on the column's signs, as do the signs imclt_pairs left out;
- * kr[r] is the row's factor. */
+ * kr[r] is the row's factor (UNIT: 1 for every row). */
+template <bool UNIT = false>
 __device__ __forceinline__ void unfold_column(const float2 a02[8], const float2 a13[8], int l, int c, float cf,
                                               const float (&kr)[16], float2 t[8])
 {
@@ -154,7 +155,8 @@ __device__ __forceinline__ void unfold_column(const float2 a02[8], const float2 
             /* vertical signs: rows 0-3 (+,+); 4-11 (-,+); 12-15 (-,-) */
             d[i] = ((rq != 0) ? -e[u].x : e[u].x) + ((rq == 3) ? -e[u].y : e[u].y);
         }
-        t[rp] = mul2(make_float2(d[0], d[1]), make_float2(kr[2 * rp], kr[2 * rp + 1]));
+        t[rp] = make_float2(d[0], d[1]);
+        if (!UNIT) t[rp] = mul2(t[rp], make_float2(kr[2 * rp], kr[2 * rp + 1]));
     }
 }
 
