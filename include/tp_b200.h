@@ -442,6 +442,23 @@ int tp_mlp_gemm(int M, int N, int K, const float *A, int lda, int trans_a, const
 int tp_mlp_gemm_tc(int M, int N, int K, const float *A, int lda, int trans_a, const float *B, int ldb, int trans_b,
                    float beta, float *C, int ldc, const float *bias, float *z, int ldz, int *err,
                    tp_stream_t stream);
+/* The network's forward pass at rows feature rows x (leading dimension ldx >=
+ * 1350): z1, h1 [rows][256] and z2, h2 [rows][128] the pre-activations and
+ * activations, out [rows][2]; layers 1 and 2 as tp_mlp_gemm_tc, layer 3 in
+ * FP32.  params: host array of the six device arrays W1, b1, W2, b2, W3, b3.
+ * h2 16-byte and out 8-byte aligned. */
+int tp_mlp_forward(int rows, const float *x, int ldx, const float *const *params, float *z1, float *h1, float *z2,
+                   float *h2, float *out, int *err, tp_stream_t stream);
+/* The loss of tp_mlp_nll and the gradients of inv_count * its sum, from a
+ * tp_mlp_forward pass: dout [rows][2], loss_rows [rows] and their sum in
+ * *loss_sum (device double), dz2 [rows][128] and dz1 [rows][256] (the
+ * gradients of z2 and z1), and grads (host array of six device arrays, as
+ * params; overwritten).  The sums over rows are not added in a fixed order.
+ * dout and loss_sum 8-byte aligned. */
+int tp_mlp_loss_backward(int rows, const float *x, int ldx, const float *const *params, const float *z1,
+                         const float *h1, const float *z2, const float *h2, const float *out, const float *target,
+                         const float *w, float inv_count, float *dout, float *loss_rows, double *loss_sum, float *dz2,
+                         float *dz1, float *const *grads, int *err, tp_stream_t stream);
 /* dz = dh * gelu'(z), rows x cols, leading dimension ld */
 int tp_mlp_gelu_backward(int rows, int cols, int ld, const float *z, const float *dh, float *dz,
                          tp_stream_t stream);
@@ -474,6 +491,10 @@ int tp_mlp_combine(size_t n, const float *plain, const float *out, float gate, f
 /* Adam step `step` (1, 2, ...) on n parameters */
 int tp_mlp_adam(size_t n, float *param, const float *grad, float *m, float *v, float lr, float beta1, float beta2,
                 float eps, int step, tp_stream_t stream);
+/* The same step on `count` (at most 8) arrays in one launch: host arrays of
+ * their lengths and device pointers */
+int tp_mlp_adam_set(int count, const size_t *n, float *const *param, const float *const *grad, float *const *m,
+                    float *const *v, float lr, float beta1, float beta2, float eps, int step, tp_stream_t stream);
 
 /* ---- tensor-core precision forms of the stages ----------------------------------
  * The same calls as above, with each stage's batched 8x8 transforms (the

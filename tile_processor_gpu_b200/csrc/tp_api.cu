@@ -120,7 +120,7 @@ int shape_per_sm(int which)
  * their attribute once per device (the first call; make it before capturing
  * a stream into a graph). */
 std::mutex g_attr_mutex;
-bool g_tex_attr[8][128], g_frame_attr[128], g_tc_attr[128], g_gemm_tc_attr[128], g_cv_attr[128];
+bool g_tex_attr[8][128], g_frame_attr[128], g_tc_attr[128], g_gemm_tc_attr[4][128], g_cv_attr[128];
 
 int set_smem_once(bool *done, const void *func, size_t bytes, const char *what)
 {
@@ -807,6 +807,51 @@ int tp_mlp_gemm(int M, int N, int K, const float *A, int lda, int trans_a, const
     return cuda_status(cudaGetLastError(), "mlp_gemm launch");
 }
 
+/* floats per load along an operand's contiguous K (1 when K is not contiguous) */
+static tp::GtOperand gt_operand(const float *p, int ld, int rows, int across)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const int vec = across ? 1 : (!(a & 15) && !(ld & 3)) ? 4 : (!(a & 7) && !(ld & 1)) ? 2 : 1;
+    return tp::GtOperand{p, ld, rows, across ? 1 : 0, vec};
+}
+
+/* C = op(A) op(B) with the given epilogue, arguments checked by the caller */
+static int gemm_tc_launch(int M, int N, int K, const float *A, int lda, int trans_a, const float *B, int ldb,
+                          int trans_b, const tp::GtEpilogue &e, bool zeroed, int *err, cudaStream_t s)
+{
+    int rc, sms;
+    const bool ta = trans_a != 0, tb = !trans_b;
+    const auto kernel = ta ? (tb ? tp::k_gemm_tc<true, true> : tp::k_gemm_tc<true, false>)
+                           : (tb ? tp::k_gemm_tc<false, true> : tp::k_gemm_tc<false, false>);
+    if ((rc = set_smem_once(g_gemm_tc_attr[2 * ta + tb], (const void *)kernel, tp::kGtSmemBytes,
+                            "cudaFuncSetAttribute(k_gemm_tc)")))
+        return rc;
+    if ((rc = sm_count(&sms))) return rc;
+    dim3 grid((unsigned)((N + tp::kGtN - 1) / tp::kGtN), (unsigned)((M + tp::kGtM - 1) / tp::kGtM), 1);
+    /* A plain product (no bias, beta 0, no GELU) with at most half as many tiles
+     * as SMs and a long K (the weight gradients: K = the batch) splits K over
+     * as many CTAs as fill the SMs once (a CTA takes an SM's shared memory), at
+     * least four chunks each, adding their partial sums into C, zeroed first
+     * (the order of those few additions per element is not fixed). */
+    const long long tiles = (long long)grid.x * grid.y;
+    const int chunks = (K + tp::kGtK - 1) / tp::kGtK;
+    if (!e.bias && !e.z && e.beta == 0.0f && tiles <= sms / 2 && chunks >= 8) {
+        long long splits = sms / tiles;
+        if (splits > chunks / 4) splits = chunks / 4;
+        if (splits > 1) {
+            grid.z = (unsigned)splits;
+            if (!zeroed) {
+                const cudaError_t x = cudaMemset2DAsync(e.C, (size_t)e.ldc * sizeof(float), 0,
+                                                        (size_t)N * sizeof(float), (size_t)M, s);
+                if (x != cudaSuccess) return cuda_status(x, "mlp_gemm_tc clear");
+            }
+        }
+    }
+    kernel<<<grid, tp::kGtThreads, tp::kGtSmemBytes, s>>>(K, gt_operand(A, lda, M, ta), gt_operand(B, ldb, N, tb), e,
+                                                          err);
+    return cuda_status(cudaGetLastError(), "mlp_gemm_tc launch");
+}
+
 int tp_mlp_gemm_tc(int M, int N, int K, const float *A, int lda, int trans_a, const float *B, int ldb, int trans_b,
                    float beta, float *C, int ldc, const float *bias, float *z, int ldz, int *err, tp_stream_t stream)
 {
@@ -816,32 +861,77 @@ int tp_mlp_gemm_tc(int M, int N, int K, const float *A, int lda, int trans_a, co
     if (lda < (trans_a ? M : K) || ldb < (trans_b ? K : N) || ldc < N || (z && ldz < N))
         return fail(TP_ERR_ARG, "gemm leading dimension too small");
     if ((M + tp::kGtM - 1) / tp::kGtM > 65535) return fail(TP_ERR_ARG, "gemm M %d too large", M);
-    int rc;
-    if ((rc = set_smem_once(g_gemm_tc_attr, (const void *)tp::k_gemm_tc, tp::kGtSmemBytes,
-                            "cudaFuncSetAttribute(k_gemm_tc)")))
+    const tp::GtEpilogue e{beta, C, ldc, bias, z, ldz, 0, nullptr};
+    return gemm_tc_launch(M, N, K, A, lda, trans_a, B, ldb, trans_b, e, false, err, (cudaStream_t)stream);
+}
+
+/* the network of the learned residual (tp_mlp_infer_tc's) */
+enum { kNetIn = 1350, kNetH1 = 256, kNetH2 = 128 };
+
+int tp_mlp_forward(int rows, const float *x, int ldx, const float *const *params, float *z1, float *h1, float *z2,
+                   float *h2, float *out, int *err, tp_stream_t stream)
+{
+    if (rows < 0 || ldx < kNetIn) return fail(TP_ERR_ARG, "mlp_forward rows %d ldx %d", rows, ldx);
+    if (!rows) return TP_OK;
+    if (!x || !params || !z1 || !h1 || !z2 || !h2 || !out) return fail(TP_ERR_ARG, "NULL mlp_forward operand");
+    for (int i = 0; i < 6; i++)
+        if (!params[i]) return fail(TP_ERR_ARG, "NULL mlp_forward parameter %d", i);
+    if ((reinterpret_cast<uintptr_t>(h2) & 15) || (reinterpret_cast<uintptr_t>(out) & 7))
+        return fail(TP_ERR_ARG, "h2 / out must be 16- / 8-byte aligned");
+    if ((rows + tp::kGtM - 1) / tp::kGtM > 65535) return fail(TP_ERR_ARG, "mlp_forward rows %d too large", rows);
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc, sms;
+    if ((rc = gemm_tc_launch(rows, kNetH1, kNetIn, x, ldx, 0, params[0], kNetH1, 0,
+                             tp::GtEpilogue{0.0f, h1, kNetH1, params[1], z1, kNetH1, 0, nullptr}, false, err, s)))
         return rc;
-    int sms;
+    if ((rc = gemm_tc_launch(rows, kNetH2, kNetH1, h1, kNetH1, 0, params[2], kNetH2, 0,
+                             tp::GtEpilogue{0.0f, h2, kNetH2, params[3], z2, kNetH2, 0, nullptr}, false, err, s)))
+        return rc;
     if ((rc = sm_count(&sms))) return rc;
-    dim3 grid((unsigned)((N + tp::kGtN - 1) / tp::kGtN), (unsigned)((M + tp::kGtM - 1) / tp::kGtM), 1);
-    /* A plain product (no bias, beta 0, no GELU) with fewer tiles than SMs and
-     * a long K (the weight gradients: K = the batch) splits K over up to
-     * 2 x SMs CTAs, each adding its partial sums into C, zeroed first (the
-     * order of those few additions per element is not fixed). */
-    const long long tiles = (long long)grid.x * grid.y;
-    const int chunks = (K + tp::kGtK - 1) / tp::kGtK;
-    if (!bias && !z && beta == 0.0f && tiles < sms && chunks >= 8) {
-        long long splits = (2LL * sms + tiles - 1) / tiles;
-        if (splits > chunks / 4) splits = chunks / 4;
-        if (splits > 1) {
-            grid.z = (unsigned)splits;
-            const cudaError_t e = cudaMemset2DAsync(C, (size_t)ldc * sizeof(float), 0, (size_t)N * sizeof(float),
-                                                    (size_t)M, (cudaStream_t)stream);
-            if (e != cudaSuccess) return cuda_status(e, "mlp_gemm_tc clear");
-        }
+    tp::k_head_forward<<<grid_for(rows, 8, sms, 8), 256, 0, s>>>(rows, h2, params[4], params[5], out);
+    return cuda_status(cudaGetLastError(), "mlp_forward launch");
+}
+
+int tp_mlp_loss_backward(int rows, const float *x, int ldx, const float *const *params, const float *z1,
+                         const float *h1, const float *z2, const float *h2, const float *out, const float *target,
+                         const float *w, float inv_count, float *dout, float *loss_rows, double *loss_sum, float *dz2,
+                         float *dz1, float *const *grads, int *err, tp_stream_t stream)
+{
+    if (rows < 0 || ldx < kNetIn) return fail(TP_ERR_ARG, "mlp_loss_backward rows %d ldx %d", rows, ldx);
+    if (!x || !params || !z1 || !h1 || !z2 || !h2 || !out || !target || !dout || !loss_rows || !loss_sum || !dz2 ||
+        !dz1 || !grads)
+        return fail(TP_ERR_ARG, "NULL mlp_loss_backward operand");
+    for (int i = 0; i < 6; i++)
+        if (!params[i] || !grads[i]) return fail(TP_ERR_ARG, "NULL mlp_loss_backward parameter %d", i);
+    if ((reinterpret_cast<uintptr_t>(dout) & 7) || (reinterpret_cast<uintptr_t>(loss_sum) & 7))
+        return fail(TP_ERR_ARG, "dout / loss_sum must be 8-byte aligned");
+    if ((rows + tp::kGtM - 1) / tp::kGtM > 65535) return fail(TP_ERR_ARG, "mlp_loss_backward rows %d too large", rows);
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc, sms;
+    if ((rc = sm_count(&sms))) return rc;
+    tp::TensorSet g{};
+    static const long long kSizes[6] = {kNetIn * kNetH1, kNetH1, kNetH1 * kNetH2, kNetH2, kNetH2 * 2, 2};
+    for (int i = 0; i < 6; i++) {
+        g.p[i] = grads[i];
+        g.n[i] = kSizes[i];
     }
-    tp::k_gemm_tc<<<grid, 128, tp::kGtSmemBytes, (cudaStream_t)stream>>>(M, N, K, A, lda, trans_a, B, ldb, trans_b,
-                                                                       beta, C, ldc, bias, z, ldz, err);
-    return cuda_status(cudaGetLastError(), "mlp_gemm_tc launch");
+    g.count = 6;
+    tp::k_zero_set<<<sms * 4, 256, 0, s>>>(g, loss_sum);
+    if (rows == 0) return cuda_status(cudaGetLastError(), "mlp_loss_backward launch");
+    tp::k_head_backward<<<(rows + tp::kHeadRows - 1) / tp::kHeadRows, 128, 0, s>>>(
+        rows, out, target, w, inv_count, h2, z2, params[4], dout, loss_rows, dz2, loss_sum, grads[4], grads[5],
+        grads[3]);
+    if ((rc = cuda_status(cudaGetLastError(), "mlp_loss_backward launch"))) return rc;
+    /* dz1 = (dz2 W2^T) gelu'(z1), its column sums the gradient of b1 */
+    if ((rc = gemm_tc_launch(rows, kNetH1, kNetH2, dz2, kNetH2, 0, params[2], kNetH2, 1,
+                             tp::GtEpilogue{0.0f, dz1, kNetH1, nullptr, const_cast<float *>(z1), kNetH1, 1, grads[1]},
+                             false, err, s)))
+        return rc;
+    if ((rc = gemm_tc_launch(kNetH1, kNetH2, rows, h1, kNetH1, 1, dz2, kNetH2, 0,
+                             tp::GtEpilogue{0.0f, grads[2], kNetH2, nullptr, nullptr, 0, 0, nullptr}, true, err, s)))
+        return rc;
+    return gemm_tc_launch(kNetIn, kNetH1, rows, x, ldx, 1, dz1, kNetH1, 0,
+                          tp::GtEpilogue{0.0f, grads[0], kNetH1, nullptr, nullptr, 0, 0, nullptr}, true, err, s);
 }
 
 int tp_mlp_gelu_backward(int rows, int cols, int ld, const float *z, const float *dh, float *dz, tp_stream_t stream)
@@ -949,6 +1039,35 @@ int tp_mlp_adam(size_t n, float *param, const float *grad, float *m, float *v, f
     tp::k_adam<<<grid_for((long long)n, 256, sms, 8), 256, 0, (cudaStream_t)stream>>>((long long)n, param, grad, m, v,
                                                                                    lr, beta1, beta2, eps, c1, c2);
     return cuda_status(cudaGetLastError(), "mlp_adam launch");
+}
+
+int tp_mlp_adam_set(int count, const size_t *n, float *const *param, const float *const *grad, float *const *m,
+                    float *const *v, float lr, float beta1, float beta2, float eps, int step, tp_stream_t stream)
+{
+    if (step < 1) return fail(TP_ERR_ARG, "adam step %d < 1", step);
+    if (count < 0 || count > tp::kTensors) return fail(TP_ERR_ARG, "adam on %d arrays (at most %d)", count, tp::kTensors);
+    if (!count) return TP_OK;
+    if (!n || !param || !grad || !m || !v) return fail(TP_ERR_ARG, "NULL adam operand");
+    tp::TensorSet sets[4] = {};
+    size_t most = 0;
+    for (int i = 0; i < count; i++) {
+        if (n[i] && (!param[i] || !grad[i] || !m[i] || !v[i])) return fail(TP_ERR_ARG, "NULL adam operand %d", i);
+        sets[0].p[i] = param[i];
+        sets[1].p[i] = const_cast<float *>(grad[i]);
+        sets[2].p[i] = m[i];
+        sets[3].p[i] = v[i];
+        for (int k = 0; k < 4; k++) sets[k].n[i] = (long long)n[i];
+        most = n[i] > most ? n[i] : most;
+    }
+    for (int k = 0; k < 4; k++) sets[k].count = count;
+    if (!most) return TP_OK;
+    int sms, rc;
+    if ((rc = sm_count(&sms))) return rc;
+    const float c1 = (float)(1.0 / (1.0 - pow((double)beta1, step)));
+    const float c2 = (float)(1.0 / (1.0 - pow((double)beta2, step)));
+    tp::k_adam_set<<<grid_for((long long)most, 256, sms, 8), 256, 0, (cudaStream_t)stream>>>(
+        sets[0], sets[1], sets[2], sets[3], lr, beta1, beta2, eps, c1, c2);
+    return cuda_status(cudaGetLastError(), "mlp_adam_set launch");
 }
 
 int tp_psf_to_clt(const float *psf, size_t n, float *clt_kernels, tp_stream_t stream)

@@ -11,23 +11,37 @@
  * times a product) loses about 1e-5 of the result, the per-chunk sums stay
  * within 2e-6.
  *
- * One CTA of 128 threads per 128 x 64 tile of C; K in chunks of 32.  Every
- * thread loads its share of the chunk's op(A) (128 x 32) and op(B) (64 x 32)
- * from global memory in whichever order is contiguous for the operand's
- * transpose, splits it and stores both parts as K-major 128-byte-swizzled
- * images (rows of 32 TF32 values, the 16-byte chunk index XOR the row's low
- * three bits); after a barrier thread 0 issues the chunk's 12 MMAs (four K
- * steps of 8) into the chunk's tensor-memory buffer (two, by chunk parity)
- * and commits them to the stage's mbarrier.  Two stages: the threads fill one
- * while the tensor cores read the other; before overwriting a stage they wait
- * (bounded) for the MMAs of chunk c - 2, read that chunk's 64 columns of
- * their own lane (warp w: lanes 32 w .. 32 w + 31, one row of C per thread)
- * with tcgen05.ld and add them into 64 registers.  The epilogue applies bias,
- * beta C and GELU to the registers.
- * A wait that runs out sets *err, drains the issued MMAs (one more bounded
- * wait), frees the tensor memory and leaves C unwritten.
+ * One CTA per 128 x 64 tile of C (and K range), K in chunks of 32, 17 warps in
+ * three roles around four stages of shared memory and of tensor memory:
+ *   producers (eight warps): unit = one row's four consecutive K values, loaded
+ *     in the order that is contiguous for the operand's transpose (16- or
+ *     8-byte loads where the rows allow them, two chunks ahead), split, and
+ *     stored as one 16-byte piece each of the hi and the lo K-major
+ *     128-byte-swizzled image (rows of 32 values, the piece index XOR the row's
+ *     low three bits: conflict-free in either order); they arrive on full[s];
+ *   the MMA warp: one thread waits for full[s] and for the stage's accumulator,
+ *     issues the chunk's 12 MMAs (four K steps of 8) and commits them to
+ *     done[s], which frees the images and hands over the accumulator;
+ *   gather (eight warps, half a row of C per thread): add the chunk's 32 columns
+ *     into 32 registers, one tensor-memory load and wait a chunk, and release
+ *     the accumulator (accfree[s]).
+ * At the end the tile goes through shared memory and all warps apply bias,
+ * beta C, GELU, or (dgelu) the factor gelu'(z), row by row.
+ * What bounds it is shared memory: a chunk's split images are 48 KB written and
+ * 72 KB read by the MMAs (N = 64 reads A once per MMA), beside about 10 us of
+ * launch, first loads and epilogue.  The earlier form did every step of a chunk
+ * in turn with four warps, and GELU on one row per thread: layer 1's forward
+ * product at 4096 rows (4096 x 256 x 1350) took 230 us (ncu, cold cache) and now
+ * 55 (44 warm), its weight gradient 160 and now 51.  Tried without gain:
+ * sixteen producer warps, four chunks in flight (spills), two producer groups
+ * on alternate chunks.
+ *
+ * Every wait is bounded; one that runs out raises the CTA's abort flag, every
+ * role leaves its loop, the issued MMAs are drained (one more bounded wait),
+ * the tensor memory is freed, *err is set and C is left unwritten.
  */
 #pragma once
+#include "tp_tc_engine.cuh"
 #include "tp_tcgen05.cuh"
 
 namespace tp {
@@ -36,49 +50,147 @@ constexpr int kGtM = 128, kGtN = 64, kGtK = 32;
 constexpr int kGtABytes = kGtM * kGtK * 4; /* one TF32 part of the A chunk: 16 KB */
 constexpr int kGtBBytes = kGtN * kGtK * 4; /* one TF32 part of the B chunk: 8 KB  */
 constexpr int kGtStageBytes = 2 * kGtABytes + 2 * kGtBBytes;
-constexpr int kGtStages = 2;
+constexpr int kGtStages = 4;
+constexpr int kGtProdWarps = 8, kGtProd = 32 * kGtProdWarps;
+constexpr int kGtGatherWarps = 8;
+constexpr int kGtThreads = 32 * (kGtGatherWarps + 1 + kGtProdWarps);
 constexpr size_t kGtSmemBytes = (size_t)kGtStages * kGtStageBytes + 1024; /* + alignment of the swizzle atoms */
 static_assert(kGtABytes % 1024 == 0 && kGtBBytes % 1024 == 0, "images start on 1024-byte swizzle atoms");
+static_assert(kGtStages * kGtN <= 512, "an accumulator per stage");
 
-/* byte offset of element (row r, k) in a K-major image with 128-byte rows and
- * the 128-byte swizzle */
-__device__ __forceinline__ uint32_t gt_sw_off(int r, int k)
+/* An operand of the GEMM as a rows x K matrix: element (r, k) at p[r * ld + k],
+ * or p[k * ld + r] when `across`.  vec: floats of a row that one load may take
+ * (4, 2 or 1; 1 when across). */
+struct GtOperand {
+    const float *p;
+    int ld, rows, across, vec;
+};
+
+/* What happens to the finished tile.  dgelu: C = acc * gelu'(z), and colsum[n]
+ * += the column sums of C; else C = beta C + acc + bias, with z (if given) that
+ * value and C = gelu of it. */
+struct GtEpilogue {
+    float beta;
+    float *C;
+    int ldc;
+    const float *bias;
+    float *z;
+    int ldz;
+    int dgelu;
+    float *colsum;
+};
+
+/* A producer thread's N units of an operand: row r, K values 4q .. 4q + 3 of
+ * each chunk, r and q from the thread's and the unit's number in the order that
+ * is contiguous in memory.  Rows past the operand's last read that row again
+ * (they end in rows or columns of the tile that nobody stores); K past the end
+ * gives zeros.  Chunks are loaded one after another (load moves on). */
+template <bool ACROSS, int ROWS, int N>
+struct GtUnits {
+    const float *p[N]; /* the unit's first value of the next chunk */
+    uint32_t off[N];   /* its piece in an image */
+    int ld;
+    __device__ __forceinline__ static int row(int t, int u) { return ACROSS ? (t + kGtProd * u) % ROWS : (t + kGtProd * u) >> 3; }
+    __device__ __forceinline__ static int piece(int t, int u) { return ACROSS ? (t + kGtProd * u) / ROWS : t & 7; }
+    __device__ __forceinline__ GtUnits(const GtOperand &o, int r0, int k0, int t) : ld(o.ld)
+    {
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            const int r = row(t, u), q = piece(t, u);
+            const size_t m = (size_t)min(r0 + r, o.rows - 1), k = (size_t)(k0 + 4 * q);
+            p[u] = o.p + (ACROSS ? k * o.ld + m : m * o.ld + k);
+            off[u] = (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4));
+        }
+    }
+    /* the next chunk, which starts at k0 and (left >= 32) lies inside K or has
+     * `left` values left */
+    __device__ __forceinline__ void load(int vec, int left, int t, float v[N][4])
+    {
+        if (left < kGtK) {
+#pragma unroll
+            for (int u = 0; u < N; u++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    v[u][j] = 4 * piece(t, u) + j < left ? __ldg(p[u] + (ACROSS ? (size_t)j * ld : (size_t)j)) : 0.0f;
+        } else if (ACROSS) {
+#pragma unroll
+            for (int u = 0; u < N; u++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) v[u][j] = __ldg(p[u] + (size_t)j * ld);
+        } else if (vec == 4) {
+#pragma unroll
+            for (int u = 0; u < N; u++) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(p[u]));
+                v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+            }
+        } else if (vec == 2) {
+#pragma unroll
+            for (int u = 0; u < N; u++) {
+                const float2 x = __ldg(reinterpret_cast<const float2 *>(p[u]));
+                const float2 y = __ldg(reinterpret_cast<const float2 *>(p[u]) + 1);
+                v[u][0] = x.x; v[u][1] = x.y; v[u][2] = y.x; v[u][3] = y.y;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < N; u++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) v[u][j] = __ldg(p[u] + j);
+        }
+#pragma unroll
+        for (int u = 0; u < N; u++) p[u] += ACROSS ? (size_t)kGtK * ld : (size_t)kGtK;
+    }
+};
+
+/* Four K values as a hi and a lo piece.  hi is x rounded to TF32 (to nearest,
+ * ties away, as cvt.rna.tf32, which takes four integer operations a value): the
+ * bits plus half a TF32 ulp, truncated.  A NaN whose payload that carry would
+ * turn into a zero still reaches the result through lo = x - hi.  lo, a
+ * multiple of x's ulp below 2^12 of them, is stored as it is: the tensor core
+ * reads its upper 11 bits, which drops at most the one ulp that rounding it
+ * would move it by. */
+__device__ __forceinline__ void gt_put4(unsigned char *hi, unsigned char *lo, const float v[4])
 {
-    return (uint32_t)(r * 128 + ((((k >> 2) ^ (r & 7)) & 7) << 4) + (k & 3) * 4);
+    float h[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) h[i] = __uint_as_float((__float_as_uint(v[i]) + 0x1000u) & 0xffffe000u);
+    *reinterpret_cast<float4 *>(hi) = make_float4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<float4 *>(lo) = make_float4(v[0] - h[0], v[1] - h[1], v[2] - h[2], v[3] - h[3]);
 }
 
-__device__ __forceinline__ void gt_put(unsigned char *hi_img, unsigned char *lo_img, uint32_t off, float v)
-{
-    const float h = to_tf32(v);
-    *reinterpret_cast<float *>(hi_img + off) = h;
-    *reinterpret_cast<float *>(lo_img + off) = to_tf32(v - h);
-}
-
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(int M, int N, int K, const float *__restrict__ A, int lda,
-                                                    int ta, const float *__restrict__ B, int ldb, int tb, float beta,
-                                                    float *__restrict__ C, int ldc, const float *__restrict__ bias,
-                                                    float *__restrict__ z, int ldz, int *__restrict__ err)
+/* TA, TB: the operands' `across` */
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(int K, GtOperand A, GtOperand B, GtEpilogue e,
+                                                           int *__restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char gt_smem[];
-    __shared__ __align__(8) uint64_t bars[kGtStages + 2]; /* MMA done per stage, (unused), drain */
+    enum { kFull = 0, kDone = kGtStages, kAccFree = 2 * kGtStages, kDrain = 3 * kGtStages, kBars };
+    __shared__ __align__(8) uint64_t bars[kBars];
     __shared__ uint32_t tmem_slot;
+    __shared__ int flag_store; /* abort */
+    volatile int *abort_flag = &flag_store;
     const uint32_t base_s = (uint32_t)__cvta_generic_to_shared(gt_smem);
     const uint32_t pad = (1024 - (base_s & 1023)) & 1023;
     unsigned char *sm = gt_smem + pad;
     const uint32_t a_sm = base_s + pad;
     const uint32_t a_bar = (uint32_t)__cvta_generic_to_shared(bars);
+    auto bar = [&](int b) { return a_bar + 8u * (uint32_t)b; };
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * kGtM, n0 = blockIdx.x * kGtN;
+    const bool gather = warp < kGtGatherWarps, issuer = tid == 32 * kGtGatherWarps;
+    constexpr int kHalf = kGtN / 2; /* columns of a gather warp: half warp / 4 of lanes 32 (warp % 4) .. */
 
-    if (tid == 0) {
-        for (int b = 0; b < kGtStages + 2; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a_bar + 8 * b) : "memory");
+    if (issuer) {
+        for (int b = 0; b < kBars; b++) {
+            const uint32_t count = b < kDone ? (uint32_t)kGtProdWarps : (b >= kAccFree && b < kDrain) ? (uint32_t)kGtGatherWarps : 1u;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar(b)), "r"(count) : "memory");
+        }
+        *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
+    if (warp == kGtGatherWarps) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          (uint32_t)__cvta_generic_to_shared(&tmem_slot)),
-                     "n"(2 * kGtN)
+                     "n"(kGtStages * kGtN)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -86,168 +198,284 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(int M, int N, int K, const f
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc_idesc(kGtM, kGtN, 2u);
     /* this CTA's chunks: the K range blockIdx.z of gridDim.z (several only
-     * for a plain product into a zeroed C, see tp_mlp_gemm_tc) */
+     * for a plain product into a zeroed C, see gemm_tc_launch) */
     const int nch = (K + kGtK - 1) / kGtK;
     const int per = (nch + (int)gridDim.z - 1) / (int)gridDim.z;
     const int c_begin = min(nch, (int)blockIdx.z * per);
     const int nloc = min(nch, c_begin + per) - c_begin;
+    bool issued = false; /* issuer: MMAs in flight or done */
+    float acc[kHalf];    /* gather: this thread's half row of the tile */
 
-    auto stage_ptr = [&](int s) { return sm + (size_t)s * kGtStageBytes; };
-    auto stage_addr = [&](int s) { return a_sm + (uint32_t)(s * kGtStageBytes); };
-    /* One chunk of op(A) and op(B): load (all of this thread's 48 values in
-     * flight at once) into registers, then split them into stage s.  The
-     * loop below loads chunk c + 1 right after storing chunk c, so the loads'
-     * latency overlaps the barrier, the MMA issue and the next chunk's wait. */
-    constexpr int kAE = kGtM * kGtK / 128, kBE = kGtN * kGtK / 128;
-    auto a_rk = [&](int i, int *r, int *k) {
-        const int e = tid + 128 * i; /* consecutive threads walk the contiguous index */
-        *r = ta ? (e & (kGtM - 1)) : (e >> 5);
-        *k = ta ? (e >> 7) : (e & 31);
-    };
-    auto b_nk = [&](int i, int *n, int *k) {
-        const int e = tid + 128 * i;
-        *n = tb ? (e >> 5) : (e & (kGtN - 1));
-        *k = tb ? (e & 31) : (e >> 6);
-    };
-    auto load_chunk = [&](int c, float ra[kAE], float rb[kBE]) {
-        const int k0 = c * kGtK;
+    if (gather) {
 #pragma unroll
-        for (int i = 0; i < kAE; i++) {
-            int r, k;
-            a_rk(i, &r, &k);
-            const int gm = m0 + r, gk = k0 + k;
-            ra[i] = (gm < M && gk < K) ? (ta ? __ldg(A + (size_t)gk * lda + gm) : __ldg(A + (size_t)gm * lda + gk))
-                                       : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < kBE; i++) {
-            int n, k;
-            b_nk(i, &n, &k);
-            const int gn = n0 + n, gk = k0 + k;
-            rb[i] = (gn < N && gk < K) ? (tb ? __ldg(B + (size_t)gn * ldb + gk) : __ldg(B + (size_t)gk * ldb + gn))
-                                       : 0.0f;
-        }
-    };
-    auto store_chunk = [&](int s, const float ra[kAE], const float rb[kBE]) {
-        unsigned char *ahi = stage_ptr(s), *alo = ahi + kGtABytes;
-        unsigned char *bhi = alo + kGtABytes, *blo = bhi + kGtBBytes;
-#pragma unroll
-        for (int i = 0; i < kAE; i++) {
-            int r, k;
-            a_rk(i, &r, &k);
-            gt_put(ahi, alo, gt_sw_off(r, k), ra[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kBE; i++) {
-            int n, k;
-            b_nk(i, &n, &k);
-            gt_put(bhi, blo, gt_sw_off(n, k), rb[i]);
-        }
-    };
-
-    bool ok = true, failed = false;
-    bool issued = false; /* thread 0: MMAs issued */
-    float acc[kGtN];     /* this thread's row of the tile: the sum of the chunks read so far */
-#pragma unroll
-    for (int i = 0; i < kGtN; i++) acc[i] = 0.0f;
-    const uint32_t t_lane = (uint32_t)(warp * 32) << 16;
-    /* local chunk c's partial sums (buffer c & 1) into acc; its MMAs have completed */
-    auto gather = [&](int c) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int c0 = 0; c0 < kGtN; c0 += 32) {
-            float v[32];
-            tc_ld32(tmem + t_lane + (uint32_t)((c & 1) * kGtN + c0), v);
-#pragma unroll
-            for (int i = 0; i < 32; i++) acc[c0 + i] += v[i];
-        }
-    };
-    float ra[kAE], rb[kBE];
-    if (nloc > 0) load_chunk(c_begin, ra, rb);
-    for (int i = 0; i < nloc; i++) {
-        const int s = i & 1;
-        /* the MMAs of local chunk i - 2 have read stage s and filled buffer s */
-        if (i >= 2 && ok) ok = tc_wait(a_bar + 8u * s, (uint32_t)(((i - 2) >> 1) & 1));
-        if (!__syncthreads_and(ok ? 1 : 0)) {
-            failed = true;
-            break;
-        }
-        if (i >= 2) gather(i - 2);
-        store_chunk(s, ra, rb);
-        if (i + 1 < nloc) load_chunk(c_begin + i + 1, ra, rb);
-        /* the generic-proxy stores visible to the tensor cores' reads, and
-         * this thread's reads of buffer s ordered before the next MMAs */
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        for (int i = 0; i < kHalf; i++) acc[i] = 0.0f;
+        const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * kHalf);
+        for (int i = 0; i < nloc; i++) {
+            const int s = i % kGtStages;
+            const bool ok = tc_wait_or_abort(bar(kDone + s), (uint32_t)((i / kGtStages) & 1), abort_flag);
+            if (!__all_sync(0xffffffffu, ok)) {
+                *abort_flag = 1;
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a = stage_addr(s);
-            const uint32_t ahi = a, alo = a + kGtABytes, bhi = a + 2 * kGtABytes, blo = bhi + kGtBBytes;
-            const uint32_t d = tmem + (uint32_t)(s * kGtN);
+            float v[kHalf];
+            tc_ld32(t_lane + (uint32_t)(s * kGtN), v);
 #pragma unroll
-            for (int j = 0; j < kGtK / 8; j++) {
-                const uint32_t o = 32u * j;
-                tc_mma_tf32(d, tc_desc_sw128(ahi + o), tc_desc_sw128(bhi + o), idesc, j > 0 ? 1u : 0u);
-                tc_mma_tf32(d, tc_desc_sw128(ahi + o), tc_desc_sw128(blo + o), idesc, 1u);
-                tc_mma_tf32(d, tc_desc_sw128(alo + o), tc_desc_sw128(bhi + o), idesc, 1u);
-            }
-            tc_commit(a_bar + 8u * s);
-            issued = true;
+            for (int j = 0; j < kHalf; j++) acc[j] += v[j];
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_arrive(bar(kAccFree + s));
         }
-    }
-    /* the last two chunks */
-    for (int i = nloc - 2; i < nloc && !failed; i++) {
-        if (i < 0) continue;
-        const int s = i & 1;
-        if (ok) ok = tc_wait(a_bar + 8u * s, (uint32_t)((i >> 1) & 1));
-        if (!__syncthreads_and(ok ? 1 : 0)) {
-            failed = true;
-            break;
-        }
-        gather(i);
-    }
-    if (!failed) {
-        /* epilogue: warp w holds rows m0 + 32 w .. + 31, one per lane */
-        const int gm = m0 + warp * 32 + lane;
-        /* (loops fully unrolled: acc stays in registers) */
-        if (gm < M && gridDim.z > 1) {
-            /* one of several K ranges: its partial sums into the zeroed C */
-#pragma unroll
-            for (int i = 0; i < kGtN; i++) {
-                const int gn = n0 + i;
-                if (gn < N) atomicAdd(C + (size_t)gm * ldc + gn, acc[i]);
-            }
-        } else if (gm < M) {
-#pragma unroll
-            for (int i = 0; i < kGtN; i++) {
-                const int gn = n0 + i;
-                if (gn >= N) continue;
-                float x = acc[i];
-                if (bias) x += bias[gn];
-                if (beta != 0.0f) x = __fmaf_rn(beta, C[(size_t)gm * ldc + gn], x);
-                if (z) {
-                    z[(size_t)gm * ldz + gn] = x;
-                    x = gelu_f(x);
+    } else if (warp == kGtGatherWarps) {
+        if (issuer) {
+            const uint32_t idesc = tc_idesc(kGtM, kGtN, 2u);
+            for (int i = 0; i < nloc; i++) {
+                const int s = i % kGtStages;
+                const uint32_t ph = (uint32_t)((i / kGtStages) & 1);
+                bool ok = tc_wait_or_abort(bar(kFull + s), ph, abort_flag);
+                if (ok && i >= kGtStages) ok = tc_wait_or_abort(bar(kAccFree + s), ph ^ 1u, abort_flag);
+                if (!ok) {
+                    *abort_flag = 1;
+                    break;
                 }
-                C[(size_t)gm * ldc + gn] = x;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ahi = a_sm + (uint32_t)(s * kGtStageBytes), alo = ahi + kGtABytes;
+                const uint32_t bhi = alo + kGtABytes, blo = bhi + kGtBBytes;
+                const uint32_t d = tmem + (uint32_t)(s * kGtN);
+#pragma unroll
+                for (int j = 0; j < kGtK / 8; j++) {
+                    const uint32_t o = 32u * j;
+                    tc_mma_tf32(d, tc_desc_sw128(ahi + o), tc_desc_sw128(bhi + o), idesc, j > 0 ? 1u : 0u);
+                    tc_mma_tf32(d, tc_desc_sw128(ahi + o), tc_desc_sw128(blo + o), idesc, 1u);
+                    tc_mma_tf32(d, tc_desc_sw128(alo + o), tc_desc_sw128(bhi + o), idesc, 1u);
+                }
+                tc_commit(bar(kDone + s));
+                issued = true;
             }
         }
-    } else if (tid == 0) {
-        /* MMAs issued so far complete before the tensor memory is freed */
-        if (issued) {
-            tc_commit(a_bar + 8u * (kGtStages + 1));
-            (void)tc_wait(a_bar + 8u * (kGtStages + 1), 0u);
+        __syncwarp();
+    } else {
+        const int t = tid - 32 * (kGtGatherWarps + 1);
+        constexpr int kAU = kGtM * 8 / kGtProd, kBU = kGtN * 8 / kGtProd; /* units per thread: 4 and 2 */
+        const int kc = c_begin * kGtK;
+        GtUnits<TA, kGtM, kAU> au(A, m0, kc, t);
+        GtUnits<TB, kGtN, kBU> bu(B, n0, kc, t);
+        auto load = [&](int i, float ra[kAU][4], float rb[kBU][4]) {
+            if (i >= nloc) return;
+            const int left = K - kc - i * kGtK;
+            au.load(A.vec, left, t, ra);
+            bu.load(B.vec, left, t, rb);
+        };
+        /* chunk i into its stage; false: a wait ran out */
+        auto store = [&](int i, const float ra[kAU][4], const float rb[kBU][4]) -> bool {
+            const int s = i % kGtStages;
+            if (i >= kGtStages) {
+                /* the MMAs of the stage's last chunk have read its images */
+                const bool ok = tc_wait_or_abort(bar(kDone + s), (uint32_t)((i / kGtStages - 1) & 1), abort_flag);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    *abort_flag = 1;
+                    return false;
+                }
+            }
+            unsigned char *ahi = sm + (size_t)s * kGtStageBytes, *alo = ahi + kGtABytes;
+            unsigned char *bhi = alo + kGtABytes, *blo = bhi + kGtBBytes;
+#pragma unroll
+            for (int u = 0; u < kAU; u++) gt_put4(ahi + au.off[u], alo + au.off[u], ra[u]);
+#pragma unroll
+            for (int u = 0; u < kBU; u++) gt_put4(bhi + bu.off[u], blo + bu.off[u], rb[u]);
+            /* the generic-proxy stores visible to the tensor cores' reads */
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc_arrive(bar(kFull + s));
+            return true;
+        };
+        float ra0[kAU][4], rb0[kBU][4], ra1[kAU][4], rb1[kBU][4];
+        load(0, ra0, rb0);
+        load(1, ra1, rb1);
+        for (int i = 0; i < nloc; i += 2) {
+            if (!store(i, ra0, rb0)) break;
+            load(i + 2, ra0, rb0);
+            if (i + 1 >= nloc || !store(i + 1, ra1, rb1)) break;
+            load(i + 3, ra1, rb1);
         }
-        if (err) atomicExch(err, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(2 * kGtN) : "memory");
+    const bool failed = *abort_flag != 0;
+    if (issuer && failed) {
+        /* MMAs issued so far complete before the tensor memory is freed */
+        if (issued) {
+            tc_commit(bar(kDrain));
+            (void)tc_wait(bar(kDrain), 0u);
+        }
+        if (err) atomicExch(err, 1);
+    }
+    /* the tile through shared memory (every MMA has read its stage), so that all
+     * warps share the epilogue and its accesses of C and z are whole rows */
+    float(*tile)[kGtN + 1] = reinterpret_cast<float(*)[kGtN + 1]>(sm);
+    static_assert(kGtM * (kGtN + 1) * 4 <= kGtStages * kGtStageBytes, "the tile fits the stages");
+    if (gather && !failed) {
+#pragma unroll
+        for (int i = 0; i < kHalf; i++) tile[(warp & 3) * 32 + lane][(warp >> 2) * kHalf + i] = acc[i];
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == kGtGatherWarps)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kGtStages * kGtN)
+                     : "memory");
+    if (failed) return;
+    const int mrows = min(kGtM, A.rows - m0), ncols = min(kGtN, B.rows - n0);
+#pragma unroll 2
+    for (int x = tid; x < kGtM * kGtN; x += kGtThreads) {
+        const int r = x / kGtN, n = x % kGtN;
+        if (r >= mrows || n >= ncols) continue;
+        const size_t gm = (size_t)(m0 + r), gn = (size_t)(n0 + n);
+        float *c = e.C + gm * e.ldc + gn;
+        float v = tile[r][n];
+        if (gridDim.z > 1) { /* one of several K ranges: its partial sum into the zeroed C */
+            atomicAdd(c, v);
+            continue;
+        }
+        if (e.dgelu) {
+            v *= gelu_grad_f(e.z[gm * e.ldz + gn]);
+            tile[r][n] = v;
+        } else {
+            if (e.bias) v += e.bias[gn];
+            if (e.beta != 0.0f) v = __fmaf_rn(e.beta, *c, v);
+            if (e.z) {
+                e.z[gm * e.ldz + gn] = v;
+                v = gelu_f(v);
+            }
+        }
+        *c = v;
+    }
+    if (e.dgelu && e.colsum) {
+        __syncthreads();
+        const int n = tid % kGtN;
+        float sum = 0.0f;
+        for (int r = tid / kGtN; r < mrows; r += kGtThreads / kGtN) sum += tile[r][n];
+        if (tid < kGtThreads / kGtN * kGtN && n < ncols) atomicAdd(e.colsum + n0 + n, sum);
+    }
+}
+
+/* ---- the network's head and bookkeeping ------------------------------------- */
+
+/* out[r] = h2[r] W3 + b3: a warp per row of 128, lane l the values 4l .. 4l + 3 */
+__global__ void __launch_bounds__(256) k_head_forward(int rows, const float *__restrict__ h2,
+                                                      const float *__restrict__ W3, const float *__restrict__ b3,
+                                                      float *__restrict__ out)
+{
+    const int lane = threadIdx.x & 31;
+    float w0[4], w1[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        w0[i] = __ldg(W3 + 2 * (4 * lane + i));
+        w1[i] = __ldg(W3 + 2 * (4 * lane + i) + 1);
+    }
+    const float bias0 = __ldg(b3), bias1 = __ldg(b3 + 1);
+    for (int r = blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8) {
+        const float4 h = __ldg(reinterpret_cast<const float4 *>(h2 + (size_t)r * 128) + lane);
+        float o0 = h.x * w0[0], o1 = h.x * w1[0];
+        o0 = __fmaf_rn(h.y, w0[1], o0); o1 = __fmaf_rn(h.y, w1[1], o1);
+        o0 = __fmaf_rn(h.z, w0[2], o0); o1 = __fmaf_rn(h.z, w1[2], o1);
+        o0 = __fmaf_rn(h.w, w0[3], o0); o1 = __fmaf_rn(h.w, w1[3], o1);
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            o0 += __shfl_xor_sync(0xffffffffu, o0, d);
+            o1 += __shfl_xor_sync(0xffffffffu, o1, d);
+        }
+        if (lane == 0) *reinterpret_cast<float2 *>(out + 2 * (size_t)r) = make_float2(o0 + bias0, o1 + bias1);
+    }
+}
+
+/* The loss and everything of the backward pass that is per row of the head, on
+ * kHeadRows rows a block, thread c = column c of layer 2: the loss and its
+ * gradient dout (k_nll), dz2 = (dout W3^T) gelu'(z2), and the gradients of W3,
+ * b3 and b2 and the loss sum, added into zeroed memory once per block. */
+constexpr int kHeadRows = 16;
+__global__ void __launch_bounds__(128) k_head_backward(int rows, const float *__restrict__ out,
+                                                       const float *__restrict__ target, const float *__restrict__ w,
+                                                       float inv_count, const float *__restrict__ h2,
+                                                       const float *__restrict__ z2, const float *__restrict__ W3,
+                                                       float *__restrict__ dout, float *__restrict__ loss_rows,
+                                                       float *__restrict__ dz2, double *loss_sum, float *gW3,
+                                                       float *gb3, float *gb2)
+{
+    __shared__ float s_d[kHeadRows][2];
+    const int c = threadIdx.x, r0 = blockIdx.x * kHeadRows, nr = min(kHeadRows, rows - r0);
+    if (c < 32) {
+        float loss = 0.0f, d0 = 0.0f, d1 = 0.0f;
+        if (c < nr) {
+            nll_row(r0 + c, out, target, w, inv_count, &loss, &d0, &d1);
+            loss_rows[r0 + c] = loss;
+            *reinterpret_cast<float2 *>(dout + 2 * (size_t)(r0 + c)) = make_float2(d0, d1);
+            s_d[c][0] = d0;
+            s_d[c][1] = d1;
+        }
+        double ls = (double)loss;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            ls += __shfl_xor_sync(0xffffffffu, ls, d);
+            d0 += __shfl_xor_sync(0xffffffffu, d0, d);
+            d1 += __shfl_xor_sync(0xffffffffu, d1, d);
+        }
+        if (c == 0) {
+            atomicAdd(loss_sum, ls);
+            atomicAdd(gb3, d0);
+            atomicAdd(gb3 + 1, d1);
+        }
+    }
+    __syncthreads();
+    const float w0 = __ldg(W3 + 2 * c), w1 = __ldg(W3 + 2 * c + 1);
+    float sb = 0.0f, s0 = 0.0f, s1 = 0.0f;
+    float z[kHeadRows], h[kHeadRows];
+#pragma unroll
+    for (int i = 0; i < kHeadRows; i++) {
+        const size_t o = (size_t)(r0 + min(i, nr - 1)) * 128 + c;
+        z[i] = __ldg(z2 + o);
+        h[i] = __ldg(h2 + o);
+    }
+#pragma unroll
+    for (int i = 0; i < kHeadRows; i++) {
+        if (i >= nr) break;
+        const float d0 = s_d[i][0], d1 = s_d[i][1];
+        const float g = __fmaf_rn(d1, w1, d0 * w0) * gelu_grad_f(z[i]);
+        dz2[(size_t)(r0 + i) * 128 + c] = g;
+        sb += g;
+        s0 = __fmaf_rn(h[i], d0, s0);
+        s1 = __fmaf_rn(h[i], d1, s1);
+    }
+    atomicAdd(gb2 + c, sb);
+    atomicAdd(gW3 + 2 * c, s0);
+    atomicAdd(gW3 + 2 * c + 1, s1);
+}
+
+/* up to kTensors arrays of a network in one launch */
+constexpr int kTensors = 8;
+struct TensorSet {
+    float *p[kTensors];
+    long long n[kTensors];
+    int count;
+};
+
+__global__ void __launch_bounds__(256) k_zero_set(TensorSet t, double *sum)
+{
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    if (first == 0) *sum = 0.0;
+    for (int i = 0; i < t.count; i++)
+        for (long long k = first; k < t.n[i]; k += step) t.p[i][k] = 0.0f;
+}
+
+/* k_adam on every array of a set: p, with its gradient, and its two moments */
+__global__ void __launch_bounds__(256) k_adam_set(TensorSet p, TensorSet g, TensorSet m, TensorSet v, float lr,
+                                                  float b1, float b2, float eps, float c1, float c2)
+{
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (int i = 0; i < p.count; i++)
+        for (long long k = first; k < p.n[i]; k += step) adam_element(p.p[i], g.p[i], m.p[i], v.p[i], k, lr, b1, b2, eps, c1, c2);
 }
 
 } /* namespace tp */

@@ -249,38 +249,49 @@ __global__ void __launch_bounds__(32 * kColLanes) k_colsum(int rows, int cols, i
  * gradient dout = d loss / d out for the mean over rows (weights w[r] in
  * {0, 1} select the rows that count; count = their number).  loss_rows[r]
  * receives the per-row loss. */
+__device__ __forceinline__ void nll_row(int r, const float *__restrict__ out, const float *__restrict__ target,
+                                        const float *__restrict__ w, float inv_count, float *loss, float *d_d,
+                                        float *d_s)
+{
+    const float d = out[2 * r], s = fminf(12.0f, fmaxf(-12.0f, out[2 * r + 1]));
+    const float wr = w ? w[r] : 1.0f;
+    const float e = d - target[r];
+    const float ivar = expf(-s);
+    *loss = wr * (0.5f * ivar * e * e + 0.5f * s);
+    *d_d = wr * inv_count * ivar * e;
+    const float ds = 0.5f - 0.5f * ivar * e * e;
+    const bool live = out[2 * r + 1] > -12.0f && out[2 * r + 1] < 12.0f;
+    *d_s = live ? wr * inv_count * ds : 0.0f;
+}
+
 __global__ void k_nll(int rows, const float *__restrict__ out, const float *__restrict__ target,
                       const float *__restrict__ w, float inv_count, float *__restrict__ dout,
                       float *__restrict__ loss_rows)
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
-    const float d = out[2 * r], s = fminf(12.0f, fmaxf(-12.0f, out[2 * r + 1]));
-    const float wr = w ? w[r] : 1.0f;
-    const float e = d - target[r];
-    const float ivar = expf(-s);
-    loss_rows[r] = wr * (0.5f * ivar * e * e + 0.5f * s);
-    dout[2 * r] = wr * inv_count * ivar * e;
-    const float ds = 0.5f - 0.5f * ivar * e * e;
-    const bool live = out[2 * r + 1] > -12.0f && out[2 * r + 1] < 12.0f;
-    dout[2 * r + 1] = live ? wr * inv_count * ds : 0.0f;
+    nll_row(r, out, target, w, inv_count, &loss_rows[r], &dout[2 * r], &dout[2 * r + 1]);
 }
 
 /* Adam: m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2; p -= lr mhat / (sqrt(vhat) + eps) */
+__device__ __forceinline__ void adam_element(float *__restrict__ p, const float *__restrict__ g,
+                                             float *__restrict__ m, float *__restrict__ v, long long i, float lr,
+                                             float b1, float b2, float eps, float c1, float c2)
+{
+    const float gi = g[i];
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+}
+
 __global__ void k_adam(long long n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
                        float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2)
 {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-    }
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        adam_element(p, g, m, v, i, lr, b1, b2, eps, c1, c2);
 }
-
-
 
 /* ---- inference on the tensor cores (tcgen05 + TMA) --------------------------
  *

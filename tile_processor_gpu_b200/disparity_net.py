@@ -65,6 +65,11 @@ def gemm(A, B, C, M, N, K, ta=0, tb=0, beta=0.0, bias=None, z=None, lda=None, ld
         _native.call("tp_mlp_gemm", *args, _stream(stream))
 
 
+def _pointers(tensors):
+    """host array of the tensors' device pointers"""
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
 def features(geom, corrs, corr_stride, corr_radius, num_corr, corr_indices, out, feature_stride=N_IN,
              stream=None):
     """Rows out[tile] of the tiles with correlation entries (others untouched)."""
@@ -105,7 +110,8 @@ class DisparityMLP:
             f = lambda n: torch.empty((rows, n), dtype=torch.float32, device=self.device)
             self._ws = {"rows": rows, "z1": f(N_H1), "h1": f(N_H1), "z2": f(N_H2), "h2": f(N_H2), "out": f(N_OUT),
                         "dout": f(N_OUT), "dh2": f(N_H2), "dz2": f(N_H2), "dh1": f(N_H1), "dz1": f(N_H1),
-                        "loss": torch.empty(rows, dtype=torch.float32, device=self.device)}
+                        "loss": torch.empty(rows, dtype=torch.float32, device=self.device),
+                        "loss_sum": torch.empty(1, dtype=torch.float64, device=self.device)}
         return self._ws
 
     def forward(self, x, rows, ldx=N_IN, stream=None):
@@ -113,6 +119,11 @@ class DisparityMLP:
         keeps the activations for backward."""
         w = self._work(rows)
         p = self.p
+        if self.tc:
+            _native.call("tp_mlp_forward", int(rows), _dptr(x), int(ldx), _pointers([p[k] for k in PARAMS]),
+                         _dptr(w["z1"]), _dptr(w["h1"]), _dptr(w["z2"]), _dptr(w["h2"]), _dptr(w["out"]),
+                         _dptr(self._err), _stream(stream))
+            return w["out"][:rows]
         gemm(x, p["W1"], w["h1"], rows, N_H1, N_IN, bias=p["b1"], z=w["z1"], lda=ldx,
              stream=stream, tc=self.tc, err=self._err)
         gemm(w["h1"], p["W2"], w["h2"], rows, N_H2, N_H1, bias=p["b2"], z=w["z2"],
@@ -127,6 +138,13 @@ class DisparityMLP:
         w = self._work(rows)
         p, g = self.p, self.g
         count = float(weight[:rows].sum().item()) if weight is not None else float(rows)
+        if self.tc:
+            _native.call("tp_mlp_loss_backward", int(rows), _dptr(x), int(ldx), _pointers([p[k] for k in PARAMS]),
+                         _dptr(w["z1"]), _dptr(w["h1"]), _dptr(w["z2"]), _dptr(w["h2"]), _dptr(w["out"]),
+                         _dptr(target), _dptr(weight), 1.0 / max(count, 1.0), _dptr(w["dout"]), _dptr(w["loss"]),
+                         _dptr(w["loss_sum"]), _dptr(w["dz2"]), _dptr(w["dz1"]),
+                         _pointers([g[k] for k in PARAMS]), _dptr(self._err), _stream(stream))
+            return float(w["loss_sum"].item()) / max(count, 1.0)
         _native.call("tp_mlp_nll", int(rows), _dptr(w["out"]), _dptr(target),
                      _dptr(weight) if weight is not None else None, 1.0 / max(count, 1.0), _dptr(w["dout"]),
                      _dptr(w["loss"]), _stream(stream))
@@ -162,10 +180,10 @@ class DisparityMLP:
 
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, stream=None):
         self.step_count += 1
-        for k in PARAMS:
-            _native.call("tp_mlp_adam", int(self.p[k].numel()), _dptr(self.p[k]), _dptr(self.g[k]),
-                         _dptr(self.m[k]), _dptr(self.v[k]), float(lr), float(beta1), float(beta2), float(eps),
-                         int(self.step_count), _stream(stream))
+        sizes = (ctypes.c_size_t * len(PARAMS))(*[self.p[k].numel() for k in PARAMS])
+        _native.call("tp_mlp_adam_set", len(PARAMS), sizes, *[_pointers([d[k] for k in PARAMS])
+                                                              for d in (self.p, self.g, self.m, self.v)],
+                     float(lr), float(beta1), float(beta2), float(eps), int(self.step_count), _stream(stream))
 
     def pack(self, stream=None):
         """W1^T in TF32 and W2^T in BF16 for the tensor-core inference (after any update)."""
