@@ -787,7 +787,7 @@ int tp_mlp_features(const tp_geometry *g, const float *corrs, size_t corr_stride
     if (feature_stride < (size_t)(6 * n2)) return fail(TP_ERR_ARG, "feature_stride %zu < %d", feature_stride, 6 * n2);
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    tp::k_mlp_features<<<grid_for((long long)num_corr_tiles, 8, sms, 8), 256, 0, (cudaStream_t)stream>>>(
+    tp::k_mlp_features<<<grid_for((long long)num_corr_tiles, 256, sms, 8), 256, 0, (cudaStream_t)stream>>>(
         gd.TX * gd.TY, corrs, corr_stride, n2, (long long)num_corr_tiles, corr_indices, features, feature_stride);
     return cuda_status(cudaGetLastError(), "mlp_features launch");
 }
@@ -1008,7 +1008,7 @@ int tp_mlp_infer_tc(int rows, const float *x, int ldx, const void *w1t, const fl
                             "cudaFuncSetAttribute(k_mlp_infer_tc)")))
         return rc;
     const int tiles = (rows + tp::kTcM - 1) / tp::kTcM;
-    tp::k_mlp_infer_tc<<<tiles < sms ? tiles : sms, 128, tp::kTcSmemBytes, (cudaStream_t)stream>>>(
+    tp::k_mlp_infer_tc<<<tiles < sms ? tiles : sms, tp::kTcThreads, tp::kTcSmemBytes, (cudaStream_t)stream>>>(
         tmap, rows, static_cast<const float *>(w1t), b1, static_cast<const __nv_bfloat16 *>(w2t), b2, W3, b3, out,
         err);
     return cuda_status(cudaGetLastError(), "mlp_infer_tc launch");
@@ -1099,7 +1099,7 @@ int tp_disparity_fit(const tp_geometry *g, const float *corrs, size_t corr_strid
     if (corr_stride < sz) return fail(TP_ERR_ARG, "corr_stride %zu < (2r+1)^2 = %zu", corr_stride, sz);
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    const unsigned grid = grid_for((long long)num_corr_tiles, 8, sms, 8);
+    const unsigned grid = grid_for((long long)num_corr_tiles, 256, sms, 8);
     tp::k_disparity_fit<<<grid, 256, 0, (cudaStream_t)stream>>>(gd.TX * gd.TY, corrs, corr_stride, corr_radius,
                                                                (long long)num_corr_tiles, corr_indices,
                                                                port_offsets, pair_mask, mode, disparity, strength);
