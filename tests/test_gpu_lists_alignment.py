@@ -172,3 +172,80 @@ def test_imclt_all_is_the_twelve_passes(native, width, height, marks, floats, pi
     api.imclt_rbg_all(g, clt, got, stride)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("count", [1, 31, 33, 1024, 8191, 8192, 8193, 12288])
+def test_texture_list_lengths(native, oracle, count):
+    """Task lists on both sides of the one-kernel rule, shuffled, some without
+    texture bits: tasks, counts and window equal the oracle's, each sub-list
+    holds the oracle's entries, on buffers that held another list before."""
+    import torch
+    from tile_processor_gpu_b200 import api, synth
+    geom = synth.geometry(1024, 768)
+    g = api.Geometry.from_dict(geom)
+    TX, TY, TYA = synth.tiles(geom)
+    rng = np.random.default_rng(count)
+    tasks = synth.tasks_grid(geom, rng)[rng.permutation(TX * TY)][:count].copy()
+    tasks["task"][rng.random(count) < 0.1] = 0x3F0
+    idx = torch.full((TX * TYA,), 0x7F, dtype=torch.int32, device="cuda")
+    counts = torch.full((8,), 5, dtype=torch.int32, device="cuda")
+    woi = torch.full((4,), -3, dtype=torch.int32, device="cuda")
+    t = api.tasks_to_device(tasks)
+    api.prepare_texture_list(g, t, count, idx, counts, woi, TX, TY)
+    torch.cuda.synchronize()
+    want_t, want_i, want_c, want_w = oracle.prepare_texture_list(geom, tasks, TX, TY)
+    assert np.array_equal(api.tasks_from_device(t)["task"], want_t["task"])
+    assert np.array_equal(woi.cpu().numpy(), want_w)
+    got_c, got_i, q = counts.cpu().numpy(), idx.cpu().numpy(), TX * (TYA >> 2)
+    assert np.array_equal(got_c, want_c)
+    for s in range(8):
+        lo = (s >> 1) * q if not s & 1 else (s >> 1) * q + q - want_c[s]
+        assert np.array_equal(np.sort(got_i[lo:lo + want_c[s]]), np.sort(want_i[lo:lo + want_c[s]])), s
+
+
+@pytest.mark.parametrize("radius", [7, 3])
+def test_disparity_runs_across_windows(native, oracle, radius):
+    """Runs that straddle the 32-entry windows the fit and the features work
+    in: tiles with one to six pairs, pair codes of other kinds between them,
+    longer runs of repeated pairs, against the oracle, in any window phase."""
+    import torch
+    from tile_processor_gpu_b200 import api, disparity_net as D, synth
+    geom = synth.geometry(256, 192)
+    g = api.Geometry.from_dict(geom)
+    tiles = 32 * 24
+    rng = np.random.default_rng(radius)
+    n2 = (2 * radius + 1) ** 2
+    for lead in (0, 1, 5):
+        codes = [(tiles - 1 << 8) | (i % 6) for i in range(lead)]
+        for tile in range(200):
+            pairs = [p for p in range(6) if rng.random() < 0.8] or [2]
+            if tile % 17 == 3:
+                pairs = pairs + [7]
+            if tile % 23 == 5:
+                pairs = [i % 6 for i in range(11 + tile % 40)]
+            codes += [(tile << 8) | p for p in pairs]
+        codes += [(tiles + 3 << 8) | 0]
+        idx = np.array(codes, np.int32)
+        co = rng.random((len(idx), n2)).astype(np.float32)
+        po = torch.from_numpy(synth.PORT_OFFSETS.reshape(-1).copy()).cuda()
+        dd, ss = (torch.full((tiles,), np.nan, device="cuda") for _ in range(2))
+        feat = torch.full((tiles, 6 * n2 + 2), -5.0, device="cuda")
+        dco, didx = torch.from_numpy(co).cuda(), torch.from_numpy(idx).cuda()
+        api.disparity_fit(g, dco, n2, radius, len(idx), didx, po, dd, ss)
+        D.features(g, dco, n2, radius, len(idx), didx, feat, feature_stride=6 * n2 + 2)
+        torch.cuda.synchronize()
+        want_d, want_s = oracle.disparity_fit(geom, co, idx, radius)
+        got_d, got_s = dd.cpu().numpy(), ss.cpu().numpy()
+        assert np.array_equal(np.isnan(got_d), np.isnan(want_d))
+        ok = ~np.isnan(want_d)
+        assert np.max(np.abs(got_d[ok] - want_d[ok])) < 1e-4 and np.max(np.abs(got_s[ok] - want_s[ok])) < 1e-5
+        got = feat.cpu().numpy()
+        for tile in list(range(200)) + [tiles - 1]:
+            run = [(e, c & 0xFF) for e, c in enumerate(codes) if c >> 8 == tile and (c & 0xFF) < 6]
+            row = np.zeros(6 * n2, np.float64)
+            for e, p in run:
+                row[p * n2:(p + 1) * n2] = co[e]
+            if run:
+                row /= max(np.abs(co[e]).max() for e, _ in run)
+                assert np.max(np.abs(got[tile, :6 * n2] - row)) < 1e-6, tile
+        assert np.all(got[:, 6 * n2:] == -5.0) and np.all(got[200:tiles - 1] == -5.0)

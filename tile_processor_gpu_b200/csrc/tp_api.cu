@@ -501,6 +501,10 @@ static cudaError_t launch_chained(bool dependent, dim3 grid, dim3 block, size_t 
 }
 } /* extern "C++" */
 
+/* task lists up to this length are listed by one kernel on one cluster (one task
+ * per thread and turn), longer ones by a chain of five kernels on all SMs */
+constexpr int kListOneKernel = 8192;
+
 /* prepare_texture_list listing only tiles of rows [row_first, row_last) */
 static int prepare_list(const tp_geometry *g, tp_task *tasks, int num_tiles, int *texture_indices,
                         int *num_texture_tiles, int *woi, int width, int height, int row_first, int row_last,
@@ -516,33 +520,32 @@ static int prepare_list(const tp_geometry *g, tp_task *tasks, int num_tiles, int
         return fail(TP_ERR_ARG, "list extent %dx%d outside %dx%d tiles", width, height, gd.TX, gd.TY);
     cudaStream_t s = (cudaStream_t)stream;
     const long long cap = (long long)gd.TX * gd.TYA;
-    /* the first kernel is an ordinary launch (it follows the caller's work);
-     * each later one is a programmatic dependent of the one before, which it
-     * waits for on entry (chain_entry) */
-    bool dep = false;
-    cudaError_t err = cudaSuccess;
-    if (height > 0) {
-        dim3 b0((width + 1 + 255) / 256, height, 1);
-        err = launch_chained(dep, b0, 256, 0, s, tp::k_clear_texture_list, texture_indices, width, height, gd.TX,
-                             cap);
-        dep = true;
+    const int quarter = gd.TX * (gd.TYA >> 2);
+    /* the first kernel is an ordinary launch: it follows the caller's work; each
+     * later one is a programmatic dependent of the one before, which it waits
+     * for on entry (chain_entry) */
+    cudaError_t err;
+    if (num_tiles <= kListOneKernel) {
+        err = launch_chained(false, tp::kListCtas, tp::kListThreads, 0, s, tp::k_texture_list, tasks, num_tiles,
+                             texture_indices, num_texture_tiles, woi, width, height, gd.TX, gd.TY, quarter, cap,
+                             row_first, row_last);
+    } else {
+        const unsigned bt = (unsigned)((num_tiles + 255) / 256);
+        const dim3 b0((width + 1 + 255) / 256, height > 0 ? height : 1, 1);
+        err = launch_chained(false, b0, 256, 0, s, tp::k_clear_texture_list, texture_indices, woi, num_texture_tiles,
+                             width, height, gd.TX, gd.TY, cap);
+        if (err == cudaSuccess)
+            err = launch_chained(true, bt, 256, 0, s, tp::k_mark_texture_tiles, (const tp_task *)tasks, num_tiles,
+                                 texture_indices, gd.TX, cap);
+        if (err == cudaSuccess)
+            err = launch_chained(true, bt, 256, 0, s, tp::k_mark_neighbor_tiles, tasks, num_tiles,
+                                 (const int *)texture_indices, woi, gd.TX, gd.TY, cap);
+        if (err == cudaSuccess)
+            err = launch_chained(true, bt, 256, 0, s, tp::k_gen_texture_list, (const tp_task *)tasks, num_tiles,
+                                 texture_indices, num_texture_tiles, (const int *)woi, gd.TX, quarter, cap, row_first,
+                                 row_last);
+        if (err == cudaSuccess) err = launch_chained(true, 1, 32, 0, s, tp::k_woi_finalize, woi);
     }
-    const unsigned bt = (unsigned)((num_tiles + 255) / 256);
-    if (bt && err == cudaSuccess) {
-        err = launch_chained(dep, bt, 256, 0, s, tp::k_mark_texture_tiles, (const tp_task *)tasks, num_tiles,
-                             texture_indices, gd.TX, cap);
-        dep = true;
-    }
-    if (err == cudaSuccess)
-        err = launch_chained(dep, 1, 32, 0, s, tp::k_woi_init, woi, num_texture_tiles, gd.TX, gd.TY);
-    if (bt && err == cudaSuccess)
-        err = launch_chained(true, bt, 256, 0, s, tp::k_mark_neighbor_tiles, tasks, num_tiles,
-                             (const int *)texture_indices, woi, gd.TX, gd.TY, cap);
-    if (bt && err == cudaSuccess)
-        err = launch_chained(true, bt, 256, 0, s, tp::k_gen_texture_list, (const tp_task *)tasks, num_tiles,
-                             texture_indices, num_texture_tiles, (const int *)woi, gd.TX, gd.TX * (gd.TYA >> 2),
-                             cap, row_first, row_last);
-    if (err == cudaSuccess) err = launch_chained(true, 1, 32, 0, s, tp::k_woi_finalize, woi);
     if (err != cudaSuccess) return cuda_status(err, "prepare_texture_list launch");
     return cuda_status(cudaGetLastError(), "prepare_texture_list launch");
 }
