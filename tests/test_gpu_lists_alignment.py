@@ -249,3 +249,36 @@ def test_disparity_runs_across_windows(native, oracle, radius):
                 row /= max(np.abs(co[e]).max() for e, _ in run)
                 assert np.max(np.abs(got[tile, :6 * n2] - row)) < 1e-6, tile
         assert np.all(got[:, 6 * n2:] == -5.0) and np.all(got[200:tiles - 1] == -5.0)
+
+
+@pytest.mark.parametrize("impl", ["tc_fp16", "tc_bf16"])
+@pytest.mark.parametrize("floats", [1, 4])
+def test_tensor_core_stages_of_unaligned_buffers(native, impl, floats):
+    """The precision form on buffers off 32-byte boundaries (kernel tables, CLT,
+    tile scratch) gives the bits of aligned ones, stage by stage; entry counts
+    that leave a block of 128 rows and a warp's 32 entries part full."""
+    import gpu_runner as R
+    from cases import Case
+    from tile_processor_gpu_b200 import api
+    c = Case(128, 96, seed=35, border_mode=1)
+    fr, un = R.Frame(c), R.Frame(c)
+    for name in ("kernels", "clt"):
+        moved = _at_offset(getattr(un, name), floats)
+        setattr(un, name, moved)
+        setattr(un, "p_" + name, api.PointerArray(moved))
+    un.tile_scratch()
+    un._tiles = _at_offset(un._tiles, floats)
+    un.p_tiles = api.PointerArray(un._tiles)
+    for n in (13, c.num_tiles):
+        a, b = R.convert(fr, impl=impl, num_tiles=n), R.convert(un, impl=impl, num_tiles=n)
+        assert all(np.array_equal(a[k], b[k]) for k in range(4)), n
+    idx = c.corr_idx[:333].copy()
+    idx[7] = (3 << 8) | 6
+    idx[40] = (c.TX * c.TY + 1) << 8
+    for radius in (7, 2):
+        assert np.array_equal(R.correlate(fr, idx, impl=impl, radius=radius),
+                              R.correlate(un, idx, impl=impl, radius=radius))
+    for colors in (3, 1):
+        assert np.array_equal(R.textures_tiles(fr, c.tex_idx, keep_weights=1, impl=impl, colors=colors),
+                              R.textures_tiles(un, c.tex_idx, keep_weights=1, impl=impl, colors=colors))
+    assert api.tc_status() == 0

@@ -243,6 +243,12 @@ __device__ __forceinline__ void ld8_global(const float *p, float v[8])
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                  : "l"(p));
 }
+__device__ __forceinline__ void st8_global(float *p, const float v[8])
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
 
 /* y[k] = sum_n M[k][n] x[n] for the four 8-point transforms of the tables:
  * DCT-IV / DST-IV (KIND 0 / 1) through dct4_fast, DCT-II / DST-II (KIND 2 /

@@ -93,73 +93,6 @@ __device__ __forceinline__ JobGeometry job_geometry(const Geom &g, const float *
  * rows of 20 floats from the 16-byte boundary at or left of the corner */
 constexpr int kCvWinW = 20, kCvWinH = 16;
 
-/* The fold by rows, as the tensor-core form wants it: lane l builds DTT row l
- * of the folded, windowed Bayer samples of the job's colour (P: the cosine
- * fold; Q: the sine-windowed fold of green, zeros for red and blue), both
- * Bayer phases of green summed (src/TileProcessor.cuh:3257-3416).  (hc, hs)
- * and (vc, vs): (cos, sin)(pi s / 16) of the job's residual shifts. */
-__device__ __forceinline__ void fold_rows(const Geom &g, size_t dstride, const float *__restrict__ img,
-                                          const JobGeometry &j, int color, int l, float hc, float hs, float vc,
-                                          float vs, float P[8], float Q[8])
-{
-    const int itlx = j.itlx, itly = j.itly;
-    const int c0 = color & 1, c1 = (color >> 1) & 1;
-    const bool fast = (itlx >= 0) && (itlx < g.W - 16) && (itly >= 0) && (itly < g.H - 16);
-    const long long last = (long long)g.image_rows * (long long)dstride - 1;
-#pragma unroll
-    for (int v = 0; v < 8; v++) { P[v] = 0.0f; Q[v] = 0.0f; }
-#pragma unroll
-    for (int gp = 0; gp < 2; gp++) {
-        if (gp > c1) break;
-        const int colp = (itlx & 1) ^ (1 ^ c0 ^ c1 ^ gp);
-        const int rowp = (itly & 1) ^ (c0 ^ gp);
-        const int lr = fold_sample(l, rowp);
-        const float wv = fold_sign_c(lr) * shifted_window_lane(lr, vc, vs);
-        long long rowbase;
-        int eff_col = 0;
-        if (fast) {
-            rowbase = (long long)(itly + lr) * (long long)dstride + itlx;
-        } else if (g.border_mode == TP_BORDER_CLAMP) {
-            rowbase = (long long)pair_clamp(itly + lr, g.H) * (long long)dstride;
-        } else {
-            /* src/TileProcessor.cuh:3328-3361: columns clamped by IMG_HEIGHT/2,
-             * rows by IMG_WIDTH/2, row offset `rowp` added once */
-            const int i = (lr - rowp) >> 1;
-            int rp = min(g.W / 2 - 1, max(0, (itly >> 1) + i));
-            int cp = min(g.H / 2 - 1, max(0, itlx >> 1));
-            eff_col = (cp << 1) + (itlx & 1);
-            rowbase = (long long)(rowp + (rp << 1) + (itly & 1)) * (long long)dstride + eff_col;
-        }
-#pragma unroll
-        for (int v = 0; v < 8; v++) {
-            /* the sample's column for either Bayer phase and its window values
-             * are compile-time constants; the job's phase selects one (the
-             * groups of a warp hold jobs of either phase, so a table indexed
-             * by the run-time column would serialise their reads) */
-            constexpr float kW[16] = TP_HWIN_INIT, kWc[16] = TP_HWINC_INIT;
-            const int lc0 = fold_sample(v, 0), lc1 = fold_sample(v, 1);
-            const int lc = colp ? lc1 : lc0;
-            const float ww = colp ? kW[lc1] : kW[lc0], wwc = colp ? kWc[lc1] : kWc[lc0];
-            const float whs_raw = __fmaf_rn(ww, hc, wwc * hs);
-            float pix;
-            if (fast) {
-                pix = __ldg(img + rowbase + lc);
-            } else if (g.border_mode == TP_BORDER_CLAMP) {
-                pix = __ldg(img + rowbase + pair_clamp(itlx + lc, g.W));
-            } else {
-                long long a = rowbase + lc;
-                a = a > last ? last : (a < 0 ? 0 : a);
-                pix = __ldg(img + a);
-            }
-            const float d = pix * wv;
-            const float sgn_c = colp ? fold_sign_c(lc1) : fold_sign_c(lc0);
-            const float sgn_s = colp ? fold_sign_s(lc1) : fold_sign_s(lc0);
-            P[v] = __fmaf_rn(d, sgn_c * whs_raw, P[v]);
-            if (c1) Q[v] = __fmaf_rn(d, sgn_s * whs_raw, Q[v]);
-        }
-    }
-}
-
 /* (cos, sin) of a lane's residual-shift rotations: column l horizontally, row
  * l vertically, pi s (2l + 1) / 16.  Lane 0's are the rotations of the shifted
  * windows. */

@@ -21,6 +21,10 @@
  *     un-windowed tile T = d / (4 sin r sin c) for colour textures, the
  *     windowed M = (w_r / 2)(w_c / 2) d for mono; stored row-major [16][16]
  *     at the job's CLT offset of the tile buffer (the same layout as the CLT).
+ * Bound by the latency of its loads and stores; in 256-bit accesses a 1024x768
+ * frame takes 0.107 ms (ncu; 0.128 in 16-byte ones), and the four passes that
+ * read its tiles 0.026 ms each (0.039 before their copy into shared memory was
+ * free of bank conflicts).
  * k_textures<true> then runs the debayer and the camera fusion from those
  * tiles.
  */
@@ -35,6 +39,7 @@ struct InvTcStage {
     static constexpr int kQuads = 4, kProdWarps = 16, kEpiWarps = 8;
     static constexpr int kThreads = 32 * (kProdWarps + kEpiWarps);
     static constexpr int kMeta = 2;
+    static constexpr int kGroupBuf = 0, kWarpBuf = 0;
     static constexpr int kAStages = 1;
     Geom g;
     float *const *clt;   /* in: per camera [tiles][3][256]                  */
@@ -72,20 +77,23 @@ struct InvTcStage {
 
     template <int FMT>
     __device__ __forceinline__ void produce(long long n, int row, int l, unsigned gm, const TcA<4> &A,
-                                            uint32_t *meta) const
+                                            uint32_t *meta, float *) const
     {
         int cam, color;
         const int tile = job(n, &cam, &color);
         float x[4][8];
         if (tile >= 0) {
             const float *src = clt[cam] + ((size_t)tile * 3 + color) * 256 + l * 8;
-            const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
+            const bool al32 = !(reinterpret_cast<uintptr_t>(src) & 31), al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
             const float *lpf = d_lpf[colors > 1 ? color : 3] + l * 8;
             float f[8];
             load_row8(lpf, true, f);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                load_row8(src + q * 64, al16, x[q]);
+                if (al32)
+                    ld8_global(src + q * 64, x[q]);
+                else
+                    load_row8(src + q * 64, al16, x[q]);
 #pragma unroll
                 for (int k = 0; k < 8; k++) x[q][k] *= f[k];
             }
@@ -119,7 +127,7 @@ struct InvTcStage {
         }
     }
 
-    __device__ __forceinline__ void epilogue(long long n, uint32_t tb, const uint32_t *meta, int part) const
+    __device__ __forceinline__ void epilogue(long long n, uint32_t tb, const uint32_t *meta, int part, float *) const
     {
         int cam, color;
         (void)job(n, &cam, &color);
@@ -153,10 +161,9 @@ struct InvTcStage {
                     const float d = (n01 ? -e0 : e0) + (n23 ? -e1 : e1);
                     o[c] = d * __ldg(&fac[r * 17 + c]);
                 }
-                if (!(reinterpret_cast<uintptr_t>(dst) & 15)) {
-                    float4 *p = reinterpret_cast<float4 *>(dst + r * 16);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) p[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+                if (!(reinterpret_cast<uintptr_t>(dst) & 31)) {
+                    st8_global(dst + r * 16, o);
+                    st8_global(dst + r * 16 + 8, o + 8);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 16; c++) dst[r * 16 + c] = o[c];

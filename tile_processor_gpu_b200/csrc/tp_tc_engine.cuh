@@ -185,11 +185,13 @@ __device__ __forceinline__ void tc_producer_sync(int nthreads)
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
 }
 
-/* dynamic shared memory of k_tc_stage for a stage of Q quadrants, M
- * metadata words per row and AS A images */
-__host__ __device__ constexpr int tc_stage_smem(int Q, int M, int AS)
+/* dynamic shared memory of k_tc_stage for stage S: its A images and B tables,
+ * two buffers of metadata, a buffer per producer group and per epilogue warp */
+template <class S>
+__host__ __device__ constexpr int tc_stage_smem()
 {
-    return 1024 + AS * 2 * Q * kTcQuadBytes + 2 * Q * kTcBQuadBytes + 2 * kTcRows * M * 4 + 8 * 8 + 32;
+    return 1024 + S::kAStages * 2 * S::kQuads * kTcQuadBytes + 2 * S::kQuads * kTcBQuadBytes +
+           2 * kTcRows * S::kMeta * 4 + 4 * S::kGroupBuf * 4 * S::kProdWarps + 4 * S::kWarpBuf * S::kEpiWarps + 8 * 8 + 32;
 }
 
 template <class S, int FMT>
@@ -210,7 +212,9 @@ __global__ void __launch_bounds__(S::kThreads, 1) k_tc_stage(const S st, const u
     unsigned char *sm = tcs_smem + pad;
     const uint32_t aA = base_s + pad, aB = aA + kABytes;
     uint32_t *meta = reinterpret_cast<uint32_t *>(sm + kABytes + kBBytes); /* [2][128][kMetaWords] */
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(meta + 2 * kTcRows * kMetaWords);
+    float *gbuf = reinterpret_cast<float *>(meta + 2 * kTcRows * kMetaWords); /* producer groups' buffers */
+    float *wbuf = gbuf + 4 * S::kProdWarps * S::kGroupBuf;                    /* epilogue warps' buffers  */
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(wbuf + S::kEpiWarps * S::kWarpBuf);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + kBars);
     volatile int *flags = reinterpret_cast<volatile int *>(tmem_slot + 1); /* [0] abort, [1] producers go */
     const uint32_t aBar = (uint32_t)__cvta_generic_to_shared(mbar);
@@ -276,7 +280,8 @@ __global__ void __launch_bounds__(S::kThreads, 1) k_tc_stage(const S st, const u
             const TcA<Q> A{sm + (lb % kAStages) * kAImage};
 #pragma unroll 1
             for (int row = grp; row < kTcRows; row += kProd / 8)
-                st.template produce<FMT>(blk * kTcRows + row, row, l, gm, A, mb + row * kMetaWords);
+                st.template produce<FMT>(blk * kTcRows + row, row, l, gm, A, mb + row * kMetaWords,
+                                         gbuf + grp * S::kGroupBuf);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_arrive(bar(kBarMeta + (lb & 1)));
             tc_producer_sync(kProd);
@@ -314,7 +319,8 @@ __global__ void __launch_bounds__(S::kThreads, 1) k_tc_stage(const S st, const u
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             st.epilogue(blk * kTcRows + row, lane_base + 64u * Q * (uint32_t)(lb & 1),
-                        meta + ((lb & 1) * kTcRows + row) * kMetaWords, part);
+                        meta + ((lb & 1) * kTcRows + row) * kMetaWords, part,
+                        wbuf + (warp - S::kProdWarps) * S::kWarpBuf);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) tc_arrive(bar(kBarFree + (lb & 1)));

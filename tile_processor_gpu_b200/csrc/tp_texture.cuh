@@ -664,20 +664,25 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             float *tj = smem + grp * kTexJob, *dj = tj + kTexD;
             float2 t[2][8];
             if (FROM_T) {
-                /* lane l: rows 2 l and 2 l + 1, one row pair */
-                const float *src = job_clt(mine);
-                const bool al16 = !(reinterpret_cast<uintptr_t>(src) & 15);
-                float2 *t2 = reinterpret_cast<float2 *>(tj);
+                /* lane l: columns 2 l and 2 l + 1 of every row pair (a row of the
+                 * group's loads is 64 bytes, its stores 16 bytes a lane) */
+                const float *src = job_clt(mine) + 2 * l;
+                const bool al8 = !(reinterpret_cast<uintptr_t>(src) & 7);
+                float4 *t4 = reinterpret_cast<float4 *>(tj);
+                float2 v[8][2];
 #pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    float v[8], w[8];
-                    load_row8(src + l * 32 + half * 8, al16, v);
-                    load_row8(src + l * 32 + 16 + half * 8, al16, w);
+                for (int rp = 0; rp < 8; rp++)
 #pragma unroll
-                    for (int c = 0; c < 8; c++) t2[JT2(l, half * 8 + c)] = make_float2(v[c], w[c]);
-                }
+                    for (int i = 0; i < 2; i++) {
+                        const float *p = src + (2 * rp + i) * 16;
+                        v[rp][i] = al8 ? *reinterpret_cast<const float2 *>(p) : make_float2(p[0], p[1]);
+                    }
+#pragma unroll
+                for (int rp = 0; rp < 8; rp++)
+                    t4[rp * 8 + l] = make_float4(v[rp][0].x, v[rp][1].x, v[rp][0].y, v[rp][1].y);
                 if (colors > 1) {
                     __syncwarp(gm);
+                    const float2 *t2 = reinterpret_cast<const float2 *>(tj);
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 #pragma unroll
