@@ -10,12 +10,11 @@
  * arithmetic is the same device code as the drop-in kernels, so the CLT and
  * the correlations are bit-identical to theirs.
  *
- * One 128-thread block (12 groups of 8 lanes with jobs; the fourth warp joins
- * for the fusion) per tile, grid-stride over the task list, five blocks per SM
- * at 96 registers and 27.6 KB of shared memory each.  More blocks leave less
- * of the SM's memory as L1 for the Bayer and kernel-tile reads and spill
- * (2592x1936 frame: five 2.60 ms, six 2.67, seven 2.69; 96-thread blocks at
- * seven 2.73, at eight 3.07):
+ * One 96-thread block (12 groups of 8 lanes) per tile, grid-stride over the
+ * task list, five blocks per SM at 27.6 KB of shared memory each.  More blocks
+ * leave less of the SM's memory as L1 for the Bayer and kernel-tile reads and
+ * fewer registers (2592x1936 frame, packed-pair stages: 96 threads at five
+ * blocks 2.05 ms, at six 2.07; 128 threads at four 2.32, five 2.11, six 2.17):
  *   1. forward CLT: group = (colour, camera) job, CLT into shared memory;
  *   2. correlations: groups 0-5, one camera pair each, from shared memory;
  *   3. texture: group = (camera, colour) job, inverse CLT into the
@@ -49,7 +48,7 @@ struct FrameParams {
     TextureParams tex; /* colors == 3, keep_weights == 0 */
 };
 
-constexpr int kFrameThreads = 128;
+constexpr int kFrameThreads = 96;
 constexpr int kFrameBlocksPerSm = 5;
 /* dynamic shared memory of k_frame, in floats: per job its CLT, then T in
  * place (kJob floats); per group the transpose buffer, the correlation
