@@ -19,7 +19,8 @@
  * The sub-pixel offset is kept within [-1, 1]; a fit without a maximum gives
  * k*.  strength = the fitted peak value / number of pairs.
  *
- * A warp takes 32 consecutive entries, finds the first entries of the tiles'
+ * A warp takes `win` consecutive entries (a power of two up to 32, by the
+ * list's length: see list_window), finds the first entries of the tiles'
  * runs among them (entries of one tile adjacent in the list) and fits two
  * tiles at a time, one per half warp, lane k evaluating S(k - r).  Where each
  * lane samples each pair's tile does not depend on the tile, so it is worked
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(256, 6) k_disparity_fit(int ntiles, const floa
                                                        size_t corr_stride, int r, long long num,
                                                        const int *__restrict__ idx,
                                                        const float *__restrict__ port_offsets, int pair_mask,
-                                                       int mode, float *__restrict__ disparity,
+                                                       int mode, int win, float *__restrict__ disparity,
                                                        float *__restrict__ strength)
 {
     __shared__ FitSample s_at[6][16];
@@ -143,13 +144,13 @@ __global__ void __launch_bounds__(256, 6) k_disparity_fit(int ntiles, const floa
     __syncthreads();
     const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4;
     const unsigned hm = 0xffffu << (16 * half);
-    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * 32;
-    for (long long e0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; e0 < num; e0 += step) {
+    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * win;
+    for (long long e0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * win; e0 < num; e0 += step) {
         /* the runs that start in this window */
         const long long my = e0 + lane;
         const int mytile = my < num ? __ldg(&idx[my]) >> 8 : -1;
         const int before = __shfl_up_sync(0xffffffffu, mytile, 1);
-        bool first = my < num && mytile >= 0 && mytile < ntiles;
+        bool first = lane < win && my < num && mytile >= 0 && mytile < ntiles;
         if (first) first = lane ? before != mytile : (my == 0 || (__ldg(&idx[my - 1]) >> 8) != mytile);
         unsigned starts = __ballot_sync(0xffffffffu, first);
         while (starts) {

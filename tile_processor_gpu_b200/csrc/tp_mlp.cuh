@@ -29,8 +29,9 @@ namespace tp {
 
 /* ---- features ------------------------------------------------------------- */
 
-/* A warp takes 32 consecutive correlation entries and writes the row of each
- * tile whose run (entries of one tile adjacent) starts among them:
+/* A warp takes `win` consecutive correlation entries (a power of two up to 32,
+ * by the list's length: see list_window) and writes the row of each tile
+ * whose run (entries of one tile adjacent) starts among them:
  * feat[tile][p * n2 + k] = C_p[k] / max |C| over the run, zeros for pairs the
  * run does not list (a pair listed twice: the later entry's plane, both in
  * the maximum; entries with p >= 6 are skipped).  The warp reads idx[e ..
@@ -42,19 +43,19 @@ namespace tp {
  * (0.85 GB, 6.2 TB/s). */
 __global__ void __launch_bounds__(256) k_mlp_features(int ntiles, const float *__restrict__ corrs,
                                                       size_t corr_stride, int n2, long long num,
-                                                      const int *__restrict__ idx, float *__restrict__ feat,
+                                                      const int *__restrict__ idx, int win, float *__restrict__ feat,
                                                       size_t feat_stride)
 {
     constexpr int kPer = 8;  /* ceil(225 / 32): n2 <= 225 */
     constexpr int kRow = 22; /* ceil(675 / 32): float2 of a row per lane */
     const int lane = threadIdx.x & 31;
-    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * 32;
+    const long long step = (long long)gridDim.x * (blockDim.x >> 5) * win;
     const bool tight = corr_stride == (size_t)n2 && !(reinterpret_cast<uintptr_t>(corrs) & 7) &&
                        !(reinterpret_cast<uintptr_t>(feat) & 7) && !(feat_stride & 1);
-    for (long long e0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; e0 < num; e0 += step) {
+    for (long long e0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * win; e0 < num; e0 += step) {
       const int mytile = e0 + lane < num ? __ldg(&idx[e0 + lane]) >> 8 : -1;
       const int before = __shfl_up_sync(0xffffffffu, mytile, 1);
-      bool first = e0 + lane < num && mytile >= 0 && mytile < ntiles;
+      bool first = lane < win && e0 + lane < num && mytile >= 0 && mytile < ntiles;
       if (first) first = lane ? before != mytile : (e0 == 0 || (__ldg(&idx[e0 - 1]) >> 8) != mytile);
       unsigned starts = __ballot_sync(0xffffffffu, first);
       for (; starts; starts &= starts - 1) {
