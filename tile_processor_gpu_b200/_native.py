@@ -133,10 +133,9 @@ def load():
 
 def call(name, *args):
     """Call a tp_* entry point; raise TpError on a negative status."""
-    lib = load()
-    rc = getattr(lib, name)(*args)
+    rc = getattr(_lib if _lib is not None else load(), name)(*args)
     if rc < 0:
-        raise TpError(name, rc, lib.tp_last_error().decode())
+        raise TpError(name, rc, _lib.tp_last_error().decode())
     return rc
 
 

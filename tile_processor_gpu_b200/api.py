@@ -67,25 +67,24 @@ class PointerArray:
 
 def _parr(x):
     if isinstance(x, PointerArray):
-        return x.ptr
+        return x.dev.data_ptr()
     if isinstance(x, (list, tuple)):
         return PointerArray(x).ptr
     raise TypeError("expected a list of tensors or a PointerArray")
 
 
 def _dptr(t):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    """device address of a tensor for a pointer argument (None = NULL)"""
+    return None if t is None else t.data_ptr()
 
 
 def _stream(stream):
     """torch stream (None = torch's current stream), or a raw cudaStream_t int"""
-    if isinstance(stream, int):
-        return ctypes.c_void_p(stream)
     if stream is None:
-        if not torch.cuda.is_available():
-            return ctypes.c_void_p(0)
+        if not torch.cuda.is_initialized() and not torch.cuda.is_available():
+            return None
         stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
+    return stream if isinstance(stream, int) else stream.cuda_stream
 
 
 def tasks_to_device(tasks, device="cuda"):
