@@ -236,8 +236,18 @@ __device__ __forceinline__ void load_row8s(const float *p, float v[8])
     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
 }
 
-/* 8 consecutive floats of global memory (32-byte aligned): one 256-bit access */
+/* 8 consecutive floats of global memory (32-byte aligned): one 256-bit access.  ld8_global is for rows that
+   the SM reads once (CLT tiles of the textures and the inverse transform, deconvolution kernel rows): it leaves
+   L1 to what is read again.  With plain loads the tensor-core inverse's tables were evicted by the tiles that
+   pass: the fp16 image of 2592x1936 took 436 us, 418 this way; the texture list 611 and 608.  ld8_l1 is for
+   the correlation, whose pairs share a tile's rows. */
 __device__ __forceinline__ void ld8_global(const float *p, float v[8])
+{
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void ld8_l1(const float *p, float v[8])
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])

@@ -73,8 +73,8 @@ __device__ __forceinline__ void corr_product(const float *a, const float *b, int
                 if (al32) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        ld8_global(pa + q * 64, A[q]);
-                        ld8_global(pb + q * 64, B[q]);
+                        ld8_l1(pa + q * 64, A[q]);
+                        ld8_l1(pb + q * 64, B[q]);
                     }
                 } else {
 #pragma unroll
