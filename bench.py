@@ -6,9 +6,8 @@ points:
   1. tp_convert_correct_tiles  forward CLT + aberration kernels + shifts
   2. tp_correlate2D            6 camera pairs per tile, 15x15 outputs
   3. tp_generate_RBGA          texture list + overlapped RGBA texture
-The same frame through tp_process_frame (one kernel per tile parity with the
-tile's CLT kept in shared memory) is timed too and reported as
-`fused_frame_ms`.
+The same frame through process_frame (one call, the CLT in a workspace by task)
+is timed too and reported as `fused_frame_ms`.
 `value` is whole-job frames/s (N GPUs each process their own frames:
 frame-level replicas, weak scaling).  `e2e` is the same pipeline driven
 through the public API with host buffers: each step copies the frame's four
@@ -71,7 +70,7 @@ def bench_config(world):
 
 
 def dram_traffic():
-    """DRAM bytes per frame of each stage (and of the fused frame kernel)
+    """DRAM bytes per frame of each stage (and of the one-call frame)
     from the ncu captures recorded with the package (captures, not
     measurements of this run): (per stage, source, fused bytes, fused source)"""
     path = os.path.join(ROOT, "tile_processor_gpu_b200", "data", "dram_traffic.json")
@@ -573,7 +572,7 @@ class FramePipeline:
 
     STAGES = ("convert", "correlate", "texture")
     LAUNCHES = {"convert": 1, "correlate": 1, "texture": 10}  # texture: 5 list kernels, RGBA clear, 4 passes
-    FRAME_LAUNCHES = 10  # 5 list kernels, RGBA clear, 4 parity launches
+    FRAME_LAUNCHES = 12  # 5 list kernels, RGBA clear, convert, correlate, 4 passes
 
     def step(self):
         self.convert()
@@ -714,7 +713,7 @@ def run_b200(args, rank, world, local, pg):
     frames_timed = args.steps * F
     stage_ms = {s: sum(a.elapsed_time(b) for a, b in ev[s]) / frames_timed for s in pipe.STAGES}
 
-    # the same frame through tp_process_frame (fused per tile), reported beside
+    # the same frame through process_frame (one call), reported beside
     fused_steps = max(3, min(args.steps, 10))
     for _ in range(2):
         pipe.frame()

@@ -364,6 +364,26 @@ int tp_process_frame(const tp_geometry *g,
                      float *const *clt,
                      tp_stream_t stream);
 
+/* tp_process_frame with a device workspace of the caller's (256-byte aligned,
+ * contents undefined before and after; nothing else may use it until the call's
+ * work on the stream is done).  With at least tp_process_frame_workspace
+ * (num_tiles) bytes of it and clt NULL, the frame runs in stages, up to 131072
+ * tasks at a time through the workspace: the same correlations and the
+ * same image up to the order of its additions, in about two thirds of the time.
+ * With less, with clt, or without a workspace it runs as tp_process_frame. */
+size_t tp_process_frame_workspace(int num_tiles);
+int tp_process_frame_ws(const tp_geometry *g,
+                        float *const *kernel_offsets, float *const *kernels, float *const *images,
+                        size_t dstride, tp_task *tasks, int num_tiles, int lpf_mask,
+                        int corr_colors, float corr_scale0, float corr_scale1, float corr_scale2,
+                        float fat_zero, int corr_radius, size_t corr_stride, float *corrs,
+                        const float *port_offsets, float min_shot, float scale_shot, float diff_sigma,
+                        float weight0, float weight1, float weight2, int dust_remove,
+                        int *texture_indices, int *num_texture_tiles, int *woi,
+                        size_t texture_rbga_stride, float *texture_rbga,
+                        float *const *clt, void *workspace, size_t workspace_bytes,
+                        tp_stream_t stream);
+
 /* ---- disparity from the pair correlations ---------------------------------------
  * No counterpart in the reference, which hands its correlation tiles to the
  * Java caller (src/TileProcessor.cuh:1176-1443 is where it stops).  For each

@@ -65,6 +65,8 @@ SIGNATURES = {
                               _I, _I, _P],
     "tp_process_frame": [_G, _P, _P, _P, _S, _P, _I, _I, _I, _F, _F, _F, _F, _I, _S, _P, _P, _F, _F, _F, _F, _F,
                          _F, _I, _P, _P, _P, _S, _P, _P, _P],
+    "tp_process_frame_ws": [_G, _P, _P, _P, _S, _P, _I, _I, _I, _F, _F, _F, _F, _I, _S, _P, _P, _F, _F, _F, _F, _F,
+                            _F, _I, _P, _P, _P, _S, _P, _P, _P, _S, _P],
     "tp_disparity_fit": [_G, _P, _S, _I, _S, _P, _P, _I, _I, _P, _P, _P],
     "tp_psf_to_clt": [_P, _S, _P, _P],
     "tp_tasks_from_portsxy": [_P, _I, _I, _I, _P],
@@ -102,7 +104,8 @@ SIGNATURES = {
 }
 STRING_FUNCS = ("tp_last_error", "tp_version")
 # entry points returning a count (long long) instead of a status
-COUNT_FUNCS = {"tp_read_floats": [ctypes.c_char_p, _P, _S], "tp_write_floats": [ctypes.c_char_p, _P, _S]}
+COUNT_FUNCS = {"tp_read_floats": [ctypes.c_char_p, _P, _S], "tp_write_floats": [ctypes.c_char_p, _P, _S],
+               "tp_process_frame_workspace": [_I]}
 
 _lib = None
 

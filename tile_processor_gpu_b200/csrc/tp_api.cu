@@ -131,7 +131,7 @@ int shape_per_sm(int which)
  * their attribute once per device (the first call; make it before capturing
  * a stream into a graph). */
 std::mutex g_attr_mutex;
-bool g_tex_attr[8][128], g_frame_attr[128], g_tc_attr[128], g_gemm_tc_attr[4][128], g_cv_attr[128];
+bool g_tex_attr[9][128], g_frame_attr[128], g_tc_attr[128], g_gemm_tc_attr[4][128], g_cv_attr[128];
 
 int set_smem_once(bool *done, const void *func, size_t bytes, const char *what)
 {
@@ -156,13 +156,14 @@ static auto tex_kernel(int colors)
 
 int texture_smem_setup()
 {
-    const void *const kernels[8] = {
+    const void *const kernels[9] = {
         (const void *)tp::k_textures<false, true, 1>,  (const void *)tp::k_textures<false, true, 3>,
         (const void *)tp::k_textures<true, true, 1>,   (const void *)tp::k_textures<true, true, 3>,
         (const void *)tp::k_textures<false, false, 1>, (const void *)tp::k_textures<false, false, 3>,
-        (const void *)tp::k_textures<true, false, 1>,  (const void *)tp::k_textures<true, false, 3>};
+        (const void *)tp::k_textures<true, false, 1>,  (const void *)tp::k_textures<true, false, 3>,
+        (const void *)tp::k_textures<false, false, 3, true>};
     int rc = TP_OK;
-    for (int i = 0; i < 8 && !rc; i++)
+    for (int i = 0; i < 9 && !rc; i++)
         rc = set_smem_once(g_tex_attr[i], kernels[i], tp::kTexSmemBytes, "cudaFuncSetAttribute(k_textures)");
     return rc;
 }
@@ -281,7 +282,7 @@ int tp_resident_ctas(int kernel)
     if (kernel == TP_SHAPE_CONVERT) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_convert_correct_tiles<3>, tp::kConvertThreads, 0);
     } else if (kernel == TP_SHAPE_CORRELATE) {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_correlate2D, tp::kCorrThreads, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_correlate2D<false>, tp::kCorrThreads, 0);
     } else {
         if ((rc = texture_smem_setup())) return rc;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, tp::k_textures<false, false, 3>, tp::kTexThreads,
@@ -322,6 +323,21 @@ int tp_reset_lpf(void)
     return TP_OK;
 }
 
+/* one colour per warp item while those items fit the resident warps (3 CTAs
+ * per SM) in one turn, else all three (see the kernel) */
+struct ConvertShape {
+    bool small;
+    unsigned grid;
+};
+static ConvertShape convert_shape(int num_tiles, int sms)
+{
+    const long long chunks = ((long long)num_tiles + 3) / 4;
+    const bool small = chunks * 12 <= (long long)sms * 3 * (tp::kConvertThreads / 32);
+    unsigned grid = grid_for(chunks * (small ? 12 : 4), tp::kConvertThreads / 32, sms, shape_per_sm(TP_SHAPE_CONVERT));
+    if (!small) grid = (grid + 3) & ~3u; /* a warp keeps its camera */
+    return {small, grid};
+}
+
 int tp_convert_correct_tiles(const tp_geometry *g, float *const *kernel_offsets, float *const *kernels,
                              float *const *images, const tp_task *tasks, float *const *clt, size_t dstride,
                              int num_tiles, int lpf_mask, tp_stream_t stream)
@@ -336,15 +352,10 @@ int tp_convert_correct_tiles(const tp_geometry *g, float *const *kernel_offsets,
     if (num_tiles == 0) return TP_OK;
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    /* one colour per warp item while those items fit the resident warps (3 CTAs
-     * per SM) in one turn, else all three (see the kernel) */
-    const long long chunks = ((long long)num_tiles + 3) / 4;
-    const bool small = chunks * 12 <= (long long)sms * 3 * (tp::kConvertThreads / 32);
-    unsigned grid = grid_for(chunks * (small ? 12 : 4), tp::kConvertThreads / 32, sms, shape_per_sm(TP_SHAPE_CONVERT));
-    if (!small) grid = (grid + 3) & ~3u; /* a warp keeps its camera */
-    const auto kernel = small ? tp::k_convert_correct_tiles<1> : tp::k_convert_correct_tiles<3>;
-    kernel<<<grid, tp::kConvertThreads, 0, (cudaStream_t)stream>>>(gd, dstride, kernel_offsets, kernels, images, tasks, clt,
-                                                   num_tiles, lpf_mask);
+    const ConvertShape cs = convert_shape(num_tiles, sms);
+    const auto kernel = cs.small ? tp::k_convert_correct_tiles<1> : tp::k_convert_correct_tiles<3>;
+    kernel<<<cs.grid, tp::kConvertThreads, 0, (cudaStream_t)stream>>>(gd, dstride, kernel_offsets, kernels, images, tasks, clt,
+                                                   num_tiles, lpf_mask, tp::FrameSlots{});
     return cuda_status(cudaGetLastError(), "convert_correct_tiles launch");
 }
 
@@ -367,9 +378,9 @@ int tp_correlate2D(const tp_geometry *g, float *const *clt, int colors, float sc
     if ((rc = sm_count(&sms))) return rc;
     const unsigned grid = grid_for((long long)num_corr_tiles, tp::kCorrThreads / 8, sms,
                                    shape_per_sm(TP_SHAPE_CORRELATE));
-    tp::k_correlate2D<<<grid, tp::kCorrThreads, 0, (cudaStream_t)stream>>>(
+    tp::k_correlate2D<false><<<grid, tp::kCorrThreads, 0, (cudaStream_t)stream>>>(
         gd, clt, colors, scale0, scale1, scale2, fat_zero, (long long)num_corr_tiles, corr_indices, corr_stride,
-        corr_radius, corrs);
+        corr_radius, corrs, nullptr, nullptr);
     return cuda_status(cudaGetLastError(), "correlate2D launch");
 }
 
@@ -409,7 +420,7 @@ static int launch_textures(Kernel kernel, const tp::Geom &gd, const int *woi, fl
         const unsigned grid = grid_for(n, tp::tex_tiles(p.colors), sms, shape_per_sm(TP_SHAPE_TEXTURES));
         kernel<<<grid, tp::kTexThreads, tp::kTexSmemBytes, (cudaStream_t)stream>>>(
             gd, woi, clt, n, indices + n0, nullptr, 0, 0, 0, port_offsets, p, rbg_stride, rbg, tile_stride,
-            tiles ? tiles + n0 * tile_stride : nullptr);
+            tiles ? tiles + n0 * tile_stride : nullptr, tp::FrameSlots{});
         const int rc = cuda_status(cudaGetLastError(), "textures_accumulate launch");
         if (rc) return rc;
     }
@@ -512,6 +523,12 @@ static cudaError_t launch_chained(bool dependent, dim3 grid, dim3 block, size_t 
 }
 } /* extern "C++" */
 
+/* process_frame in stages: at most this many tasks go through the workspace at a
+ * time (1.6 GB; a 2592x1936 frame has 78,408).  Short parts would keep their CLT
+ * in L2, but the last waves of six launches per part cost more: 2592x1936 in
+ * parts of 4096 tasks 1.64 ms, 8192 1.50, 16384 1.36, whole 1.31. */
+constexpr int kFrameChunk = 131072;
+
 /* task lists up to this length are listed by one kernel on one cluster (one task
  * per thread and turn), longer ones by a chain of five kernels on all SMs */
 constexpr int kListOneKernel = 8192;
@@ -581,7 +598,7 @@ int tp_clear_texture_rbga(const tp_geometry *g, int texture_width, int texture_s
     int sms;
     if ((rc = sm_count(&sms))) return rc;
     tp::k_clear_rbga<<<grid_for(texture_slice_height, 1, sms, 16), 256, 0, (cudaStream_t)stream>>>(
-        nullptr, 0, texture_width, texture_slice_height, texture_rbga_stride, texture_tiles);
+        nullptr, 0, texture_width, texture_slice_height, texture_rbga_stride, texture_tiles, nullptr, 0);
     return cuda_status(cudaGetLastError(), "clear_texture_rbga launch");
 }
 
@@ -626,7 +643,8 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
     {
         const int max_rows = (gd.TY + 1) * 8 * (colors + 1);
         const cudaError_t err = launch_chained(true, grid_for(max_rows, 1, sms, 16), 256, 0, s, tp::k_clear_rbga,
-                                               (const int *)woi, colors, 0, 0, texture_rbga_stride, texture_tiles);
+                                               (const int *)woi, colors, 0, 0, texture_rbga_stride, texture_tiles,
+                                               (int *)nullptr, 0);
         if (err != cudaSuccess) return cuda_status(err, "generate_RBGA clear launch");
     }
     float *const *src = clt;
@@ -647,7 +665,7 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
         const cudaError_t err =
             launch_chained(true, grid, tp::kTexThreads, tp::kTexSmemBytes, s, tex, gd, (const int *)woi, src, 0,
                            (const int *)base, (const int *)num_texture_tiles, parity << 1, quarter, -quarter,
-                           port_offsets, p, texture_rbga_stride, texture_tiles, (size_t)0, (float *)nullptr);
+                           port_offsets, p, texture_rbga_stride, texture_tiles, (size_t)0, (float *)nullptr, tp::FrameSlots{});
         if (err != cudaSuccess) return cuda_status(err, "generate_RBGA texture pass launch");
     }
     return cuda_status(cudaGetLastError(), "generate_RBGA launch");
@@ -681,13 +699,15 @@ int tp_generate_RBGA_rows(const tp_geometry *g, tp_task *tasks, int num_tiles, i
                          stream);
 }
 
-int tp_process_frame(const tp_geometry *g, float *const *kernel_offsets, float *const *kernels, float *const *images,
+static size_t frame_slots(void *workspace, int num_tiles, tp::FrameSlots *slots);
+
+static int process_frame(const tp_geometry *g, float *const *kernel_offsets, float *const *kernels, float *const *images,
                      size_t dstride, tp_task *tasks, int num_tiles, int lpf_mask, int corr_colors, float corr_scale0,
                      float corr_scale1, float corr_scale2, float fat_zero, int corr_radius, size_t corr_stride,
                      float *corrs, const float *port_offsets, float min_shot, float scale_shot, float diff_sigma,
                      float weight0, float weight1, float weight2, int dust_remove, int *texture_indices,
                      int *num_texture_tiles, int *woi, size_t texture_rbga_stride, float *texture_rbga,
-                     float *const *clt, tp_stream_t stream)
+                     float *const *clt, void *workspace, size_t workspace_bytes, tp_stream_t stream)
 {
     tp::Geom gd;
     int rc = check_geometry(g, &gd);
@@ -713,12 +733,58 @@ int tp_process_frame(const tp_geometry *g, float *const *kernel_offsets, float *
     cudaStream_t s = (cudaStream_t)stream;
     int sms;
     if ((rc = sm_count(&sms))) return rc;
+    /* In stages where the caller gave a workspace: forward transform,
+     * correlations and textures each in a kernel of its own launch shape, with the
+     * CLT by task in between, against one kernel in which every phase takes the
+     * registers and shared memory of the largest and half its warps wait in
+     * the correlation.  Faster at every size (us on chip -> in stages: 64x64 59 -> 37,
+     * 256x256 81 -> 49, 640x512 133 -> 116, 1608x1208 797 -> 519,
+     * 2592x1936 2054 -> 1310), so the on-chip form remains for calls without
+     * that memory and with a CLT output.  (A texture list code holds 23 bits of tile.) */
+    tp::FrameSlots slots = {};
+    const size_t need = frame_slots(workspace, num_tiles, &slots);
+    const bool staged = !clt && workspace && workspace_bytes >= need && !((uintptr_t)workspace & 255) &&
+                        (long long)gd.TX * gd.TY <= (1 << 23);
+    const int chunks = (num_tiles - 1) / kFrameChunk + 1;
     {
         /* a programmatic dependent of the list's last kernel, as in generate_rbga */
         const int max_rows = (gd.TY + 1) * 8 * 4;
         const cudaError_t err = launch_chained(true, grid_for(max_rows, 1, sms, 16), 256, 0, s, tp::k_clear_rbga,
-                                               (const int *)woi, 3, 0, 0, texture_rbga_stride, texture_rbga);
+                                               (const int *)woi, 3, 0, 0, texture_rbga_stride, texture_rbga,
+                                               staged ? slots.counts : (int *)nullptr, staged ? 4 * chunks : 0);
         if (err != cudaSuccess) return cuda_status(err, "process_frame clear launch");
+    }
+    if (staged) {
+        if ((rc = texture_smem_setup())) return rc;
+        cudaError_t err = cudaSuccess;
+        /* The textures start while the correlations end (both read the CLT, which
+         * was complete when the correlations started); the next part's forward
+         * transform, an ordinary launch, follows them all. */
+        for (int i = 0; i < chunks && err == cudaSuccess; i++, slots.counts += 4) {
+            const tp_task *t = tasks + (size_t)i * kFrameChunk;
+            const int n = num_tiles - i * kFrameChunk < kFrameChunk ? num_tiles - i * kFrameChunk : kFrameChunk;
+            const ConvertShape cs = convert_shape(n, sms);
+            err = launch_chained(false, cs.grid, tp::kConvertThreads, 0, s,
+                                 cs.small ? tp::k_convert_correct_tiles<1, true> : tp::k_convert_correct_tiles<3, true>,
+                                 gd, dstride, kernel_offsets, kernels, images, t, (float *const *)nullptr, n, lpf_mask,
+                                 slots);
+            if (err == cudaSuccess)
+                err = launch_chained(false, grid_for(6LL * n, tp::kCorrThreads / 8, sms, shape_per_sm(TP_SHAPE_CORRELATE)), tp::kCorrThreads, 0, s,
+                                     tp::k_correlate2D<true>, gd, (float *const *)nullptr, corr_colors, corr_scale0,
+                                     corr_scale1, corr_scale2, fat_zero, 6LL * n, (const int *)nullptr, corr_stride,
+                                     corr_radius, corrs + (size_t)i * kFrameChunk * 6 * corr_stride, t,
+                                     (const float *)slots.clt);
+            for (int parity = 0; parity < 4 && err == cudaSuccess; parity++) {
+                tp::FrameSlots ts = slots;
+                ts.list += (size_t)parity * n;
+                err = launch_chained(true, grid_for((n - 1) / 4 + 1, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES)), tp::kTexThreads, tp::kTexSmemBytes, s,
+                                     tp::k_textures<false, false, 3, true>, gd, (const int *)woi,
+                                     (float *const *)nullptr, 0, (const int *)nullptr, (const int *)slots.counts,
+                                     parity, n, 0, port_offsets, tex, texture_rbga_stride, texture_rbga, (size_t)0,
+                                     (float *)nullptr, ts);
+            }
+        }
+        return cuda_status(err != cudaSuccess ? err : cudaGetLastError(), "process_frame launch");
     }
     tp::FrameParams fp;
     fp.lpf_mask = lpf_mask;
@@ -750,6 +816,57 @@ int tp_process_frame(const tp_geometry *g, float *const *kernel_offsets, float *
         if (err != cudaSuccess) return cuda_status(err, "process_frame launch");
     }
     return cuda_status(cudaGetLastError(), "process_frame launch");
+}
+
+/* The workspace's parts (slots; NULL: none) and its size for num_tiles tasks: the
+ * texture list counts of every part, the lists and the CLT of one part. */
+static size_t frame_slots(void *workspace, int num_tiles, tp::FrameSlots *slots)
+{
+    if (num_tiles <= 0) return 0;
+    const size_t chunk = num_tiles < kFrameChunk ? num_tiles : kFrameChunk;
+    const size_t chunks = (num_tiles + (size_t)kFrameChunk - 1) / kFrameChunk;
+    const size_t head = (chunks * 4 * sizeof(int) + 255) & ~(size_t)255;
+    const size_t lists = (chunk * 4 * sizeof(int2) + 255) & ~(size_t)255;
+    if (slots) {
+        char *p = (char *)workspace;
+        slots->counts = (int *)p;
+        slots->list = (int2 *)(p + head);
+        slots->clt = (float *)(p + head + lists);
+    }
+    return head + lists + chunk * tp::kSlot * sizeof(float);
+}
+
+int tp_process_frame(const tp_geometry *g, float *const *kernel_offsets, float *const *kernels, float *const *images,
+                     size_t dstride, tp_task *tasks, int num_tiles, int lpf_mask, int corr_colors, float corr_scale0,
+                     float corr_scale1, float corr_scale2, float fat_zero, int corr_radius, size_t corr_stride,
+                     float *corrs, const float *port_offsets, float min_shot, float scale_shot, float diff_sigma,
+                     float weight0, float weight1, float weight2, int dust_remove, int *texture_indices,
+                     int *num_texture_tiles, int *woi, size_t texture_rbga_stride, float *texture_rbga,
+                     float *const *clt, tp_stream_t stream)
+{
+    return process_frame(g, kernel_offsets, kernels, images, dstride, tasks, num_tiles, lpf_mask, corr_colors,
+                         corr_scale0, corr_scale1, corr_scale2, fat_zero, corr_radius, corr_stride, corrs,
+                         port_offsets, min_shot, scale_shot, diff_sigma, weight0, weight1, weight2, dust_remove,
+                         texture_indices, num_texture_tiles, woi, texture_rbga_stride, texture_rbga, clt, nullptr, 0,
+                         stream);
+}
+
+size_t tp_process_frame_workspace(int num_tiles) { return frame_slots(nullptr, num_tiles, nullptr); }
+
+int tp_process_frame_ws(const tp_geometry *g, float *const *kernel_offsets, float *const *kernels,
+                        float *const *images, size_t dstride, tp_task *tasks, int num_tiles, int lpf_mask,
+                        int corr_colors, float corr_scale0, float corr_scale1, float corr_scale2, float fat_zero,
+                        int corr_radius, size_t corr_stride, float *corrs, const float *port_offsets, float min_shot,
+                        float scale_shot, float diff_sigma, float weight0, float weight1, float weight2,
+                        int dust_remove, int *texture_indices, int *num_texture_tiles, int *woi,
+                        size_t texture_rbga_stride, float *texture_rbga, float *const *clt, void *workspace,
+                        size_t workspace_bytes, tp_stream_t stream)
+{
+    return process_frame(g, kernel_offsets, kernels, images, dstride, tasks, num_tiles, lpf_mask, corr_colors,
+                         corr_scale0, corr_scale1, corr_scale2, fat_zero, corr_radius, corr_stride, corrs,
+                         port_offsets, min_shot, scale_shot, diff_sigma, weight0, weight1, weight2, dust_remove,
+                         texture_indices, num_texture_tiles, woi, texture_rbga_stride, texture_rbga, clt, workspace,
+                         workspace_bytes, stream);
 }
 
 int tp_generate_RBGA_noalloc(const tp_geometry *g, tp_task *tasks, int num_tiles, int width, int height,

@@ -311,4 +311,14 @@ __device__ __forceinline__ float shifted_window_lane(int n, float cs, float sn)
     return __fmaf_rn(__ldg(&d_hwin[n]), cs, __ldg(&d_hwinc[n]) * sn);
 }
 
+/* Workspace of a frame in stages (process_frame): the CLT of the tasks at hand by their
+ * place in the task list, [task][camera][colour][256], and their texture lists
+ * by tile parity (task, texture list code), written by the forward transform. */
+struct FrameSlots {
+    float *clt;
+    int2 *list;  /* [4][tasks] */
+    int *counts; /* [4]        */
+};
+constexpr int kSlot = 4 * 3 * 256;
+
 } /* namespace tp */

@@ -421,13 +421,15 @@ __device__ __forceinline__ void convert_job(const Geom &g, size_t dstride,
  * The fields of the next item's tasks are read an item ahead, the offsets of
  * the next job's kernel tile a job ahead, and the kernel tile itself is
  * prefetched into L2 an item ahead (lane l: bytes 128 l .. 128 l + 127 of the
- * 1 KB tile). */
+ * 1 KB tile).
+ * SLOTS: the CLT goes to the frame's workspace by task, and each textured task
+ * into the list of its parity (FrameSlots; the order within a list does not matter). */
 constexpr int kConvertThreads = 160;
-template <int PER>
+template <int PER, bool SLOTS = false>
 __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
     Geom g, size_t dstride, float *const *kernel_offsets, float *const *kernels,
     float *const *images, const tp_task *__restrict__ tasks, float *const *clt, int num_tiles,
-    int lpf_mask)
+    int lpf_mask, FrameSlots slots)
 {
     static_assert(PER == 1 || PER == 3, "colours per item");
     __shared__ __align__(16) float cbuf[kConvertThreads / 8][kCvBuf];
@@ -450,11 +452,18 @@ __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
         if (n >= num_tiles) return t;
         const tp_task *p = tasks + n;
         const int task = __ldg(&p->task), txy = __ldg(&p->txy);
-        const int tx = txy & 0xfff, ty = txy >> 16;
+        const int tx = txy & (SLOTS ? 0xffff : 0xfff), ty = txy >> 16;
         t.cx = __ldg(&p->xy[cam][0]);
         t.cy = __ldg(&p->xy[cam][1]);
         if (!task || tx >= g.TX || ty < 0 || ty >= g.TY) return t;
-        t.tile = ty * g.TX + tx;
+        t.tile = SLOTS ? n : ty * g.TX + tx;
+        if (SLOTS && cam == 0 && l == 0 && (PER == 3 || (w % 12) >> 2 == 0) && (task & TP_TASK_TEXTURE_BITS)) {
+            /* its entry in the texture list of its parity */
+            const int parity = (tx & 1) | ((ty & 1) << 1);
+            const int k = atomicAdd(&slots.counts[parity], 1);
+            slots.list[(size_t)parity * num_tiles + k] =
+                make_int2(n, ((ty * g.TX + tx) << 8) | (1 << 7) | (task & TP_TASK_TEXTURE_BITS));
+        }
         /* the kernel tile (as job_geometry chooses it) */
         const float step_inv = __int_as_float((127 - g.ls) << 23);
         const int ktx = min(g.KH - 1, max(0, __float2int_rn(__fmaf_rn(t.cx, step_inv, 1.0f))));
@@ -472,7 +481,7 @@ __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
     /* PER 3: the grid, and so the step, is a multiple of 4: a warp keeps its camera */
     int cam = PER == 3 ? w & 3 : (w % 12) & 3;
     const float *kern = kernels[cam], *extra = kernel_offsets[cam], *img = images[cam];
-    float *out = clt[cam];
+    float *out = SLOTS ? slots.clt + cam * 768 : clt[cam];
     Task next = fetch(w);
     float nex[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     if (next.tile >= 0) fetch_extra(extra, next.ktile, PER == 3 ? 0 : (w % 12) >> 2, nex);
@@ -488,7 +497,7 @@ __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
             kern_n = kernels[c];
             extra_n = kernel_offsets[c];
             img_n = images[c];
-            out_n = clt[c];
+            out_n = SLOTS ? slots.clt + c * 768 : clt[c];
         }
 #pragma unroll 1
         for (int i = 0; i < PER; i++) {
@@ -505,7 +514,7 @@ __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(kern_n + (size_t)(next.ktile + color_n + i) * 256 + l * 32));
             if (t.tile < 0) continue;
             convert_job<true>(g, dstride, extra, kern, img, t.cx, t.cy, color, lpf_mask,
-                              out + ((size_t)t.tile * 3 + color) * 256, cbuf[grp], l, gm, ex);
+                                out + (size_t)t.tile * (SLOTS ? kSlot : 768) + color * 256, cbuf[grp], l, gm, ex);
         }
         if (PER == 1) {
             kern = kern_n;

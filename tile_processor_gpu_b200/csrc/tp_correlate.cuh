@@ -215,12 +215,16 @@ __device__ __forceinline__ void corr_job(const float *a, const float *b, int cst
 
 constexpr int kCorrThreads = 128;
 
+/* SLOTS: entry n is pair n % 6 of task n / 6, whose CLT lies in the frame's workspace by task (FrameSlots) */
+template <bool SLOTS>
 __global__ void __launch_bounds__(kCorrThreads, 4) k_correlate2D(Geom g, float *const *clt, int colors,
                                                                  float scale0, float scale1, float scale2,
                                                                  float fat_zero, long long num_corr_tiles,
                                                                  const int *__restrict__ corr_indices,
                                                                  size_t corr_stride, int corr_radius,
-                                                                 float *__restrict__ corrs)
+                                                                 float *__restrict__ corrs,
+                                                                 const tp_task *__restrict__ tasks,
+                                                                 const float *slot_clt)
 {
     __shared__ __align__(16) float tbuf[kCorrThreads / 8][kCorrBuf];
     const int l = threadIdx.x & 7;
@@ -228,12 +232,24 @@ __global__ void __launch_bounds__(kCorrThreads, 4) k_correlate2D(Geom g, float *
     const unsigned gm = group_mask();
     const long long groups_total = (long long)gridDim.x * (blockDim.x >> 3);
     const int ntiles = g.TX * g.TY;
+    /* the frame's textures may fill the SM slots this grid frees */
+    if (SLOTS) grid_dependents_launch();
     for (long long n = (long long)blockIdx.x * (blockDim.x >> 3) + grp; n < num_corr_tiles; n += groups_total) {
-        const int code = corr_indices[n];
-        const int tile = code >> 8, pair = code & 0xff;
-        if (pair >= 6 || tile < 0 || tile >= ntiles) continue;
-        const float *ta = clt[c_pairs[pair][0]] + (size_t)tile * 768;
-        const float *tb2 = clt[c_pairs[pair][1]] + (size_t)tile * 768;
+        const float *ta, *tb2;
+        if (SLOTS) {
+            const int slot = (int)(n / 6), pair = (int)n - 6 * slot;
+            const int task = __ldg(&tasks[slot].task), txy = __ldg(&tasks[slot].txy);
+            const int tx = txy & 0xffff, ty = txy >> 16;
+            if (!((task >> (TP_TASK_CORR_BITS + pair)) & 1) || tx >= g.TX || ty < 0 || ty >= g.TY) continue;
+            ta = slot_clt + (size_t)slot * (4 * 768) + c_pairs[pair][0] * 768;
+            tb2 = slot_clt + (size_t)slot * (4 * 768) + c_pairs[pair][1] * 768;
+        } else {
+            const int code = corr_indices[n];
+            const int tile = code >> 8, pair = code & 0xff;
+            if (pair >= 6 || tile < 0 || tile >= ntiles) continue;
+            ta = clt[c_pairs[pair][0]] + (size_t)tile * 768;
+            tb2 = clt[c_pairs[pair][1]] + (size_t)tile * 768;
+        }
         corr_job<true>(ta, tb2, 256, colors, scale0, scale1, scale2, fat_zero, corr_radius, tbuf[grp],
                        corrs + (size_t)n * corr_stride, l, gm);
     }

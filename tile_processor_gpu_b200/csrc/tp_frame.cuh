@@ -3,6 +3,10 @@
  * chip: forward CLT with aberration correction, the tile's camera-pair
  * correlations and its texture, one tile at a time per block.
  *
+ * It serves the calls that give no workspace for the CLT or want it written out;
+ * with one the frame runs in stages (process_frame in tp_api.cu), faster at every
+ * size: here each phase takes the registers and shared memory of the largest.
+ *
  * This has no single counterpart in the reference, which runs the three
  * stages as separate kernels through a 963 MB CLT buffer in device memory
  * (convert_correct_tiles, correlate2D, textures_accumulate via generate_RBGA:

@@ -270,9 +270,12 @@ __global__ void k_woi_finalize(int *woi)
  * 8 floats a thread writes past them when the grid reaches that far, over
  * (woi_h + 1) * 8 * (colors + 1) rows.  woi == NULL: explicit extent. */
 __global__ void k_clear_rbga(const int *woi, int colors, int texture_width, int slice_height,
-                             size_t stride, float *buf)
+                             size_t stride, float *buf, int *zero, int nzero)
 {
     chain_entry();
+    /* process_frame's list counts */
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < nzero; i += blockDim.x) zero[i] = 0;
     int tw = texture_width, rows = slice_height;
     if (woi) {
         tw = (woi[2] + 1) * 8;

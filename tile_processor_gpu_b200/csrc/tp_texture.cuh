@@ -497,14 +497,15 @@ static_assert(sizeof(float) * 16 * tex_job(1) <= kTexSmemBytes, "mono fits the s
  * copies the tile into shared memory instead of inverting the CLT.
  * ALL: the texture-tile outputs and the keep-weights statistics are built
  * (false: the RGBA image only).  COLORS: the colour count, 1 or 3 (p.colors;
- * a compile-time count lets each form keep only its own colour path). */
-template <bool FROM_T, bool ALL, int COLORS>
+ * a compile-time count lets each form keep only its own colour path).  SLOTS: the
+ * CLT and the list lie in the frame's workspace (FrameSlots; one parity a launch). */
+template <bool FROM_T, bool ALL, int COLORS, bool SLOTS = false>
 __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
     Geom g, const int *__restrict__ woi, float *const *clt, int num_texture_tiles,
     const int *__restrict__ list, const int *__restrict__ dev_counts, int count_slot, int list_cap,
     int border_quarter, const float *__restrict__ port_offsets, TextureParams p,
     size_t texture_rbg_stride, float *__restrict__ texture_rbg, size_t texture_stride,
-    float *__restrict__ texture_tiles)
+    float *__restrict__ texture_tiles, FrameSlots slots)
 {
     extern __shared__ __align__(16) float smem[];
     __shared__ float *s_cp[4];
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
     const int cam = job / colors, color = job - cam * colors;
     /* -1 / (2 sigma^2) times log2(e): the fusion's weights are powers of two */
     const float nksigma = -((float)(1.0 / (2.0 * (double)p.diff_sigma * (double)p.diff_sigma)) * kLog2e);
-    if (tid < 4) s_cp[tid] = clt[tid];
+    if (tid < 4) s_cp[tid] = SLOTS ? slots.clt + tid * 768 : clt[tid];
     if (tid == 0) {
         int k = 0;
         for (int i = 0; i < 4; i++)
@@ -573,8 +574,13 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
     const int ntiles = g.TX * g.TY;
     /* entry n of this pass: its code, or 0 when there is none or it is not a
      * texture tile */
-    auto entry = [&](int n) -> int {
+    auto entry = [&](int n, int &at) -> int {
         if (n >= count) return 0;
+        if (SLOTS) {
+            const int2 e = slots.list[n];
+            at = e.x;
+            return e.y;
+        }
         const int code = lst[n + (n >= split ? gap : 0)], tile = code >> 8;
         return ((code & (1 << 7)) && tile >= 0 && tile < ntiles) ? code : 0;
     };
@@ -602,17 +608,21 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * 768 floats per camera, mono 8 lines of 256) and, after the fusion, the
      * RGBA rows their pixels update (both ends of each 16-pixel row of each
      * slice; the previous pass, which writes them, has completed by then). */
+    constexpr int kTileStride = SLOTS ? kSlot : 768;
     constexpr int kLines = colors == 3 ? 24 : 8;
-    auto prefetch_clt = [&](const int *codes) {
+    auto prefetch_clt = [&](const int *codes, const int *ats) {
         const int t = colors == 3 ? 0 : tid >> 5, k = colors == 3 ? tid : tid & 31;
         if (k >= 4 * kLines) return;
-        int code = 0;
+        int code = 0, at = 0;
 #pragma unroll
         for (int i = 0; i < kTiles; i++)
-            if (t == i) code = codes[i];
+            if (t == i) {
+                code = codes[i];
+                if (SLOTS) at = ats[i];
+            }
         if (!code) return;
         const int pcam = k / kLines, line = k - pcam * kLines;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(s_cp[pcam] + (size_t)(code >> 8) * 768 + line * 32));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(s_cp[pcam] + (size_t)(SLOTS ? at : code >> 8) * kTileStride + line * 32));
     };
     auto prefetch_rgba = [&](int code, int gy0, int gx0) {
         /* row r of slice sl */
@@ -625,7 +635,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             asm volatile("prefetch.global.L2 [%0];" ::"l"(b + 15));
         }
     };
-    /* this group's entry of a block's codes (0: none) */
+    /* this group's entry of a block's codes or places (0: none) */
     auto pick = [&](const int *codes) -> int {
         int code = 0;
 #pragma unroll
@@ -633,8 +643,8 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             if (sub == i) code = codes[i];
         return code;
     };
-    auto job_clt = [&](int code) -> const float * {
-        return s_cp[cam] + ((size_t)(code >> 8) * 3 + color) * 256;
+    auto job_clt = [&](int code, int at) -> const float * {
+        return s_cp[cam] + ((size_t)(SLOTS ? at : code >> 8) * (kTileStride / 256) + color) * 256;
     };
 
     /* the next tile-parity pass may be scheduled on the SM slots this grid
@@ -647,16 +657,16 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * Everything they read (the list and its counts, the window, the CLT, the
      * port offsets) was complete before that launch let this one start. */
     bool waited = false;
-    int codes[kTiles], gy0 = 0, gx0 = 0;
+    int codes[kTiles], ats[kTiles] = {}, gy0 = 0, gx0 = 0;
 #pragma unroll
-    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x * kTiles + i);
-    int mine = pick(codes);
+    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x * kTiles + i, ats[i]);
+    int mine = pick(codes), mine_at = pick(ats);
     if (colors == 3 && want_rbg) rgba_origin(codes[0] >> 8, &gy0, &gx0);
 
     for (int n = (int)blockIdx.x * kTiles; n < count; n += (int)gridDim.x * kTiles) {
-        int next[kTiles];
+        int next[kTiles], next_at[kTiles] = {};
 #pragma unroll
-        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * kTiles + i);
+        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * kTiles + i, next_at[i]);
 
         /* ---- stages 1-2: per (tile, camera, color) group ---- */
         if (mine) {
@@ -666,7 +676,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
             if (FROM_T) {
                 /* lane l: columns 2 l and 2 l + 1 of every row pair (a row of the
                  * group's loads is 64 bytes, its stores 16 bytes a lane) */
-                const float *src = job_clt(mine) + 2 * l;
+                const float *src = job_clt(mine, mine_at) + 2 * l;
                 const bool al8 = !(reinterpret_cast<uintptr_t>(src) & 7);
                 float4 *t4 = reinterpret_cast<float4 *>(tj);
                 float2 v[8][2];
@@ -690,13 +700,13 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
                 }
             } else {
                 float raw[4][8];
-                load_clt_rows<true>(job_clt(mine), raw, l);
+                load_clt_rows<true>(job_clt(mine, mine_at), raw, l);
                 imclt_unfold_job<COLORS == 1>(raw, d_lpf[colors > 1 ? color : 3], tj, tj, t, l, gm);
             }
             if (colors > 1) debayer_job<ALL>(t, tj, dj, color < 2, p.min_shot, p.scale_shot, l, gm);
         }
         __syncthreads();
-        prefetch_clt(next);
+        prefetch_clt(next, next_at);
         if (!waited) {
             grid_dependency_wait();
             waited = true;
@@ -764,6 +774,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
 #pragma unroll
         for (int i = 0; i < kTiles; i++) codes[i] = next[i];
         mine = pick(codes);
+        mine_at = pick(next_at);
         if (want_rbg) {
             if (colors == 3) {
                 rgba_origin(codes[0] >> 8, &gy0, &gx0);
