@@ -757,19 +757,22 @@ static int process_frame(const tp_geometry *g, float *const *kernel_offsets, flo
     if (staged) {
         if ((rc = texture_smem_setup())) return rc;
         cudaError_t err = cudaSuccess;
-        /* The textures start while the correlations end (both read the CLT, which
-         * was complete when the correlations started); the next part's forward
-         * transform, an ordinary launch, follows them all. */
+        /* A chain of programmatic dependents.  The forward transform and the
+         * correlations wait on entry for the launch before them and release their
+         * dependent only then, so the textures start while the correlations end,
+         * with the CLT and the lists complete; the next part's forward transform
+         * starts its work when the last pass is complete (512x384 77.2 -> 73.5 us, 64x64
+         * 37.1 -> 35.8 against ordinary launches of the two). */
         for (int i = 0; i < chunks && err == cudaSuccess; i++, slots.counts += 4) {
             const tp_task *t = tasks + (size_t)i * kFrameChunk;
             const int n = num_tiles - i * kFrameChunk < kFrameChunk ? num_tiles - i * kFrameChunk : kFrameChunk;
             const ConvertShape cs = convert_shape(n, sms);
-            err = launch_chained(false, cs.grid, tp::kConvertThreads, 0, s,
+            err = launch_chained(true, cs.grid, tp::kConvertThreads, 0, s,
                                  cs.small ? tp::k_convert_correct_tiles<1, true> : tp::k_convert_correct_tiles<3, true>,
                                  gd, dstride, kernel_offsets, kernels, images, t, (float *const *)nullptr, n, lpf_mask,
                                  slots);
             if (err == cudaSuccess)
-                err = launch_chained(false, grid_for(6LL * n, tp::kCorrThreads / 8, sms, shape_per_sm(TP_SHAPE_CORRELATE)), tp::kCorrThreads, 0, s,
+                err = launch_chained(true, grid_for(6LL * n, tp::kCorrThreads / 8, sms, shape_per_sm(TP_SHAPE_CORRELATE)), tp::kCorrThreads, 0, s,
                                      tp::k_correlate2D<true>, gd, (float *const *)nullptr, corr_colors, corr_scale0,
                                      corr_scale1, corr_scale2, fat_zero, 6LL * n, (const int *)nullptr, corr_stride,
                                      corr_radius, corrs + (size_t)i * kFrameChunk * 6 * corr_stride, t,

@@ -436,6 +436,12 @@ __global__ void __launch_bounds__(kConvertThreads, 3) k_convert_correct_tiles(
     const int l = threadIdx.x & 7;
     const int grp = threadIdx.x >> 3;
     const unsigned gm = group_mask();
+    /* a programmatic dependent of the RGBA clear (or of the part before, whose
+     * workspace it takes over); the correlations may be scheduled behind it */
+    if (SLOTS) {
+        grid_dependency_wait();
+        grid_dependents_launch();
+    }
     const int step = gridDim.x * (blockDim.x >> 5);
     const int items = ((num_tiles + 3) >> 2) * (12 / PER);
     /* a task of the list as this group sees it: its tile (-1: none) and centre */

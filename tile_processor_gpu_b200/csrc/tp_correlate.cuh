@@ -232,8 +232,13 @@ __global__ void __launch_bounds__(kCorrThreads, 4) k_correlate2D(Geom g, float *
     const unsigned gm = group_mask();
     const long long groups_total = (long long)gridDim.x * (blockDim.x >> 3);
     const int ntiles = g.TX * g.TY;
-    /* the frame's textures may fill the SM slots this grid frees */
-    if (SLOTS) grid_dependents_launch();
+    /* a programmatic dependent of the forward transform; only once that is complete
+     * the frame's textures, which read its CLT and lists too, may fill the SM
+     * slots this grid frees */
+    if (SLOTS) {
+        grid_dependency_wait();
+        grid_dependents_launch();
+    }
     for (long long n = (long long)blockIdx.x * (blockDim.x >> 3) + grp; n < num_corr_tiles; n += groups_total) {
         const float *ta, *tb2;
         if (SLOTS) {
