@@ -22,7 +22,6 @@ namespace tp {
 
 /* ---- constant tables (generated by gen_tables.py) -------------------------- */
 __device__ __constant__ float c_hwin[16] = TP_HWIN_INIT;
-__device__ __constant__ float c_hwinc[16] = TP_HWINC_INIT;
 /* Tables that lanes index by their own row / column live in global memory
  * and are read through the read-only data cache: the lanes of a warp then
  * fetch distinct words in one pass, where the constant cache would serialise
@@ -45,26 +44,11 @@ struct Geom {
     int debug_marks;
 };
 
-/* Per-group buffer for four 8x9 quadrant transposes, padded to 296 floats
- * (296 % 32 == 8) so that the four groups of a warp hit distinct banks. */
-constexpr int kTB4 = 4 * 72 + 8;
-#define TBI(q, r, c) ((q) * 72 + (r) * 9 + (c))
-
 __device__ __forceinline__ unsigned group_mask() { return 0xffu << (threadIdx.x & 24); }
-
-/* One (camera, colour) CLT tile staged in shared memory: 256 coefficients
- * padded to 264 floats (264 % 32 == 8, 16-byte multiple), so the four groups
- * of a warp reading column l of their own job hit distinct banks. */
-constexpr int kCltJob = 264;
 
 /* Asynchronous global -> shared copies (LDGSTS).  Completion is awaited with
  * cp_async_wait_all() by the issuing thread; other threads see the data after
  * a following block barrier. */
-__device__ __forceinline__ void cp_async16(void *sdst, const void *gsrc)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async4(void *sdst, const void *gsrc)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
@@ -272,19 +256,6 @@ __device__ __forceinline__ void dtt8(const float x[8], float y[8])
         dct2_fast<KIND == 3>(x, y);
 }
 
-/* 8x8 transpose inside an 8-lane group through an 8x9 buffer: lane l
- * contributes row l (in[0..7]) and receives column l (out[0..7]). */
-__device__ __forceinline__ void group_transpose(float (*buf)[9], const float in[8], float out[8], int l,
-                                                unsigned gm)
-{
-#pragma unroll
-    for (int k = 0; k < 8; k++) buf[l][k] = in[k];
-    __syncwarp(gm);
-#pragma unroll
-    for (int k = 0; k < 8; k++) out[k] = buf[k][l];
-    __syncwarp(gm);
-}
-
 /* window sample n -> DTT index (4..7, 7..4, 3..0, 0..3) and back: the two
  * samples that fold onto index u have opposite parity; return the one with
  * parity p. */
@@ -295,17 +266,7 @@ __device__ __forceinline__ int fold_sample(int u, int p)
     return ((a & 1) == p) ? a : b;
 }
 
-/* sign of the cosine / sine fold branch for window sample n */
-__device__ __forceinline__ float fold_sign_c(int n) { return n < 4 ? 1.0f : -1.0f; }
-__device__ __forceinline__ float fold_sign_s(int n) { return n < 12 ? 1.0f : -1.0f; }
-
-/* window value w(n + s) = sin(pi (2 (n + s) + 1) / 32) from (cos, sin)(pi s / 16);
- * n uniform across the warp */
-__device__ __forceinline__ float shifted_window(int n, float cs, float sn)
-{
-    return __fmaf_rn(c_hwin[n], cs, c_hwinc[n] * sn);
-}
-/* the same with a lane-dependent n */
+/* window value w(n + s) = sin(pi (2 (n + s) + 1) / 32) from (cos, sin)(pi s / 16) */
 __device__ __forceinline__ float shifted_window_lane(int n, float cs, float sn)
 {
     return __fmaf_rn(__ldg(&d_hwin[n]), cs, __ldg(&d_hwinc[n]) * sn);

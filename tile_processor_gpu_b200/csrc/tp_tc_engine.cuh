@@ -107,13 +107,6 @@ struct TcA {
         *reinterpret_cast<uint4 *>(img + off) = make_uint4(h[0], h[1], h[2], h[3]);
         *reinterpret_cast<uint4 *>(img + Q * kTcQuadBytes + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
-    /* zeros for row r, quadrant q, halves k0 .. k0 + 7 */
-    __device__ __forceinline__ void zero8(int r, int q, int k0) const
-    {
-        const uint32_t off = (uint32_t)q * kTcQuadBytes + tc_sw_off(r, k0);
-        *reinterpret_cast<uint4 *>(img + off) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4 *>(img + Q * kTcQuadBytes + off) = make_uint4(0u, 0u, 0u, 0u);
-    }
 };
 
 /* The 12 Q MMAs of one block: for each quadrant, A_hi B_hi, A_hi B_lo, A_lo

@@ -145,16 +145,4 @@ __device__ __forceinline__ float to_tf32(float x)
 }
 
 
-/* tcgen05.ld of 8 consecutive TMEM columns of this thread's lane, one wait */
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, float v[8])
-{
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
-}
-
 } /* namespace tp */
