@@ -634,8 +634,8 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
     /* The RGBA clear and the four passes continue prepare_list's chain of
      * programmatic dependents.  The clear waits on entry for the list's last
      * kernel and releases its dependent only after that wait.  A pass releases
-     * its own dependent on entry, then prefetches its first tile's CLT and
-     * reads the list, and only then waits for the launch before it (the
+     * its own dependent on entry, then reads the list and inverts and debayers
+     * its first tile, and only then waits for the launch before it (the
      * clear, or the previous pass, which read-modify-writes the RGBA image).
      * So a pass can start only after every earlier pass has started, and the
      * first pass only after the clear released it, which the clear did once

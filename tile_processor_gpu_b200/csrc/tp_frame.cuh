@@ -25,7 +25,7 @@
  *      un-windowed tile T in place of the job's CLT, debayer into D;
  *   4. fusion of the four cameras at the block's 256 pixels, faded by the
  *      neighbour mask and added into the overlapped RGBA image.
- * Idle groups in one phase leave their issue slots to the other six blocks
+ * Idle groups in one phase leave their issue slots to the other four blocks
  * of the SM, which are in other phases.
  *
  * The frame runs as four launches, one per 2x2 tile parity, so the tiles of

@@ -2,7 +2,7 @@
  * tp_gemm_tc.cuh - the learned residual's training GEMM on the tensor cores:
  * C = op(A) op(B) (+ bias, + beta C, optional pre-activation z and GELU), the
  * operation of k_gemm, with FP32 operands split into two TF32 parts,
- *   x = hi + lo,  hi = tf32(x),  lo = tf32(x - hi),
+ *   x = hi + lo,  hi = tf32(x),  lo = x - hi (the MMA reads its TF32 bits),
  * and each product formed as three tcgen05 TF32 MMAs, A_hi B_hi + A_hi B_lo +
  * A_lo B_hi (about 21 significant bits per operand; the dropped A_lo B_lo
  * term is below 2^-21 of a product).  Each K chunk of 32 is accumulated in

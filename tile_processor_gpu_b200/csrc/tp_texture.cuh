@@ -4,10 +4,11 @@
  * :3847-4017, debayer_shot / debayer :4019-4199 and tile_combine_rgba
  * :4202-4665).
  *
- * One 128-thread block per listed tile (mono: per four tiles), grid-stride.  The CLT is read straight from global memory by the inverse
- * transform; the next tile's CLT and the RGBA rows it will update are
- * prefetched into L2 while the block works on the current tile.  Per
- * (camera, colour) job one 8-lane group, working only with __syncwarp on its
+ * One 128-thread block per listed tile (mono: per four tiles), grid-stride.
+ * The CLT is read straight from global memory by the inverse transform; the
+ * next tile's CLT and the RGBA rows it will update are prefetched into L2 while
+ * the block works on the current tile.  Per (camera, colour) job one 8-lane
+ * group, working only with __syncwarp on its
  * own buffers:
  *   1. low-pass filter and invert the CLT tile (horizontal DCT-IV/DST-IV on
  *      the held rows, transpose, vertical pass on the held column) and unfold
@@ -24,10 +25,10 @@
  * (add2 / mul2 / fma2): two quadrants per pair in the transforms, two rows of
  * a column per pair from the unfold on.  The RGBA-only colour form takes 4776
  * warp instructions a tile (7238 in scalar form); the four passes of a
- * 2592x1936 frame with their list and clear went from 0.787 to 0.614 ms.
+ * 2592x1936 frame with their list and clear went from 0.787 to 0.607 ms.
  * Seven blocks of four warps share an SM; three-warp blocks (no idle warp
- * in the transforms, but two turns of the fusion for one warp) took 0.671.  Tiles in shared memory hold pairs of
- * rows: pair (rp, c) = rows 2 rp and 2 rp + 1 of column c at float2 16 rp + c,
+ * in the transforms, but two turns of the fusion for one warp) took 0.671.
+ * Tiles in shared memory hold pairs of rows: pair (rp, c) = rows 2 rp and 2 rp + 1 of column c at float2 16 rp + c,
  * so a warp of the fusion reads two row pairs of 16 columns in 64-bit loads
  * without a bank conflict and its RGBA accesses stay whole 64-byte rows.
  */
