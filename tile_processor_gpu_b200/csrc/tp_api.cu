@@ -639,7 +639,11 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
      * clear, or the previous pass, which read-modify-writes the RGBA image).
      * So a pass can start only after every earlier pass has started, and the
      * first pass only after the clear released it, which the clear did once
-     * the list was complete: every pass reads a finished list. */
+     * the list was complete: every pass reads a finished list.  With the
+     * inverse transform on the tensor cores in between, the first pass reads
+     * the pixel tiles that kernel writes, before its wait: it is an ordinary
+     * launch, which starts when those tiles are complete, and the later passes
+     * start after it. */
     {
         const int max_rows = (gd.TY + 1) * 8 * (colors + 1);
         const cudaError_t err = launch_chained(true, grid_for(max_rows, 1, sms, 16), 256, 0, s, tp::k_clear_rbga,
@@ -663,9 +667,10 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
     for (int parity = 0; parity < 4; parity++) {
         const int *base = texture_indices + parity * quarter;
         const cudaError_t err =
-            launch_chained(true, grid, tp::kTexThreads, tp::kTexSmemBytes, s, tex, gd, (const int *)woi, src, 0,
-                           (const int *)base, (const int *)num_texture_tiles, parity << 1, quarter, -quarter,
-                           port_offsets, p, texture_rbga_stride, texture_tiles, (size_t)0, (float *)nullptr, tp::FrameSlots{});
+            launch_chained(format < 0 || parity > 0, grid, tp::kTexThreads, tp::kTexSmemBytes, s, tex, gd,
+                           (const int *)woi, src, 0, (const int *)base, (const int *)num_texture_tiles, parity << 1,
+                           quarter, -quarter, port_offsets, p, texture_rbga_stride, texture_tiles, (size_t)0,
+                           (float *)nullptr, tp::FrameSlots{});
         if (err != cudaSuccess) return cuda_status(err, "generate_RBGA texture pass launch");
     }
     return cuda_status(cudaGetLastError(), "generate_RBGA launch");

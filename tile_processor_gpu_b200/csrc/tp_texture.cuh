@@ -652,11 +652,15 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * frees as its blocks finish */
     grid_dependents_launch();
     /* A pass launched as a programmatic dependent of the launch before it (the
-     * RGBA clear, or the previous tile-parity pass) waits for it before its
-     * first access to the RGBA image, which that launch writes; the inverse
-     * transform and debayer of its first tiles run before that wait.
-     * Everything they read (the list and its counts, the window, the CLT, the
-     * port offsets) was complete before that launch let this one start. */
+     * RGBA clear, the correlations of the frame in stages, or the previous
+     * tile-parity pass) waits for it before its first access to the RGBA image,
+     * which that launch or one before it writes; the inverse transform and
+     * debayer of its first tiles run before that wait.  So a launch may be the
+     * predecessor of a dependent pass only if everything those steps read (the
+     * list and its counts, the window, the CLT or the pixel tiles, the port
+     * offsets) was complete before it let the pass start.  The tensor-core
+     * inverse transform (FROM_T), which writes the pixel tiles, is not: the
+     * first pass after it is an ordinary launch. */
     bool waited = false;
     int codes[kTiles], ats[kTiles] = {}, gy0 = 0, gx0 = 0;
 #pragma unroll
