@@ -36,10 +36,13 @@ __device__ __forceinline__ void chain_entry()
     grid_dependents_launch();
 }
 
-/* all threads of the cluster; orders their global and shared accesses */
+/* all threads of the cluster; orders their global and shared accesses.  Not the
+ * .aligned forms: those want a warp's threads to execute them together, and
+ * nothing makes the threads of a warp meet again after the loops before the
+ * barriers, which they leave one by one. */
 __device__ __forceinline__ void cluster_sync()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
 __device__ __forceinline__ int marker_at(const int *idx, long long i, long long cap)
