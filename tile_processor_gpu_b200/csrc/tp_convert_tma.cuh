@@ -18,10 +18,10 @@
  *     host);
  *     one lane per item arms the slot's `full` mbarrier with the item's bytes;
  *   consumer warp c: items c, c + kCvConsumers, ...; waits for the slot,
- *     folds the four jobs (one 8-lane group each) from the staged windows
- *     (border windows: the global-memory path with the reference's clamps),
- *     releases the slot (its `empty` mbarrier) and finishes the jobs
- *     (transforms, convolution, shifts, store) while the producer refills it.
+ *     reads the four jobs' samples (one 8-lane group each) from the staged
+ *     windows (border windows: the global-memory path with the reference's
+ *     clamps), releases the slot (its `empty` mbarrier) and does the jobs (fold,
+ *     transforms, convolution, shifts, store) while the producer refills it.
  * Every wait is bounded; one that runs out sets *err and stops the block's
  * work (the CLT is then incomplete); the producer waits (bounded) for its
  * last loads before it exits.
@@ -32,7 +32,11 @@
 
 namespace tp {
 
-constexpr int kCvConsumers = 8;
+/* Seven consumers: two blocks share an SM (see kCvSmemBytes) with registers for
+ * a job without spills.  With eight the ring and the fold's buffers fit an SM
+ * once: 3.24 ms for a 2592x1936 frame, 1.67 this way (the producers' row copies
+ * bound it: the plain kernel takes 0.33). */
+constexpr int kCvConsumers = 7;
 constexpr int kCvThreads = 32 * (kCvConsumers + 1);
 constexpr int kCvSlots = 2 * kCvConsumers;
 constexpr int kCvBatch = 8; /* items per producer pass: 32 lanes = 8 items x 4 tasks */
@@ -50,6 +54,9 @@ struct __align__(16) CvMeta {
 };
 
 constexpr size_t kCvSmemBytes = (size_t)kCvSlots * 4 * (kCvWinBytes + sizeof(CvMeta)) + 128;
+/* two blocks on an SM: 228 KB, of which each block takes 1 KB beside its own */
+static_assert(2 * (kCvSmemBytes + sizeof(float) * kCvConsumers * 4 * kCvBuf + 16 * kCvSlots + 1024) <= 228 * 1024,
+              "two blocks of k_convert_tma share an SM");
 
 __device__ __forceinline__ void cv_arrive(uint32_t mbar)
 {
@@ -119,7 +126,7 @@ __global__ void __launch_bounds__(kCvThreads, 2) k_convert_tma(
                         m.txy = txy;
                         m.jg = job_geometry(g, kernel_offsets[cam], __ldg(&t->xy[cam][0]), __ldg(&t->xy[cam][1]),
                                             color, nullptr);
-                        /* the in-image condition of fold_rows, and rows that start on
+                        /* the in-image condition of load_pixels, and rows that start on
                          * 16-byte boundaries for the bulk copies */
                         m.fast = (m.jg.itlx >= 0) && (m.jg.itlx < g.W - 16) && (m.jg.itly >= 0) &&
                                  (m.jg.itly < g.H - 16) && !(dstride & 3) &&
