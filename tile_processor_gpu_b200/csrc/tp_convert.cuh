@@ -226,35 +226,77 @@ __device__ __forceinline__ void fold_cols(const JobGeometry &j, const JobAngles 
     }
 }
 
-/* Row l of the four quadrants of a kernel tile (p: row l of the first),
- * read-only for the whole launch: one 256-bit load each where the tile lies on
- * a 32-byte boundary */
-__device__ __forceinline__ void load_kernel_rows(const float *p, float2 v[4][4])
+/* Lane l's part of the four quadrants of a kernel tile, read-only for the whole
+ * launch.  True: row l, one 256-bit load each where the tile lies on a 32-byte
+ * boundary, two of 16 bytes on a 16-byte one.  Else column l (a load of the
+ * group is a run of 32 bytes), which kernel_rows turns into row l when the rows
+ * are needed. */
+__device__ __forceinline__ bool load_kernel(const float *tile, int l, float2 v[4][4])
 {
-    if (!(reinterpret_cast<uintptr_t>(p) & 31)) {
+    const float *p = tile + l * 8;
+    if (!(reinterpret_cast<uintptr_t>(tile) & 31)) {
 #pragma unroll
         for (int q = 0; q < 4; q++)
             asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                          : "=f"(v[q][0].x), "=f"(v[q][0].y), "=f"(v[q][1].x), "=f"(v[q][1].y), "=f"(v[q][2].x),
                            "=f"(v[q][2].y), "=f"(v[q][3].x), "=f"(v[q][3].y)
                          : "l"(p + q * 64));
-    } else {
+        return true;
+    }
+    if (!(reinterpret_cast<uintptr_t>(tile) & 15)) {
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int k = 0; k < 4; k++) v[q][k] = make_float2(__ldg(p + q * 64 + 2 * k), __ldg(p + q * 64 + 2 * k + 1));
+            for (int k = 0; k < 2; k++) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(p + q * 64) + k);
+                v[q][2 * k] = make_float2(x.x, x.y);
+                v[q][2 * k + 1] = make_float2(x.z, x.w);
+            }
+        return true;
+    }
+    p = tile + l;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            v[q][k] = make_float2(__ldg(p + q * 64 + 16 * k), __ldg(p + q * 64 + 16 * k + 8));
+    return false;
+}
+
+/* columns of load_kernel to rows, through tr (200 floats of the group's) */
+__device__ __forceinline__ void kernel_rows(float2 v[4][4], float *tr, int l, unsigned gm)
+{
+#pragma unroll
+    for (int q = 0; q < 4; q += 2) {
+        __syncwarp(gm);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                tr[(8 * h + 2 * k) * kCvTrRow + l] = v[q + h][k].x;
+                tr[(8 * h + 2 * k + 1) * kCvTrRow + l] = v[q + h][k].y;
+            }
+        __syncwarp(gm);
+#pragma unroll
+        for (int h = 0; h < 2; h++) lds_row(tr + (8 * h + l) * kCvTrRow, v[q + h]);
     }
 }
 
-/* Row l of the four quadrants of a result (p: row l of the first).  STREAM:
+/* Row l of the four quadrants of a result at out.  STREAM:
  * global memory, evict-first (the kernel writes 963 MB of CLT for a full quad
  * frame, far more than L2 holds, and later kernels read it back; retaining the
  * stores in L2 would only evict the kernel tiles and Bayer rows that
- * neighbouring jobs of this kernel still read); else shared memory, 16-byte
- * aligned */
+ * neighbouring jobs of this kernel still read): 32 bytes a lane where the tile
+ * lies on a 32-byte boundary, two times 16 on a 16-byte one, else through tr
+ * (200 floats of the group's), so that a store of the group is a run of 32
+ * bytes; !STREAM: shared memory, 16-byte aligned.  A 2592x1936 frame (0.326 ms
+ * aligned) with kernel tables and CLT 16 / 8 / 4 bytes off such a boundary takes
+ * 0.386 / 0.496 / 0.496 ms; 0.699 / 0.666 / 0.649 with a lane's row moved value
+ * by value in both directions. */
 template <bool STREAM>
-__device__ __forceinline__ void store_rows(float *p, const float2 v[4][4])
+__device__ __forceinline__ void store_rows(float *out, const float2 v[4][4], float *tr, int l, unsigned gm)
 {
+    float *p = out + l * 8;
     if (!STREAM) {
 #pragma unroll
         for (int q = 0; q < 4; q++)
@@ -269,23 +311,36 @@ __device__ __forceinline__ void store_rows(float *p, const float2 v[4][4])
                          "f"(v[q][0].x), "f"(v[q][0].y), "f"(v[q][1].x), "f"(v[q][1].y), "f"(v[q][2].x),
                          "f"(v[q][2].y), "f"(v[q][3].x), "f"(v[q][3].y)
                          : "memory");
-    } else {
+    } else if (!(reinterpret_cast<uintptr_t>(p) & 15)) {
 #pragma unroll
         for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                __stcs(p + q * 64 + 2 * k, v[q][k].x);
-                __stcs(p + q * 64 + 2 * k + 1, v[q][k].y);
-            }
+            for (int k = 0; k < 2; k++)
+                __stcs(reinterpret_cast<float4 *>(p + q * 64) + k,
+                       make_float4(v[q][2 * k].x, v[q][2 * k].y, v[q][2 * k + 1].x, v[q][2 * k + 1].y));
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            __syncwarp(gm);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    reinterpret_cast<float4 *>(tr + (8 * h + l) * kCvTrRow)[k] =
+                        make_float4(v[q + h][2 * k].x, v[q + h][2 * k].y, v[q + h][2 * k + 1].x, v[q + h][2 * k + 1].y);
+            __syncwarp(gm);
+#pragma unroll
+            for (int r = 0; r < 16; r++) __stcs(out + q * 64 + r * 8 + l, tr[r * kCvTrRow + l]);
+        }
     }
 }
 
-/* The rest of a job after its fold (fold_cols: P, Q, the rotations in buf; kq:
- * row l of its kernel tile): 2-D transform, CLT-domain convolution with the kernel tile, residual
+/* The rest of a job after its fold (fold_cols: P, Q, the rotations in buf; kq,
+ * rows: its kernel tile as load_kernel leaves it): 2-D transform, CLT-domain convolution with the kernel tile, residual
  * shifts, LPF, store. */
 template <bool STREAM>
 __device__ __forceinline__ void convert_finish(const JobGeometry &jg, const JobAngles &ang, int color, int lpf_mask, float *__restrict__ out,
-                                               float *buf, int l, unsigned gm, const float2 kq[4][4],
+                                               float *buf, int l, unsigned gm, float2 kq[4][4], bool rows,
                                                const float2 P[4], const float2 Q[4])
 {
     const int itlx = jg.itlx, itly = jg.itly;
@@ -357,6 +412,7 @@ __device__ __forceinline__ void convert_finish(const JobGeometry &jg, const JobA
     /* ---- CLT-domain convolution (src/TileProcessor.cuh:2778-2827), then the
      * residual shift: horizontal (per column, shared across the group), then
      * vertical (this lane's row) (:2715-2776) ---- */
+    if (!rows) kernel_rows(kq, tr, l, gm);
     float2 ch[4], sh[4];
     lds_row(buf + kCvRot, ch);
     lds_row(buf + kCvRot + 8, sh);
@@ -386,7 +442,7 @@ __device__ __forceinline__ void convert_finish(const JobGeometry &jg, const JobA
 #pragma unroll
             for (int k = 0; k < 4; k++) o[q][k] = mul2(o[q][k], f[k]);
     }
-    store_rows<STREAM>(out + l * 8, o);
+    store_rows<STREAM>(out, o, tr, l, gm);
     __syncwarp(gm); /* buf free for the group's next job */
 }
 
@@ -404,11 +460,11 @@ __device__ __forceinline__ void convert_job(const Geom &g, size_t dstride,
     float pix[2][8];
     load_pixels(g, dstride, img, jg, color, l, pix);
     float2 kq[4][4];
-    load_kernel_rows(kern_tab + jg.kidx * 256 + l * 8, kq);
+    const bool rows = load_kernel(kern_tab + jg.kidx * 256, l, kq);
     const JobAngles ang = job_angles(jg, l);
     float2 P[4], Q[4];
     fold_cols(jg, ang, color, l, gm, buf, pix, P, Q);
-    convert_finish<STREAM>(jg, ang, color, lpf_mask, out, buf, l, gm, kq, P, Q);
+    convert_finish<STREAM>(jg, ang, color, lpf_mask, out, buf, l, gm, kq, rows, P, Q);
 }
 
 /* A warp's item of the grid-stride loop is four consecutive tasks of one camera

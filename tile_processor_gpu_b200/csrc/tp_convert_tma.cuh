@@ -189,10 +189,10 @@ __global__ void __launch_bounds__(kCvThreads, 2) k_convert_tma(
                 const int tx = m.txy & 0xfff, ty = m.txy >> 16;
                 float *out = clt[cam] + (((size_t)ty * g.TX + tx) * 3 + color) * 256;
                 float2 kq[4][4], P[4], Q[4];
-                load_kernel_rows(kernels[cam] + m.jg.kidx * 256 + l * 8, kq);
+                const bool rows = load_kernel(kernels[cam] + m.jg.kidx * 256, l, kq);
                 const JobAngles ang = job_angles(m.jg, l);
                 fold_cols(m.jg, ang, color, l, gm, cbuf[warp * 4 + grp], pix, P, Q);
-                convert_finish<true>(m.jg, ang, color, lpf_mask, out, cbuf[warp * 4 + grp], l, gm, kq, P, Q);
+                convert_finish<true>(m.jg, ang, color, lpf_mask, out, cbuf[warp * 4 + grp], l, gm, kq, rows, P, Q);
             }
         }
     }
