@@ -169,7 +169,7 @@ struct FwdTcStage {
         const float *kr = valid ? kernels[cam] + (size_t)meta[1] * 256 : nullptr;
         float *out = valid ? clt[cam] + ((size_t)meta[3] * 3 + color) * 256 : nullptr;
         const bool k32 = !(reinterpret_cast<uintptr_t>(kr) & 31), k16 = !(reinterpret_cast<uintptr_t>(kr) & 15);
-        const bool o32 = !(reinterpret_cast<uintptr_t>(out) & 31);
+        const bool o32 = !(reinterpret_cast<uintptr_t>(out) & 31), o16 = !(reinterpret_cast<uintptr_t>(out) & 15);
 #pragma unroll 1
         for (int mm = 0; mm < 2; mm++) {
             const int m = 2 * part + mm;
@@ -229,6 +229,9 @@ struct FwdTcStage {
                     float *d = out + q * 64 + i * 8;
                     if (o32) {
                         st8_global(d, o[q]);
+                    } else if (o16) {
+                        reinterpret_cast<float4 *>(d)[0] = make_float4(o[q][0], o[q][1], o[q][2], o[q][3]);
+                        reinterpret_cast<float4 *>(d)[1] = make_float4(o[q][4], o[q][5], o[q][6], o[q][7]);
                     } else {
 #pragma unroll
                         for (int j = 0; j < 8; j++) d[j] = o[q][j];

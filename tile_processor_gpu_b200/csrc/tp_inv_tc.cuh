@@ -164,6 +164,10 @@ struct InvTcStage {
                 if (!(reinterpret_cast<uintptr_t>(dst) & 31)) {
                     st8_global(dst + r * 16, o);
                     st8_global(dst + r * 16 + 8, o + 8);
+                } else if (!(reinterpret_cast<uintptr_t>(dst) & 15)) {
+                    float4 *p = reinterpret_cast<float4 *>(dst + r * 16);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) p[k] = make_float4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
                 } else {
 #pragma unroll
                     for (int c = 0; c < 16; c++) dst[r * 16 + c] = o[c];
