@@ -92,3 +92,19 @@ def test_gemm_edges(native, M, N, K, ta, tb, pad):
             assert np.max(np.abs(rows - ref)) / np.abs(ref).max() < 1e-5
         if bad is not None:
             assert not np.any(np.isfinite(got[0, :N]))
+
+
+def test_step_on_no_rows(native):
+    """A step on an empty batch (tensors without elements have no address): loss
+    0 and zero gradients, as a batch that happens to hold no tile gives."""
+    import torch
+    from tile_processor_gpu_b200 import disparity_net as D
+    net = D.DisparityMLP(D.init_params(4))
+    x, t = torch.randn((4, D.N_IN), device="cuda"), torch.randn(4, device="cuda")
+    net.forward(x, 4)
+    net.loss_backward(x, 4, t)
+    none = torch.empty((0, D.N_IN), device="cuda")
+    assert net.forward(none, 0).shape == (0, 2)
+    assert net.loss_backward(none, 0, torch.empty(0, device="cuda")) == 0.0
+    torch.cuda.synchronize()
+    assert all(not bool(net.g[k].any()) for k in D.PARAMS)

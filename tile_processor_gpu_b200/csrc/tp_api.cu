@@ -1039,8 +1039,8 @@ int tp_mlp_loss_backward(int rows, const float *x, int ldx, const float *const *
                          float *dz1, float *const *grads, int *err, tp_stream_t stream)
 {
     if (rows < 0 || ldx < kNetIn) return fail(TP_ERR_ARG, "mlp_loss_backward rows %d ldx %d", rows, ldx);
-    if (!x || !params || !z1 || !h1 || !z2 || !h2 || !out || !target || !dout || !loss_rows || !loss_sum || !dz2 ||
-        !dz1 || !grads)
+    if (!params || !loss_sum || !grads) return fail(TP_ERR_ARG, "NULL mlp_loss_backward operand");
+    if (rows && (!x || !z1 || !h1 || !z2 || !h2 || !out || !target || !dout || !loss_rows || !dz2 || !dz1))
         return fail(TP_ERR_ARG, "NULL mlp_loss_backward operand");
     for (int i = 0; i < 6; i++)
         if (!params[i] || !grads[i]) return fail(TP_ERR_ARG, "NULL mlp_loss_backward parameter %d", i);
