@@ -473,7 +473,9 @@ int tp_mlp_forward(int rows, const float *x, int ldx, const float *const *params
  * tp_mlp_forward pass: dout [rows][2], loss_rows [rows] and their sum in
  * *loss_sum (device double), dz2 [rows][128] and dz1 [rows][256] (the
  * gradients of z2 and z1), and grads (host array of six device arrays, as
- * params; overwritten).  The sums over rows are not added in a fixed order.
+ * params; overwritten).  The loss and the gradients of b1, b2, W3 and b3 are
+ * added in a fixed order and repeat bit for bit; those of W1 and W2 do where
+ * their products do not split the rows (up to 224 rows).
  * dout and loss_sum 8-byte aligned. */
 int tp_mlp_loss_backward(int rows, const float *x, int ldx, const float *const *params, const float *z1,
                          const float *h1, const float *z2, const float *h2, const float *out, const float *target,

@@ -108,3 +108,58 @@ def test_step_on_no_rows(native):
     assert net.loss_backward(none, 0, torch.empty(0, device="cuda")) == 0.0
     torch.cuda.synchronize()
     assert all(not bool(net.g[k].any()) for k in D.PARAMS)
+
+
+@pytest.mark.parametrize("rows", [1, 17, 200, 224, 1025, 4096, 5000])
+def test_step_repeats(native, rows):
+    """The loss and the gradients of the biases and of the head repeat bit for
+    bit, whatever the order blocks finish in; with up to 224 rows (no product
+    splits its K) so does every gradient.  The buffers hold other values
+    before each step."""
+    import torch
+    from tile_processor_gpu_b200 import disparity_net as D
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, D.N_IN), generator=gen, device="cuda")
+    t = torch.randn(rows, generator=gen, device="cuda")
+    net = D.DisparityMLP(D.init_params(4))
+    first = None
+    for turn in range(30):
+        for k in D.PARAMS:
+            net.g[k].fill_(float(turn + 1))
+        net.forward(x, rows)
+        loss = net.loss_backward(x, rows, t)
+        got = {k: net.g[k].clone() for k in D.PARAMS}
+        if first is None:
+            first = loss, got
+        assert loss == first[0]
+        for k in D.PARAMS:
+            if rows <= 224 or k not in ("W1", "W2"):
+                assert torch.equal(got[k], first[1][k]), (k, turn)
+
+
+@pytest.mark.parametrize("rows", [115200, 131072])
+def test_column_sums_of_long_batches(native, rows):
+    """Batches on both sides of the rule that lays the parts of b1's gradient
+    behind the head's, against FP64 sums of the step's own dz1, dz2 and dout
+    (relative 1e-5 of the sum of magnitudes, as a sum of that many values in
+    128-row parts stays far below)."""
+    import torch
+    from tile_processor_gpu_b200 import disparity_net as D
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, D.N_IN), generator=gen, device="cuda")
+    t = torch.randn(rows, generator=gen, device="cuda")
+    net = D.DisparityMLP(D.init_params(4))
+    net.forward(x, rows)
+    loss = net.loss_backward(x, rows, t)
+    net.check()
+    w = net._ws
+    for k, v in (("b1", w["dz1"]), ("b2", w["dz2"]), ("b3", w["dout"])):
+        v = v[:rows].double()
+        assert float(((net.g[k].double() - v.sum(0)).abs() / v.abs().sum(0)).max()) < 1e-5, k
+    want = float(w["loss"][:rows].double().sum()) / rows
+    assert abs(loss - want) <= 1e-12 * abs(want)
+    g3 = w["h2"][:rows].double().T @ w["dout"][:rows].double()
+    assert float((net.g["W3"].double() - g3).abs().max() / g3.abs().max()) < 1e-5
+    for k, a, b in (("W1", x, w["dz1"]), ("W2", w["h1"], w["dz2"])):
+        ref = a[:rows].double().T @ b[:rows].double()
+        assert float((net.g[k].double() - ref).abs().max() / ref.abs().max()) < 1e-5, k

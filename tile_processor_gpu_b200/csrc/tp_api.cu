@@ -1048,26 +1048,40 @@ int tp_mlp_loss_backward(int rows, const float *x, int ldx, const float *const *
         return fail(TP_ERR_ARG, "dout / loss_sum must be 8-byte aligned");
     if ((rows + tp::kGtM - 1) / tp::kGtM > 65535) return fail(TP_ERR_ARG, "mlp_loss_backward rows %d too large", rows);
     cudaStream_t s = (cudaStream_t)stream;
+    constexpr int kSizes[6] = {kNetIn * kNetH1, kNetH1, kNetH1 * kNetH2, kNetH2, kNetH2 * 2, 2};
+    if (rows == 0) {
+        cudaError_t e = cudaMemsetAsync(loss_sum, 0, sizeof(double), s);
+        for (int i = 0; i < 6 && e == cudaSuccess; i++) e = cudaMemsetAsync(grads[i], 0, sizeof(float) * kSizes[i], s);
+        return e == cudaSuccess ? TP_OK : cuda_status(e, "mlp_loss_backward clear");
+    }
     int rc, sms;
     if ((rc = sm_count(&sms))) return rc;
-    tp::TensorSet g{};
-    static const long long kSizes[6] = {kNetIn * kNetH1, kNetH1, kNetH1 * kNetH2, kNetH2, kNetH2 * 2, 2};
-    for (int i = 0; i < 6; i++) {
-        g.p[i] = grads[i];
-        g.n[i] = kSizes[i];
-    }
-    g.count = 6;
-    tp::k_zero_set<<<sms * 4, 256, 0, s>>>(g, loss_sum);
-    if (rows == 0) return cuda_status(cudaGetLastError(), "mlp_loss_backward launch");
-    tp::k_head_backward<<<(rows + tp::kHeadRows - 1) / tp::kHeadRows, 128, 0, s>>>(
-        rows, out, target, w, inv_count, h2, z2, params[4], dout, loss_rows, dz2, loss_sum, grads[4], grads[5],
-        grads[3]);
+    /* The sums over rows (b2, W3, b3; b1 in the GEMM) are formed in parts, which
+     * lie in the memory of W1's gradient until k_head_sums has added them: one
+     * part per block of the head and, where they fit behind those, one per 128
+     * rows of dz1 (more than 115,000 rows: dz1 is summed by itself). */
+    const int groups = (rows + tp::kHeadRows - 1) / tp::kHeadRows, most = 2 * sms;
+    const int chunks = (groups + most - 1) / most, blocks = (groups + chunks - 1) / chunks;
+    const int tiles = (rows + tp::kGtM - 1) / tp::kGtM;
+    float *part = grads[0], *cols1 = part + (size_t)blocks * tp::kHeadPart;
+    if ((long long)blocks * tp::kHeadPart > kSizes[0]) return fail(TP_ERR_ARG, "mlp_loss_backward on %d SMs", sms);
+    const bool cols_fit = (long long)blocks * tp::kHeadPart + (long long)tiles * kNetH1 <= kSizes[0];
+    const int used = blocks * tp::kHeadPart + (cols_fit ? tiles * kNetH1 : 0);
+    tp::k_head_backward<<<blocks < most ? most : blocks, 128, 0, s>>>(
+        rows, chunks, out, target, w, inv_count, h2, z2, params[4], dout, loss_rows, dz2, part, grads[0] + used,
+        kSizes[0] - used, grads[2], kSizes[2]);
     if ((rc = cuda_status(cudaGetLastError(), "mlp_loss_backward launch"))) return rc;
     /* dz1 = (dz2 W2^T) gelu'(z1), its column sums the gradient of b1 */
     if ((rc = gemm_tc_launch(rows, kNetH1, kNetH2, dz2, kNetH2, 0, params[2], kNetH2, 1,
-                             tp::GtEpilogue{0.0f, dz1, kNetH1, nullptr, const_cast<float *>(z1), kNetH1, 1, grads[1]},
+                             tp::GtEpilogue{0.0f, dz1, kNetH1, nullptr, const_cast<float *>(z1), kNetH1, 1,
+                                            cols_fit ? cols1 : nullptr},
                              false, err, s)))
         return rc;
+    if (!cols_fit && (rc = tp_mlp_colsum(rows, kNetH1, kNetH1, dz1, 1.0f, grads[1], stream))) return rc;
+    tp::k_head_sums<<<(tp::kHeadPart + kNetH1 + tp::kSumCols - 1) / tp::kSumCols + 1, tp::kSumCols * tp::kSumLanes, 0,
+                      s>>>(part, blocks, cols1, cols_fit ? tiles : 0, rows, loss_rows, grads[3], grads[4], grads[5],
+                           grads[1], loss_sum);
+    if ((rc = cuda_status(cudaGetLastError(), "mlp_loss_backward launch"))) return rc;
     if ((rc = gemm_tc_launch(kNetH1, kNetH2, rows, h1, kNetH1, 1, dz2, kNetH2, 0,
                              tp::GtEpilogue{0.0f, grads[2], kNetH2, nullptr, nullptr, 0, 0, nullptr}, true, err, s)))
         return rc;

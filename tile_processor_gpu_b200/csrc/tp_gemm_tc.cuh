@@ -66,9 +66,9 @@ struct GtOperand {
     int ld, rows, across, vec;
 };
 
-/* What happens to the finished tile.  dgelu: C = acc * gelu'(z), and colsum[n]
- * += the column sums of C; else C = beta C + acc + bias, with z (if given) that
- * value and C = gelu of it. */
+/* What happens to the finished tile.  dgelu: C = acc * gelu'(z), and
+ * colsum[N m + n] (unless NULL) = the sum of column n of the m-th 128 rows of C;
+ * else C = beta C + acc + bias, with z (if given) that value and C = gelu of it. */
 struct GtEpilogue {
     float beta;
     float *C;
@@ -353,11 +353,24 @@ __global__ void __launch_bounds__(kGtThreads, 1) k_gemm_tc(int K, GtOperand A, G
         *c = v;
     }
     if (e.dgelu && e.colsum) {
+        /* eight partial sums a column, added in their order */
+        constexpr int kParts = kGtThreads / kGtN;
+        float(*part)[kGtN] = reinterpret_cast<float(*)[kGtN]>(sm + kGtM * (kGtN + 1) * 4);
+        static_assert((kGtM * (kGtN + 1) + kParts * kGtN) * 4 <= kGtStages * kGtStageBytes, "and their sums");
         __syncthreads();
-        const int n = tid % kGtN;
-        float sum = 0.0f;
-        for (int r = tid / kGtN; r < mrows; r += kGtThreads / kGtN) sum += tile[r][n];
-        if (tid < kGtThreads / kGtN * kGtN && n < ncols) atomicAdd(e.colsum + n0 + n, sum);
+        const int n = tid % kGtN, first = tid / kGtN;
+        if (first < kParts) {
+            float sum = 0.0f;
+            for (int r = first; r < mrows; r += kParts) sum += tile[r][n];
+            part[first][n] = sum;
+        }
+        __syncthreads();
+        if (tid < ncols) {
+            float sum = part[0][tid];
+#pragma unroll
+            for (int i = 1; i < kParts; i++) sum += part[i][tid];
+            e.colsum[(size_t)blockIdx.y * B.rows + n0 + tid] = sum;
+        }
     }
 }
 
@@ -392,65 +405,139 @@ __global__ void __launch_bounds__(256) k_head_forward(int rows, const float *__r
 }
 
 /* The loss and everything of the backward pass that is per row of the head, on
- * kHeadRows rows a block, thread c = column c of layer 2: the loss and its
- * gradient dout (k_nll), dz2 = (dout W3^T) gelu'(z2), and the gradients of W3,
- * b3 and b2 and the loss sum, added into zeroed memory once per block. */
-constexpr int kHeadRows = 16;
-__global__ void __launch_bounds__(128) k_head_backward(int rows, const float *__restrict__ out,
+ * `chunks` times kHeadRows rows a block, thread c = column c of layer 2: the loss
+ * and its gradient dout (k_nll), dz2 = (dout W3^T) gelu'(z2), and this block's
+ * part of the gradients of b2 (128), W3 (256) and b3 (2) at part[block], which
+ * k_head_sums adds in a fixed order.  The grid's blocks, those past the last row
+ * too, zero what the products of the weight gradients add into: zero0 .. zero0 +
+ * n0 and zero1 .. zero1 + n1. */
+constexpr int kHeadRows = 16, kHeadPart = 128 + 256 + 2;
+__global__ void __launch_bounds__(128) k_head_backward(int rows, int chunks, const float *__restrict__ out,
                                                        const float *__restrict__ target, const float *__restrict__ w,
                                                        float inv_count, const float *__restrict__ h2,
                                                        const float *__restrict__ z2, const float *__restrict__ W3,
                                                        float *__restrict__ dout, float *__restrict__ loss_rows,
-                                                       float *__restrict__ dz2, double *loss_sum, float *gW3,
-                                                       float *gb3, float *gb2)
+                                                       float *__restrict__ dz2, float *__restrict__ part, float *zero0,
+                                                       int n0, float *zero1, int n1)
 {
     __shared__ float s_d[kHeadRows][2];
-    const int c = threadIdx.x, r0 = blockIdx.x * kHeadRows, nr = min(kHeadRows, rows - r0);
-    if (c < 32) {
-        float loss = 0.0f, d0 = 0.0f, d1 = 0.0f;
-        if (c < nr) {
-            nll_row(r0 + c, out, target, w, inv_count, &loss, &d0, &d1);
-            loss_rows[r0 + c] = loss;
-            *reinterpret_cast<float2 *>(dout + 2 * (size_t)(r0 + c)) = make_float2(d0, d1);
-            s_d[c][0] = d0;
-            s_d[c][1] = d1;
-        }
-        double ls = (double)loss;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            ls += __shfl_xor_sync(0xffffffffu, ls, d);
-            d0 += __shfl_xor_sync(0xffffffffu, d0, d);
-            d1 += __shfl_xor_sync(0xffffffffu, d1, d);
-        }
-        if (c == 0) {
-            atomicAdd(loss_sum, ls);
-            atomicAdd(gb3, d0);
-            atomicAdd(gb3 + 1, d1);
-        }
-    }
-    __syncthreads();
+    const int c = threadIdx.x;
+    for (int i = blockIdx.x * 128 + c; i < n0; i += gridDim.x * 128) zero0[i] = 0.0f;
+    for (int i = blockIdx.x * 128 + c; i < n1; i += gridDim.x * 128) zero1[i] = 0.0f;
+    if (blockIdx.x * chunks * kHeadRows >= rows) return;
     const float w0 = __ldg(W3 + 2 * c), w1 = __ldg(W3 + 2 * c + 1);
-    float sb = 0.0f, s0 = 0.0f, s1 = 0.0f;
-    float z[kHeadRows], h[kHeadRows];
+    float sb = 0.0f, s0 = 0.0f, s1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
+    for (int k = 0; k < chunks; k++) {
+        const int r0 = (blockIdx.x * chunks + k) * kHeadRows, nr = min(kHeadRows, rows - r0);
+        if (nr <= 0) break;
+        float z[kHeadRows], h[kHeadRows];
 #pragma unroll
-    for (int i = 0; i < kHeadRows; i++) {
-        const size_t o = (size_t)(r0 + min(i, nr - 1)) * 128 + c;
-        z[i] = __ldg(z2 + o);
-        h[i] = __ldg(h2 + o);
-    }
+        for (int i = 0; i < kHeadRows; i++) {
+            const size_t o = (size_t)(r0 + min(i, nr - 1)) * 128 + c;
+            z[i] = __ldg(z2 + o);
+            h[i] = __ldg(h2 + o);
+        }
+        if (k) __syncthreads(); /* the chunk before has been read */
+        if (c < 32) {
+            float loss = 0.0f, d0 = 0.0f, d1 = 0.0f;
+            if (c < nr) {
+                nll_row(r0 + c, out, target, w, inv_count, &loss, &d0, &d1);
+                loss_rows[r0 + c] = loss;
+                *reinterpret_cast<float2 *>(dout + 2 * (size_t)(r0 + c)) = make_float2(d0, d1);
+                s_d[c][0] = d0;
+                s_d[c][1] = d1;
+            }
 #pragma unroll
-    for (int i = 0; i < kHeadRows; i++) {
-        if (i >= nr) break;
-        const float d0 = s_d[i][0], d1 = s_d[i][1];
-        const float g = __fmaf_rn(d1, w1, d0 * w0) * gelu_grad_f(z[i]);
-        dz2[(size_t)(r0 + i) * 128 + c] = g;
-        sb += g;
-        s0 = __fmaf_rn(h[i], d0, s0);
-        s1 = __fmaf_rn(h[i], d1, s1);
+            for (int d = 16; d > 0; d >>= 1) {
+                d0 += __shfl_xor_sync(0xffffffffu, d0, d);
+                d1 += __shfl_xor_sync(0xffffffffu, d1, d);
+            }
+            b0 += d0;
+            b1 += d1;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kHeadRows; i++) {
+            if (i >= nr) break;
+            const float d0 = s_d[i][0], d1 = s_d[i][1];
+            const float g = __fmaf_rn(d1, w1, d0 * w0) * gelu_grad_f(z[i]);
+            dz2[(size_t)(r0 + i) * 128 + c] = g;
+            sb += g;
+            s0 = __fmaf_rn(h[i], d0, s0);
+            s1 = __fmaf_rn(h[i], d1, s1);
+        }
     }
-    atomicAdd(gb2 + c, sb);
-    atomicAdd(gW3 + 2 * c, s0);
-    atomicAdd(gW3 + 2 * c + 1, s1);
+    float *p = part + (size_t)blockIdx.x * kHeadPart;
+    p[c] = sb;
+    p[128 + 2 * c] = s0;
+    p[128 + 2 * c + 1] = s1;
+    if (c == 0) {
+        p[384] = b0;
+        p[385] = b1;
+    }
+}
+
+/* The sums over blocks, each in a fixed order (kSumLanes threads a column, then
+ * a tree), so that a step's gradients repeat bit for bit: column n < kHeadPart of
+ * the nparts rows of k_head_backward to gb2, gW3, gb3; column n - kHeadPart of
+ * ncols1 rows of 256 (the GEMM's column sums) to gb1; the last block adds the
+ * rows' losses in double.  What it has read of `part` (the memory of a gradient
+ * that a product adds into next) it zeroes. */
+constexpr int kSumLanes = 16, kSumCols = 32;
+__global__ void __launch_bounds__(kSumCols *kSumLanes) k_head_sums(float *part, int nparts, float *cols1, int ncols1,
+                                                                   int rows, const float *__restrict__ loss_rows,
+                                                                   float *gb2, float *gW3, float *gb3, float *gb1,
+                                                                   double *loss_sum)
+{
+    const int lane = threadIdx.x / kSumCols;
+    if (blockIdx.x == gridDim.x - 1) {
+        __shared__ double s_loss[kSumCols * kSumLanes];
+        double s = 0.0;
+        for (int r = threadIdx.x; r < rows; r += kSumCols * kSumLanes) s += (double)__ldg(loss_rows + r);
+        s_loss[threadIdx.x] = s;
+        for (int h = kSumCols * kSumLanes / 2; h > 0; h >>= 1) {
+            __syncthreads();
+            if (threadIdx.x < h) s_loss[threadIdx.x] += s_loss[threadIdx.x + h];
+        }
+        if (threadIdx.x == 0) *loss_sum = s_loss[0];
+        return;
+    }
+    __shared__ float s_sum[kSumLanes][kSumCols];
+    const int col = threadIdx.x % kSumCols, n = blockIdx.x * kSumCols + col, n1 = n - kHeadPart;
+    float *src = n1 < 0 ? part + n : cols1 + n1;
+    const int ld = n1 < 0 ? kHeadPart : 256, count = n1 < 0 ? nparts : n1 < 256 ? ncols1 : 0;
+    float s = 0.0f;
+    constexpr int kBatch = 8; /* values in flight */
+    for (int i0 = lane; i0 < count; i0 += kBatch * kSumLanes) {
+        float v[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+            const int i = i0 + k * kSumLanes;
+            v[k] = i < count ? src[(size_t)i * ld] : 0.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; k++) {
+            const int i = i0 + k * kSumLanes;
+            s += v[k];
+            if (i < count) src[(size_t)i * ld] = 0.0f;
+        }
+    }
+    s_sum[lane][col] = s;
+    for (int h = kSumLanes / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (lane < h) s_sum[lane][col] += s_sum[lane + h][col];
+    }
+    if (lane == 0) {
+        const float v = s_sum[0][col];
+        if (n < 128)
+            gb2[n] = v;
+        else if (n < 384)
+            gW3[n - 128] = v;
+        else if (n < kHeadPart)
+            gb3[n - 384] = v;
+        else if (n1 < 256 && ncols1)
+            gb1[n1] = v;
+    }
 }
 
 /* up to kTensors arrays of a network in one launch */
@@ -460,14 +547,6 @@ struct TensorSet {
     long long n[kTensors];
     int count;
 };
-
-__global__ void __launch_bounds__(256) k_zero_set(TensorSet t, double *sum)
-{
-    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
-    if (first == 0) *sum = 0.0;
-    for (int i = 0; i < t.count; i++)
-        for (long long k = first; k < t.n[i]; k += step) t.p[i][k] = 0.0f;
-}
 
 /* k_adam on every array of a set: p, with its gradient, and its two moments */
 __global__ void __launch_bounds__(256) k_adam_set(TensorSet p, TensorSet g, TensorSet m, TensorSet v, float lr,
