@@ -137,6 +137,27 @@ def test_step_repeats(native, rows):
                 assert torch.equal(got[k], first[1][k]), (k, turn)
 
 
+def test_step_memory_by_form(native):
+    """The tensor-core step allocates no gradient of h1 and h2; the FP32 step
+    of the same network does when it comes to it, and gives the same gradients."""
+    import torch
+    from tile_processor_gpu_b200 import disparity_net as D
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn((300, D.N_IN), generator=gen, device="cuda")
+    t = torch.randn(300, generator=gen, device="cuda")
+    net = D.DisparityMLP(D.init_params(4))
+    net.forward(x, 300)
+    net.loss_backward(x, 300, t)
+    floats = sum(v.numel() for v in net._ws.values() if isinstance(v, torch.Tensor))
+    assert floats < 300 * (3 * D.N_H1 + 3 * D.N_H2 + 8) + 64
+    got = {k: net.g[k].clone() for k in D.PARAMS}
+    net.tc = False
+    net.forward(x, 300)
+    net.loss_backward(x, 300, t)
+    for k in D.PARAMS:
+        assert float((net.g[k] - got[k]).abs().max() / got[k].abs().max()) < 1e-4, k
+
+
 @pytest.mark.parametrize("rows", [115200, 131072])
 def test_column_sums_of_long_batches(native, rows):
     """Batches on both sides of the rule that lays the parts of b1's gradient

@@ -109,7 +109,7 @@ class DisparityMLP:
         if self._ws.get("rows", 0) < rows:
             f = lambda n: torch.empty((rows, n), dtype=torch.float32, device=self.device)
             self._ws = {"rows": rows, "z1": f(N_H1), "h1": f(N_H1), "z2": f(N_H2), "h2": f(N_H2), "out": f(N_OUT),
-                        "dout": f(N_OUT), "dh2": f(N_H2), "dz2": f(N_H2), "dh1": f(N_H1), "dz1": f(N_H1),
+                        "dout": f(N_OUT), "dz2": f(N_H2), "dz1": f(N_H1),
                         "loss": torch.empty(rows, dtype=torch.float32, device=self.device),
                         "loss_sum": torch.empty(1, dtype=torch.float64, device=self.device)}
         return self._ws
@@ -145,6 +145,10 @@ class DisparityMLP:
                          _dptr(w["loss_sum"]), _dptr(w["dz2"]), _dptr(w["dz1"]),
                          _pointers([g[k] for k in PARAMS]), _dptr(self._err), _stream(stream))
             return float(w["loss_sum"].item()) / max(count, 1.0)
+        # the gradients of h2 and h1, which the tensor-core step does not form
+        for k, z in (("dh2", "z2"), ("dh1", "z1")):
+            if k not in w:
+                w[k] = _t().empty_like(w[z])
         _native.call("tp_mlp_nll", int(rows), _dptr(w["out"]), _dptr(target),
                      _dptr(weight) if weight is not None else None, 1.0 / max(count, 1.0), _dptr(w["dout"]),
                      _dptr(w["loss"]), _stream(stream))
