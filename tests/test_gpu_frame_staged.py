@@ -1,6 +1,8 @@
 """The whole frame in stages through a workspace against the form with the CLT
 on chip (same device code): the same correlation bits, the image up to the
 order of at most four additions per pixel and pass group."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -99,3 +101,54 @@ def test_frame_with_a_short_workspace(native):
     _compare(got, _run(fr, c.tasks, on_chip=True))
     assert bool((got[3] == 77).all())
     _compare(_run(fr, c.tasks, short_by=0), got)
+
+
+def test_frames_without_memory_for_the_workspace(native):
+    """Frames that find no memory for their workspace run on chip, and only the
+    first of them empties torch's cache; once there is memory they run in stages."""
+    import torch
+    from cases import Case
+    from tile_processor_gpu_b200 import _native, api
+    gc.collect()
+    torch.cuda.empty_cache()  # before the frame's buffers are cut from a block of an earlier test
+    c = Case(800, 720, seed=44, border_mode=0)
+    n, stride = c.num_tiles, (c.TX + 1) * 8
+    need = _native.call("tp_process_frame_workspace", n)
+    fr = _frame(c)
+    want = _run(fr, c.tasks, on_chip=True)[0][:, :, :225]
+    t = api.tasks_to_device(c.tasks)
+    corrs = torch.zeros((n, 6, 225), device="cuda")
+    ints = [torch.zeros(k, dtype=torch.int32, device="cuda") for k in (c.TX * c.TYA + 256, 8, 4)]
+    rgba = torch.zeros(((c.TY + 1) * 8 * 4, stride), device="cuda")
+
+    def frame():
+        corrs.zero_()
+        api.process_frame(fr.g, fr.p_extra, fr.p_kernels, fr.p_images, c.dstride, t, n, corrs, 225, fr.port_offsets,
+                          *ints, stride, rgba, fat_zero=0.05)
+
+    def count(what):
+        return torch.cuda.memory_stats()[what]
+
+    torch.cuda.empty_cache()
+    spare = torch.empty(need // 2, dtype=torch.uint8, device="cuda")
+    limit = (torch.cuda.memory_reserved() + (2 << 20)) / torch.cuda.mem_get_info()[1]
+    del spare  # in torch's cache, too small for the workspace
+    largest = max((b["size"] for seg in torch.cuda.memory_snapshot() for b in seg["blocks"] if b["state"] == "inactive"),
+                  default=0)
+    assert largest < need
+    try:
+        torch.cuda.set_per_process_memory_fraction(limit)
+        before = count("num_alloc_retries")
+        for _ in range(4):
+            frame()
+        torch.cuda.synchronize()
+        assert count("num_alloc_retries") == before + 1
+        assert np.array_equal(corrs.cpu().numpy(), want)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    torch.cuda.reset_peak_memory_stats()
+    base = torch.cuda.memory_allocated()
+    frame()
+    assert torch.cuda.max_memory_allocated() - base >= need
+    torch.cuda.synchronize()
+    assert np.array_equal(corrs.cpu().numpy(), want)

@@ -23,6 +23,8 @@ from .synth import TASK_DTYPE
 class Geometry:
     """Runtime geometry (replaces IMG_WIDTH / IMG_HEIGHT / KERNELS_* defines)."""
 
+    workspace_short = 0  # bytes of process_frame's workspace that there was last no memory for
+
     def __init__(self, img_width, img_height, kernels_hor=None, kernels_vert=None, kernels_lstep=4,
                  image_rows=None, border_mode=0, debug_marks=0):
         step = 1 << kernels_lstep
@@ -263,10 +265,24 @@ def generate_RBGA_noalloc(geom, gpu_tasks, num_tiles, width, height, gpu_clt, gp
                  _dptr(gpu_texture_tiles), _stream(stream))
 
 
-def _frame_workspace(gpu_tasks, num_tiles, handle):
+def _room_for(size, device):
+    """Whether an allocation of size bytes may succeed: from blocks torch's allocator holds, or from what the
+    device and this process's share of it have left."""
+    stats = torch.cuda.memory.memory_stats_as_nested_dict(device)
+    reserved = stats["reserved_bytes"]["all"]["current"]
+    if reserved - stats["active_bytes"]["all"]["current"] >= size:
+        return True
+    free, total = torch.cuda.mem_get_info(device)
+    return min(free, torch.cuda.get_per_process_memory_fraction(device) * total - reserved) >= size
+
+
+def _frame_workspace(geom, gpu_tasks, num_tiles, handle):
     """Workspace of process_frame's staged form, or None: on a stream other than torch's current one (the
     caching allocator hands the memory on in that stream's order), during a
-    capture (a graph may outlive it) and when the device has no memory left."""
+    capture (a graph may outlive it) and when the device has no memory left.
+    A failed allocation makes torch give back every block it holds (and waits
+    for the device), so after one the geometry's frames ask for room first,
+    until there is some (0.08 ms a call, which those with room do not spend)."""
     if not isinstance(gpu_tasks, torch.Tensor) or not gpu_tasks.is_cuda:
         return None
     size = _native.call("tp_process_frame_workspace", num_tiles)
@@ -274,10 +290,17 @@ def _frame_workspace(gpu_tasks, num_tiles, handle):
         return None
     if handle != torch.cuda.current_stream().cuda_stream or torch.cuda.is_current_stream_capturing():
         return None
-    try:
-        return torch.empty(size, dtype=torch.uint8, device=gpu_tasks.device)
-    except torch.OutOfMemoryError:
+    short = 0 < getattr(geom, "workspace_short", 0) <= size
+    if short and not _room_for(size, gpu_tasks.device):
         return None
+    try:
+        ws = torch.empty(size, dtype=torch.uint8, device=gpu_tasks.device)
+    except torch.OutOfMemoryError:
+        geom.workspace_short = size
+        return None
+    if short:
+        geom.workspace_short = 0
+    return ws
 
 
 def process_frame(geom, gpu_kernel_offsets, gpu_kernels, gpu_images, dstride, gpu_tasks, num_tiles, gpu_corrs,
@@ -290,7 +313,7 @@ def process_frame(geom, gpu_kernel_offsets, gpu_kernels, gpu_images, dstride, gp
     [num_tiles][6][corr_stride]."""
     clt = _parr(gpu_clt) if gpu_clt is not None else None
     handle = _stream(stream)
-    ws = _frame_workspace(gpu_tasks, int(num_tiles), handle) if clt is None else None
+    ws = _frame_workspace(geom, gpu_tasks, int(num_tiles), handle) if clt is None else None
     _native.call("tp_process_frame_ws", geom.ptr, _parr(gpu_kernel_offsets), _parr(gpu_kernels), _parr(gpu_images),
                  int(dstride), _dptr(gpu_tasks), int(num_tiles), int(lpf_mask), int(corr_colors), float(scale0),
                  float(scale1), float(scale2), float(fat_zero), int(corr_radius), int(corr_stride), _dptr(gpu_corrs),
