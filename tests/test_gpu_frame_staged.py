@@ -152,3 +152,51 @@ def test_frames_without_memory_for_the_workspace(native):
     assert torch.cuda.max_memory_allocated() - base >= need
     torch.cuda.synchronize()
     assert np.array_equal(corrs.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("shape", [(256, 192), (800, 720)])
+def test_captured_frame_after_an_eager_one(native, shape):
+    """An eager first call (in stages) prepares the kernels of a captured one (on
+    chip, without a workspace): the graph's replays, on new images and tasks in
+    the same buffers, give the eager call's frames."""
+    import torch
+    from cases import Case
+    from tile_processor_gpu_b200 import api
+    cases = [Case(*shape, seed=k, border_mode=1) for k in (45, 46)]
+    frs = [_frame(c) for c in cases]
+    c, fr, n, stride = cases[0], _frame(cases[0]), cases[0].num_tiles, (cases[0].TX + 1) * 8
+    t = api.tasks_to_device(c.tasks)
+    corrs = torch.zeros((n, 6, 228), device="cuda")
+    ints = [torch.zeros(k, dtype=torch.int32, device="cuda") for k in (c.TX * c.TYA + 256, 8, 4)]
+    rgba = torch.zeros(((c.TY + 1) * 8 * 4, stride), device="cuda")
+
+    def frame():
+        api.process_frame(fr.g, fr.p_extra, fr.p_kernels, fr.p_images, c.dstride, t, n, corrs, 228, fr.port_offsets,
+                          *ints, stride, rgba, fat_zero=0.05)
+
+    want = []
+    for k in (1, 0):
+        _load(fr, t, frs[k], cases[k])
+        frame()
+        torch.cuda.synchronize()
+        want.insert(0, (corrs.cpu().numpy(), ints[2].cpu().numpy(), rgba.cpu().numpy(), None, t.cpu().numpy()))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        frame()
+    for k in (0, 1, 0):
+        _load(fr, t, frs[k], cases[k])
+        corrs.zero_()
+        rgba.fill_(3.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        _compare((corrs.cpu().numpy(), ints[2].cpu().numpy(), rgba.cpu().numpy(), None, t.cpu().numpy()), want[k])
+
+
+def _load(fr, t, src, case):
+    """another frame's inputs into fr's buffers (kernel tables, offsets, images) and the task tensor"""
+    from tile_processor_gpu_b200 import api
+    for name in ("images", "kernels", "extra"):
+        for a, b in zip(getattr(fr, name), getattr(src, name)):
+            if a is not b:
+                a.copy_(b)
+    t.copy_(api.tasks_to_device(case.tasks))

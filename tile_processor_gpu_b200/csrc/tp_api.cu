@@ -732,6 +732,12 @@ static int process_frame(const tp_geometry *g, float *const *kernel_offsets, flo
         return fail(TP_ERR_ARG, "texture_rbga_stride %zu < (tilesx + 1) * 8", texture_rbga_stride);
     if (!corrs || !port_offsets || !texture_rbga) return fail(TP_ERR_ARG, "NULL corrs / port_offsets / texture_rbga");
     if (num_tiles == 0) return TP_OK;
+    /* the kernels of both forms: a first call in stages is followed by one on
+     * chip when the frame is captured (without a workspace) */
+    if ((rc = texture_smem_setup())) return rc;
+    if ((rc = set_smem_once(g_frame_attr, (const void *)tp::k_frame, tp::kFrameSmemBytes,
+                            "cudaFuncSetAttribute(k_frame)")))
+        return rc;
     if ((rc = tp_prepare_texture_list(g, tasks, num_tiles, texture_indices, num_texture_tiles, woi, gd.TX, gd.TY,
                                       stream)))
         return rc;
@@ -760,7 +766,6 @@ static int process_frame(const tp_geometry *g, float *const *kernel_offsets, flo
         if (err != cudaSuccess) return cuda_status(err, "process_frame clear launch");
     }
     if (staged) {
-        if ((rc = texture_smem_setup())) return rc;
         cudaError_t err = cudaSuccess;
         /* A chain of programmatic dependents.  The forward transform and the
          * correlations wait on entry for the launch before them and release their
@@ -804,9 +809,6 @@ static int process_frame(const tp_geometry *g, float *const *kernel_offsets, flo
     fp.corr_radius = corr_radius;
     fp.corr_stride = corr_stride;
     fp.tex = tex;
-    if ((rc = set_smem_once(g_frame_attr, (const void *)tp::k_frame, tp::kFrameSmemBytes,
-                            "cudaFuncSetAttribute(k_frame)")))
-        return rc;
     /* one resident wave, odd: a grid-stride walk over a raster task list then
      * visits both column parities in every block.  Each parity launch is a
      * programmatic dependent of the launch before it (the clear, or the
