@@ -121,6 +121,7 @@ struct CorrTcStage {
         }
         /* lane -> (entry parity, column) of the stores */
         const int col = lane & 15, odd = lane >> 4;
+        const int entries = 32 - __clz(valid); /* none after the last valid one */
 #pragma unroll 1
         for (int i = 0; i <= r; i++) {
             float v[4][8];
@@ -147,7 +148,7 @@ struct CorrTcStage {
             __syncwarp();
             if (col < sz) {
 #pragma unroll 4
-                for (int e = odd; e < 32; e += 2) {
+                for (int e = odd; e < entries; e += 2) {
                     if (!((valid >> e) & 1)) continue;
                     float *d = dst + (size_t)e * stride + col;
                     if (i) d[(r + i) * sz] = buf[e * kRowPair + col];
