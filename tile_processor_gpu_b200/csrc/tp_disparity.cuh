@@ -134,12 +134,8 @@ __global__ void __launch_bounds__(256, 6) k_disparity_fit(int ntiles, const floa
         FitSample at = fit_sample_at(r, (float)k * bx, (float)k * by);
         if (k > r) at = FitSample{-1, 0.0f, 0.0f};
         s_at[p][threadIdx.x & 15] = at;
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        int whole = 1;
-        for (int k = 0; k < 16; k++) whole &= s_at[threadIdx.x][k].fx == 0.0f && s_at[threadIdx.x][k].fy == 0.0f;
-        s_whole[threadIdx.x] = whole;
+        const unsigned whole = __ballot_sync(0xffffffffu, at.fx == 0.0f && at.fy == 0.0f);
+        if ((threadIdx.x & 15) == 0) s_whole[p] = ((whole >> (threadIdx.x & 16)) & 0xffffu) == 0xffffu;
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4;
