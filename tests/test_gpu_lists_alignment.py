@@ -47,6 +47,32 @@ def test_texture_entries_are_independent(frame, colors, count):
 
 
 @pytest.mark.parametrize("colors", [1, 3])
+def test_textures_do_not_depend_on_the_grid(native, colors):
+    """One block per SM or the built-in number: tiles and RGBA image have the
+    same bits, whether a block holds one entry or all its mono slots are full
+    (lists of 3200 and of a few more entries than blocks)."""
+    import gpu_runner as R
+    from cases import Case
+    from tile_processor_gpu_b200 import autotune
+    c = Case(512, 400, seed=36, border_mode=1)
+    fr = R.Frame(c)
+    R.convert(fr)
+    lists = [c.tex_idx, c.tex_idx[:1037], c.tex_idx[:151]]
+    got = []
+    for cap in (0, 1):
+        autotune.set_shape("textures", cap)
+        try:
+            got.append([R.textures_tiles(fr, idx, keep_weights=1, colors=colors) for idx in lists] +
+                       [R.rgba(fr, colors=colors)[0]])
+        finally:
+            autotune.reset()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    one = [R.textures_tiles(fr, c.tex_idx[k:k + 1], keep_weights=1, colors=colors)[0] for k in (0, 1036, 3199)]
+    assert all(np.array_equal(got[0][0][k], x) for k, x in zip((0, 1036, 3199), one))
+
+
+@pytest.mark.parametrize("colors", [1, 3])
 @pytest.mark.parametrize("floats", [1, 4])
 def test_textures_of_unaligned_clt(frame, colors, floats):
     import gpu_runner as R

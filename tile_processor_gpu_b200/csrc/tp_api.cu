@@ -417,7 +417,7 @@ static int launch_textures(Kernel kernel, const tp::Geom &gd, const int *woi, fl
     constexpr size_t kChunk = (size_t)1 << 30;
     for (size_t n0 = 0; n0 < count; n0 += kChunk) {
         const int n = (int)(count - n0 < kChunk ? count - n0 : kChunk);
-        const unsigned grid = grid_for(n, tp::tex_tiles(p.colors), sms, shape_per_sm(TP_SHAPE_TEXTURES));
+        const unsigned grid = grid_for(n, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES));
         kernel<<<grid, tp::kTexThreads, tp::kTexSmemBytes, (cudaStream_t)stream>>>(
             gd, woi, clt, n, indices + n0, nullptr, 0, 0, 0, port_offsets, p, rbg_stride, rbg, tile_stride,
             tiles ? tiles + n0 * tile_stride : nullptr, tp::FrameSlots{});
@@ -659,7 +659,7 @@ static int generate_rbga(const tp_geometry *g, tp_task *tasks, int num_tiles, in
         src = tile_scratch;
     }
     const int quarter = gd.TX * (gd.TYA >> 2);
-    const unsigned grid = grid_for(quarter, tp::tex_tiles(colors), sms, shape_per_sm(TP_SHAPE_TEXTURES));
+    const unsigned grid = grid_for(quarter, 1, sms, shape_per_sm(TP_SHAPE_TEXTURES));
     /* one pass per tile parity: its inner sub-list, then its border one (the
      * reference runs the four inner passes, then the four border passes;
      * tiles of one parity never overlap, so a pass needs no ordering) */

@@ -4,7 +4,8 @@
  * :3847-4017, debayer_shot / debayer :4019-4199 and tile_combine_rgba
  * :4202-4665).
  *
- * One 128-thread block per listed tile (mono: per four tiles), grid-stride.
+ * One 128-thread block per listed tile (mono: up to four tiles at a time),
+ * grid-stride.
  * The CLT is read straight from global memory by the inverse transform; the
  * next tile's CLT and the RGBA rows it will update are prefetched into L2 while
  * the block works on the current tile.  Per (camera, colour) job one 8-lane
@@ -753,16 +754,19 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * inverse transform (FROM_T), which writes the pixel tiles, is not: the
      * first pass after it is an ordinary launch. */
     bool waited = false;
+    /* A block's entries lie a grid apart, so that a mono list too short for four
+     * of them a block spreads over as many blocks as it has entries (300 mono
+     * tiles: 8.3 us, 10.3 with four neighbours a block). */
     int codes[kTiles], ats[kTiles] = {}, gy0 = 0, gx0 = 0;
 #pragma unroll
-    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x * kTiles + i, ats[i]);
+    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x + i * (int)gridDim.x, ats[i]);
     int mine = pick(codes), mine_at = pick(ats);
     if (colors == 3 && want_rbg) rgba_origin(codes[0] >> 8, &gy0, &gx0);
 
-    for (int n = (int)blockIdx.x * kTiles; n < count; n += (int)gridDim.x * kTiles) {
+    for (int n = (int)blockIdx.x; n < count; n += (int)gridDim.x * kTiles) {
         int next[kTiles], next_at[kTiles] = {};
 #pragma unroll
-        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * kTiles + i, next_at[i]);
+        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * (kTiles + i), next_at[i]);
 
         /* ---- stages 1-2: per (tile, camera, color) group ---- */
         if (mine) {
@@ -847,7 +851,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
                 combine_pair<1>(t2, kTexJob / 2, t2, kTexJob / 2, dup2(1.0f), e, s_npd2r, nksigma, s_chw, s_chws,
                                 wnd2, wi, p.dust_remove, keep_weights, o);
             if (want_tiles) {
-                float *dst = texture_tiles + (size_t)(n + k) * texture_stride + px;
+                float *dst = texture_tiles + (size_t)(n + k * (int)gridDim.x) * texture_stride + px;
 #pragma unroll
                 for (int sl = 0; sl < 12; sl++)
                     if (sl < ns_tiles) {
