@@ -928,10 +928,10 @@ int tp_mlp_features(const tp_geometry *g, const float *corrs, size_t corr_stride
     if (feature_stride < (size_t)(6 * n2)) return fail(TP_ERR_ARG, "feature_stride %zu < %d", feature_stride, 6 * n2);
     int sms;
     if ((rc = sm_count(&sms))) return rc;
-    const int win = list_window((long long)num_corr_tiles, sms, 2 * 8);
-    tp::k_mlp_features<<<grid_for((long long)num_corr_tiles, 8 * win, sms, 8), 256, 0, (cudaStream_t)stream>>>(
-        gd.TX * gd.TY, corrs, corr_stride, n2, (long long)num_corr_tiles, corr_indices, win, features,
-        feature_stride);
+    const int win = list_window((long long)num_corr_tiles, sms, 9 * tp::kFeatWarps);
+    tp::k_mlp_features<<<grid_for((long long)num_corr_tiles, tp::kFeatWarps * win, sms, 32), tp::kFeatThreads, 0,
+                         (cudaStream_t)stream>>>(gd.TX * gd.TY, corrs, corr_stride, n2, (long long)num_corr_tiles,
+                                                 corr_indices, win, features, feature_stride);
     return cuda_status(cudaGetLastError(), "mlp_features launch");
 }
 
