@@ -52,7 +52,7 @@ struct FrameParams {
     TextureParams tex; /* colors == 3, keep_weights == 0 */
 };
 
-constexpr int kFrameThreads = 96;
+constexpr int kFrameThreads = 96; /* a group per (colour, camera) job */
 constexpr int kFrameBlocksPerSm = 5;
 /* dynamic shared memory of k_frame, in floats: per job its CLT, then T in
  * place (kJob floats); per group the transpose buffer, the correlation
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
      * transform, the offsets (and the kernel tile itself into L2) after the
      * correlations, the window's Bayer rows into L2 before the fusion. */
     __shared__ __align__(16) float s_pf[12][8];
-    const int color_c = min(grp >> 2, 2), cam_c = grp & 3;
+    const int color_c = grp >> 2, cam_c = grp & 3;
     int pf_n = -1; /* the tile whose inputs s_pf holds */
     const float step_inv = __int_as_float((127 - g.ls) << 23);
     auto kernel_tile = [&](float cx, float cy) -> size_t {
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
     };
     auto fetch_offsets = [&]() {
         pf_sync();
-        if (pf_n < 0 || grp >= 12) return;
+        if (pf_n < 0) return;
         const size_t kidx = kernel_tile(s_pf[grp][6], s_pf[grp][7]);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(kernels[cam_c] + kidx * 256 + l * 32));
         if (l < 6) cp_async4(&s_pf[grp][l], kernel_offsets[cam_c] + kidx * 8 + (l < 2 ? l : l + 2));
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
      * inside the image) */
     auto prefetch_window = [&]() {
         pf_sync();
-        if (pf_n < 0 || grp >= 12) return;
+        if (pf_n < 0) return;
         const float px = s_pf[grp][6] - 8.0f - s_pf[grp][0], py = s_pf[grp][7] - 8.0f - s_pf[grp][1];
         const int x0 = min(max(__float2int_rd(px + 0.5f), 0), g.W - 16);
         const int y0 = min(max(__float2int_rd(py + 0.5f), 0), g.H - 16);
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
         const int tx = txy & 0xffff, ty = txy >> 16;
 
         /* ---- 1. forward CLT: warp = colour, group = camera ---- */
-        if (grp < 12) {
+        {
             float cx, cy, ex[6];
             if (pf_n == n) {
                 cx = s_pf[grp][6]; cy = s_pf[grp][7];
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
             pf_n = m ? n + __ffs(m) * (int)gridDim.x : -1;
             /* every lane of the group has read s_pf (before the transposes'
              * first __syncwarp in convert_job) */
-            if (grp < 12 && pf_n >= 0 && l >= 6) cp_async4(&s_pf[grp][l], &tasks[pf_n].xy[cam_c][l - 6]);
+            if (pf_n >= 0 && l >= 6) cp_async4(&s_pf[grp][l], &tasks[pf_n].xy[cam_c][l - 6]);
             cp_async_commit();
         }
         __syncthreads();
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kFrameThreads, kFrameBlocksPerSm) k_frame(
         if (nbr) {
             __syncthreads(); /* the correlations have read the CLT and freed s_x */
             /* ---- 3. inverse CLT to T (in place), debayer to D: group = job ---- */
-            if (grp < 12) {
+            {
                 const int color = grp % 3;
                 float *cj = s_clt + grp * kJob, *xj = s_x + grp * kXb;
                 float2 t[2][8];
