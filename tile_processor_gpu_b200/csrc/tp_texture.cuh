@@ -754,19 +754,24 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
      * inverse transform (FROM_T), which writes the pixel tiles, is not: the
      * first pass after it is an ordinary launch. */
     bool waited = false;
-    /* A block's entries lie a grid apart, so that a mono list too short for four
-     * of them a block spreads over as many blocks as it has entries (300 mono
-     * tiles: 8.3 us, 10.3 with four neighbours a block). */
+    /* A list that fits the blocks in one turn is spread over them, a block's
+     * entries a grid apart, so that a short mono list takes as many blocks as it
+     * has entries (300 mono tiles: 8.3 us, 10.3 with four neighbours a block); the
+     * entries of a longer one are neighbours, so that its last turn takes few
+     * blocks (5120: 22.6 us, 24.6 spread). */
+    const int grid = (int)gridDim.x;
+    const bool spread = kTiles == 1 || count <= grid * kTiles;
+    const int slot_step = spread ? grid : 1, first = (int)blockIdx.x * (spread ? 1 : kTiles);
     int codes[kTiles], ats[kTiles] = {}, gy0 = 0, gx0 = 0;
 #pragma unroll
-    for (int i = 0; i < kTiles; i++) codes[i] = entry((int)blockIdx.x + i * (int)gridDim.x, ats[i]);
+    for (int i = 0; i < kTiles; i++) codes[i] = entry(first + i * slot_step, ats[i]);
     int mine = pick(codes), mine_at = pick(ats);
     if (colors == 3 && want_rbg) rgba_origin(codes[0] >> 8, &gy0, &gx0);
 
-    for (int n = (int)blockIdx.x; n < count; n += (int)gridDim.x * kTiles) {
+    for (int n = first; n < count; n += grid * kTiles) {
         int next[kTiles], next_at[kTiles] = {};
 #pragma unroll
-        for (int i = 0; i < kTiles; i++) next[i] = entry(n + (int)gridDim.x * (kTiles + i), next_at[i]);
+        for (int i = 0; i < kTiles; i++) next[i] = entry(n + grid * kTiles + i * slot_step, next_at[i]);
 
         /* ---- stages 1-2: per (tile, camera, color) group ---- */
         if (mine) {
@@ -851,7 +856,7 @@ __global__ void __launch_bounds__(kTexThreads, 7) k_textures(
                 combine_pair<1>(t2, kTexJob / 2, t2, kTexJob / 2, dup2(1.0f), e, s_npd2r, nksigma, s_chw, s_chws,
                                 wnd2, wi, p.dust_remove, keep_weights, o);
             if (want_tiles) {
-                float *dst = texture_tiles + (size_t)(n + k * (int)gridDim.x) * texture_stride + px;
+                float *dst = texture_tiles + (size_t)(n + k * slot_step) * texture_stride + px;
 #pragma unroll
                 for (int sl = 0; sl < 12; sl++)
                     if (sl < ns_tiles) {
