@@ -727,7 +727,7 @@ def run_b200(args, rank, world, local, pg):
     torch.cuda.synchronize()
     fused_ms = f0.elapsed_time(f1) / fused_steps
 
-    # the same step captured once in a CUDA graph and replayed (17 launches)
+    # the same step captured once in a CUDA graph and replayed (12 launches)
     graph_ms = None
     try:
         side = torch.cuda.Stream()

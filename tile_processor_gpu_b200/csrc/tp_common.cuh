@@ -223,8 +223,8 @@ __device__ __forceinline__ void load_row8s(const float *p, float v[8])
 /* 8 consecutive floats of global memory (32-byte aligned): one 256-bit access.  ld8_global is for rows that
    the SM reads once (CLT tiles of the textures and the inverse transform, deconvolution kernel rows): it leaves
    L1 to what is read again.  With plain loads the tensor-core inverse's tables were evicted by the tiles that
-   pass: the fp16 image of 2592x1936 took 436 us, 418 this way; the texture list 611 and 608.  ld8_l1 is for
-   the correlation, whose pairs share a tile's rows. */
+   pass: the three tensor-core stages of 1024x768 took 436 us in FP16, 418 this way; the RGBA image of 2592x1936
+   611 and 608.  ld8_l1 is for the correlation, whose pairs share a tile's rows. */
 __device__ __forceinline__ void ld8_global(const float *p, float v[8])
 {
     asm volatile("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

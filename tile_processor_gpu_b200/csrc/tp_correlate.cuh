@@ -17,7 +17,7 @@
  * (the sums of a row and one colour of both tiles are 96 registers) and the L1
  * (91% busy before, 57% now): 256-bit loads halve the passes over the loaded
  * lines, which 16-byte loads at a 32-byte lane stride touch twice.  A
- * 2592x1936 frame's 470,448 pairs went from 0.385 to 0.321 ms (3.61 to 4.33
+ * 2592x1936 frame's 470,448 pairs went from 0.385 to 0.314 ms (3.61 to 4.42
  * TB/s of 1.39 GB).  Tried and slower: staging four tiles for one bulk store
  * (0.328), L2 prefetch of the next entry (+5%), 20 and 24 warps (spills).
  */

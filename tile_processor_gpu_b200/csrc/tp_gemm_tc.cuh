@@ -26,7 +26,8 @@
  *     into 32 registers, one tensor-memory load and wait a chunk, and release
  *     the accumulator (accfree[s]).
  * At the end the tile goes through shared memory and all warps apply bias,
- * beta C, GELU, or (dgelu) the factor gelu'(z), row by row.
+ * beta C, GELU, or (dgelu) the factor gelu'(z), row by row; the tile's column
+ * sums, where they are wanted, go out as one part a tile (k_head_sums adds them).
  * What bounds it is shared memory: a chunk's split images are 48 KB written and
  * 72 KB read by the MMAs (N = 64 reads A once per MMA), beside about 10 us of
  * launch, first loads and epilogue.  The earlier form did every step of a chunk

@@ -41,8 +41,8 @@ namespace tp {
  * entries without a repeated pair the same plane by plane; other runs take
  * the two-pass loop.  A 2592x1936 frame: 0.138 ms, 0.172 with a warp per entry
  * (0.85 GB, 6.2 TB/s).  Blocks of two warps: the last windows spread over more
- * SMs and 18 warps fit one, 16 in blocks of eight (30,000 entries of one pair a
- * tile 41.8 us, 43.0). */
+ * SMs and up to 20 warps fit one, 16 in blocks of eight (30,000 entries of one
+ * pair a tile 41.8 us, 43.0). */
 constexpr int kFeatThreads = 64, kFeatWarps = kFeatThreads / 32;
 __global__ void __launch_bounds__(kFeatThreads) k_mlp_features(int ntiles, const float *__restrict__ corrs,
                                                       size_t corr_stride, int n2, long long num,
