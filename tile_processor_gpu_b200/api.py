@@ -66,12 +66,21 @@ class PointerArray:
     def ptr(self):
         return ctypes.c_void_p(self.dev.data_ptr())
 
+    _as_parameter_ = ptr  # as an argument of a call
 
-def _parr(x):
+
+def _parr(x, stream):
+    """A pointer array for an argument: the address of a PointerArray's, or an
+    array made for this call from a list of tensors.  The latter is the argument
+    itself, so that it lives until the call has launched, and on a stream other
+    than the current one until that stream has passed the launch."""
     if isinstance(x, PointerArray):
         return x.dev.data_ptr()
     if isinstance(x, (list, tuple)):
-        return PointerArray(x).ptr
+        p = PointerArray(x)
+        if p.dev.is_cuda and stream is not None:
+            p.dev.record_stream(torch.cuda.ExternalStream(stream, p.dev.device) if isinstance(stream, int) else stream)
+        return p
     raise TypeError("expected a list of tensors or a PointerArray")
 
 
@@ -102,8 +111,8 @@ def tasks_from_device(t):
 def convert_correct_tiles(geom, gpu_kernel_offsets, gpu_kernels, gpu_images, gpu_tasks, gpu_clt, dstride,
                           num_tiles, lpf_mask=0, stream=None):
     """Forward CLT with aberration correction (convert_correct_tiles)."""
-    _native.call("tp_convert_correct_tiles", geom.ptr, _parr(gpu_kernel_offsets), _parr(gpu_kernels),
-                 _parr(gpu_images), _dptr(gpu_tasks), _parr(gpu_clt), int(dstride), int(num_tiles),
+    _native.call("tp_convert_correct_tiles", geom.ptr, _parr(gpu_kernel_offsets, stream), _parr(gpu_kernels, stream),
+                 _parr(gpu_images, stream), _dptr(gpu_tasks), _parr(gpu_clt, stream), int(dstride), int(num_tiles),
                  int(lpf_mask), _stream(stream))
 
 
@@ -111,15 +120,16 @@ def convert_correct_tiles_tma(geom, gpu_kernel_offsets, gpu_kernels, gpu_images,
                               num_tiles, lpf_mask=0, stream=None):
     """convert_correct_tiles with the Bayer windows staged in shared memory by
     the TMA unit (tp_convert_correct_tiles_tma; the same CLT)."""
-    _native.call("tp_convert_correct_tiles_tma", geom.ptr, _parr(gpu_kernel_offsets), _parr(gpu_kernels),
-                 _parr(gpu_images), _dptr(gpu_tasks), _parr(gpu_clt), int(dstride), int(num_tiles),
+    _native.call("tp_convert_correct_tiles_tma", geom.ptr, _parr(gpu_kernel_offsets, stream),
+                 _parr(gpu_kernels, stream), _parr(gpu_images, stream), _dptr(gpu_tasks), _parr(gpu_clt, stream),
+                 int(dstride), int(num_tiles),
                  int(lpf_mask), _stream(stream))
 
 
 def correlate2D(geom, gpu_clt, colors, scale0, scale1, scale2, fat_zero, num_corr_tiles, gpu_corr_indices,
                 corr_stride, corr_radius, gpu_corrs, stream=None):
     """Pairwise 2-D phase correlation (correlate2D)."""
-    _native.call("tp_correlate2D", geom.ptr, _parr(gpu_clt), int(colors), float(scale0), float(scale1),
+    _native.call("tp_correlate2D", geom.ptr, _parr(gpu_clt, stream), int(colors), float(scale0), float(scale1),
                  float(scale2), float(fat_zero), int(num_corr_tiles), _dptr(gpu_corr_indices), int(corr_stride),
                  int(corr_radius), _dptr(gpu_corrs), _stream(stream))
 
@@ -131,7 +141,7 @@ def correlate2D_tc(geom, gpu_clt, colors, scale0, scale1, scale2, fat_zero, num_
                    corr_stride, corr_radius, gpu_corrs, fmt=TC_FP16X2, stream=None):
     """correlate2D with the pixel-domain transforms on the tensor cores
     (split 16-bit operands: fmt TC_FP16X2 or TC_BF16X2)."""
-    _native.call("tp_correlate2D_tc", geom.ptr, _parr(gpu_clt), int(colors), float(scale0), float(scale1),
+    _native.call("tp_correlate2D_tc", geom.ptr, _parr(gpu_clt, stream), int(colors), float(scale0), float(scale1),
                  float(scale2), float(fat_zero), int(num_corr_tiles), _dptr(gpu_corr_indices), int(corr_stride),
                  int(corr_radius), _dptr(gpu_corrs), int(fmt), _stream(stream))
 
@@ -139,8 +149,8 @@ def correlate2D_tc(geom, gpu_clt, colors, scale0, scale1, scale2, fat_zero, num_
 def convert_correct_tiles_tc(geom, gpu_kernel_offsets, gpu_kernels, gpu_images, gpu_tasks, gpu_clt, dstride,
                              num_tiles, lpf_mask=0, fmt=TC_FP16X2, stream=None):
     """convert_correct_tiles with the 2-D DCT-IV / DST-IV on the tensor cores."""
-    _native.call("tp_convert_correct_tiles_tc", geom.ptr, _parr(gpu_kernel_offsets), _parr(gpu_kernels),
-                 _parr(gpu_images), _dptr(gpu_tasks), _parr(gpu_clt), int(dstride), int(num_tiles),
+    _native.call("tp_convert_correct_tiles_tc", geom.ptr, _parr(gpu_kernel_offsets, stream), _parr(gpu_kernels, stream),
+                 _parr(gpu_images, stream), _dptr(gpu_tasks), _parr(gpu_clt, stream), int(dstride), int(num_tiles),
                  int(lpf_mask), int(fmt), _stream(stream))
 
 
@@ -149,11 +159,11 @@ def textures_accumulate_tc(geom, woi, gpu_clt, num_texture_tiles, gpu_texture_in
                            weight2, dust_remove, keep_weights, texture_rbg_stride, gpu_texture_rbg, texture_stride,
                            gpu_texture_tiles, gpu_tile_scratch, fmt=TC_FP16X2, stream=None):
     """textures_accumulate with the inverse CLT on the tensor cores (into gpu_tile_scratch)."""
-    _native.call("tp_textures_accumulate_tc", geom.ptr, _dptr(woi), _parr(gpu_clt), int(num_texture_tiles),
+    _native.call("tp_textures_accumulate_tc", geom.ptr, _dptr(woi), _parr(gpu_clt, stream), int(num_texture_tiles),
                  _dptr(gpu_texture_indices), _dptr(gpu_port_offsets), int(colors), int(is_lwir), float(min_shot),
                  float(scale_shot), float(diff_sigma), float(diff_threshold), float(min_agree), float(weight0),
                  float(weight1), float(weight2), int(dust_remove), int(keep_weights), int(texture_rbg_stride),
-                 _dptr(gpu_texture_rbg), int(texture_stride), _dptr(gpu_texture_tiles), _parr(gpu_tile_scratch),
+                 _dptr(gpu_texture_rbg), int(texture_stride), _dptr(gpu_texture_tiles), _parr(gpu_tile_scratch, stream),
                  int(fmt), _stream(stream))
 
 
@@ -163,11 +173,11 @@ def generate_RBGA_tc(geom, gpu_tasks, num_tiles, gpu_texture_indices, num_textur
                      gpu_texture_tiles, gpu_tile_scratch, fmt=TC_FP16X2, stream=None):
     """generate_RBGA with the inverse CLT on the tensor cores (into gpu_tile_scratch)."""
     _native.call("tp_generate_RBGA_tc", geom.ptr, _dptr(gpu_tasks), int(num_tiles), _dptr(gpu_texture_indices),
-                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt),
+                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt, stream),
                  _dptr(gpu_port_offsets), int(colors), int(is_lwir), float(min_shot), float(scale_shot),
                  float(diff_sigma), float(diff_threshold), float(min_agree), float(weight0), float(weight1),
                  float(weight2), int(dust_remove), int(keep_weights), int(texture_rbga_stride),
-                 _dptr(gpu_texture_tiles), _parr(gpu_tile_scratch), int(fmt), _stream(stream))
+                 _dptr(gpu_texture_tiles), _parr(gpu_tile_scratch, stream), int(fmt), _stream(stream))
 
 
 def tc_status(clear=True):
@@ -191,7 +201,7 @@ def textures_accumulate(geom, woi, gpu_clt, num_texture_tiles, gpu_texture_indic
                         weight2, dust_remove, keep_weights, texture_rbg_stride, gpu_texture_rbg, texture_stride,
                         gpu_texture_tiles, stream=None):
     """Texture tiles and/or overlapped RGBA accumulation (textures_accumulate)."""
-    _native.call("tp_textures_accumulate", geom.ptr, _dptr(woi), _parr(gpu_clt), int(num_texture_tiles),
+    _native.call("tp_textures_accumulate", geom.ptr, _dptr(woi), _parr(gpu_clt, stream), int(num_texture_tiles),
                  _dptr(gpu_texture_indices), _dptr(gpu_port_offsets), int(colors), int(is_lwir),
                  float(min_shot), float(scale_shot), float(diff_sigma), float(diff_threshold), float(min_agree),
                  float(weight0), float(weight1), float(weight2), int(dust_remove), int(keep_weights),
@@ -230,7 +240,7 @@ def generate_RBGA(geom, gpu_tasks, num_tiles, gpu_texture_indices, num_texture_t
                   gpu_texture_tiles, stream=None):
     """List + clear + one overlap-add pass per tile parity into the RGBA image (generate_RBGA)."""
     _native.call("tp_generate_RBGA", geom.ptr, _dptr(gpu_tasks), int(num_tiles), _dptr(gpu_texture_indices),
-                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt),
+                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt, stream),
                  _dptr(gpu_port_offsets), int(colors), int(is_lwir), float(min_shot), float(scale_shot),
                  float(diff_sigma), float(diff_threshold), float(min_agree), float(weight0), float(weight1),
                  float(weight2), int(dust_remove), int(keep_weights), int(texture_rbga_stride),
@@ -245,7 +255,7 @@ def generate_RBGA_rows(geom, gpu_tasks, num_tiles, gpu_texture_indices, num_text
     listed and accumulated (pass the band's tasks plus one tile row above and
     below; sharding.band_tasks)."""
     _native.call("tp_generate_RBGA_rows", geom.ptr, _dptr(gpu_tasks), int(num_tiles), _dptr(gpu_texture_indices),
-                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt),
+                 _dptr(num_texture_tiles), _dptr(woi), int(width), int(height), _parr(gpu_clt, stream),
                  _dptr(gpu_port_offsets), int(colors), float(min_shot), float(scale_shot), float(diff_sigma),
                  float(weight0), float(weight1), float(weight2), int(dust_remove), int(texture_rbga_stride),
                  _dptr(gpu_texture_tiles), int(row_first), int(row_last), _stream(stream))
@@ -259,7 +269,7 @@ def generate_RBGA_noalloc(geom, gpu_tasks, num_tiles, width, height, gpu_clt, gp
     caller).  The first call on a device does the set-up; calls that overlap
     on the GPU race."""
     _native.call("tp_generate_RBGA_noalloc", geom.ptr, _dptr(gpu_tasks), int(num_tiles), int(width), int(height),
-                 _parr(gpu_clt), _dptr(gpu_port_offsets), int(colors), int(is_lwir), float(min_shot),
+                 _parr(gpu_clt, stream), _dptr(gpu_port_offsets), int(colors), int(is_lwir), float(min_shot),
                  float(scale_shot), float(diff_sigma), float(diff_threshold), float(min_agree), float(weight0),
                  float(weight1), float(weight2), int(dust_remove), int(keep_weights), int(texture_rbga_stride),
                  _dptr(gpu_texture_tiles), _stream(stream))
@@ -311,11 +321,12 @@ def process_frame(geom, gpu_kernel_offsets, gpu_kernels, gpu_images, dstride, gp
     """One frame through the whole hot path (forward CLT, all pair
     correlations, overlapped RGBA texture).  gpu_corrs:
     [num_tiles][6][corr_stride]."""
-    clt = _parr(gpu_clt) if gpu_clt is not None else None
+    clt = _parr(gpu_clt, stream) if gpu_clt is not None else None
     handle = _stream(stream)
     ws = _frame_workspace(geom, gpu_tasks, int(num_tiles), handle) if clt is None else None
-    _native.call("tp_process_frame_ws", geom.ptr, _parr(gpu_kernel_offsets), _parr(gpu_kernels), _parr(gpu_images),
-                 int(dstride), _dptr(gpu_tasks), int(num_tiles), int(lpf_mask), int(corr_colors), float(scale0),
+    _native.call("tp_process_frame_ws", geom.ptr, _parr(gpu_kernel_offsets, stream), _parr(gpu_kernels, stream),
+                 _parr(gpu_images, stream), int(dstride), _dptr(gpu_tasks), int(num_tiles), int(lpf_mask),
+                 int(corr_colors), float(scale0),
                  float(scale1), float(scale2), float(fat_zero), int(corr_radius), int(corr_stride), _dptr(gpu_corrs),
                  _dptr(gpu_port_offsets), float(min_shot), float(scale_shot), float(diff_sigma), float(weight0),
                  float(weight1), float(weight2), int(dust_remove), _dptr(gpu_texture_indices),
