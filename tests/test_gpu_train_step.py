@@ -158,6 +158,33 @@ def test_step_memory_by_form(native):
         assert float((net.g[k] - got[k]).abs().max() / got[k].abs().max()) < 1e-4, k
 
 
+@pytest.mark.parametrize("tc", [True, False])
+@pytest.mark.parametrize("raw", [False, True])
+def test_step_on_a_given_stream(native, tc, raw):
+    """The loss is that of the step, which waits behind other work on the stream
+    it was given (a torch stream or its handle)."""
+    import torch
+    from tile_processor_gpu_b200 import disparity_net as D
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn((100, D.N_IN), generator=gen, device="cuda")
+    t = torch.randn(100, generator=gen, device="cuda")
+    net = D.DisparityMLP(D.init_params(4), tc=tc)
+    net.forward(x, 100)
+    want = net.loss_backward(x, 100, t)
+    torch.cuda.synchronize()
+    for v in (net._ws["loss"], net._ws.get("loss_sum")):
+        if v is not None:
+            v.fill_(-1.0)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)
+    s = side.cuda_stream if raw else side
+    net.forward(x, 100, stream=s)
+    assert abs(net.loss_backward(x, 100, t, stream=s) - want) <= 1e-6 * abs(want)
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("rows", [115200, 131072])
 def test_column_sums_of_long_batches(native, rows):
     """Batches on both sides of the rule that lays the parts of b1's gradient

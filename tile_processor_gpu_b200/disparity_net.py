@@ -70,6 +70,12 @@ def _pointers(tensors):
     return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
+def _on(stream):
+    """torch's current stream set to `stream` (a torch stream, a raw handle, None: as it is) for reading results"""
+    torch = _t()
+    return torch.cuda.stream(torch.cuda.ExternalStream(stream) if isinstance(stream, int) else stream)
+
+
 def features(geom, corrs, corr_stride, corr_radius, num_corr, corr_indices, out, feature_stride=N_IN,
              stream=None):
     """Rows out[tile] of the tiles with correlation entries (others untouched)."""
@@ -144,7 +150,8 @@ class DisparityMLP:
                          _dptr(target), _dptr(weight), 1.0 / max(count, 1.0), _dptr(w["dout"]), _dptr(w["loss"]),
                          _dptr(w["loss_sum"]), _dptr(w["dz2"]), _dptr(w["dz1"]),
                          _pointers([g[k] for k in PARAMS]), _dptr(self._err), _stream(stream))
-            return float(w["loss_sum"].item()) / max(count, 1.0)
+            with _on(stream):
+                return float(w["loss_sum"].item()) / max(count, 1.0)
         # the gradients of h2 and h1, which the tensor-core step does not form
         for k, z in (("dh2", "z2"), ("dh1", "z1")):
             if k not in w:
@@ -173,7 +180,8 @@ class DisparityMLP:
         gemm(x, w["dz1"], g["W1"], N_IN, N_H1, rows, ta=1, lda=ldx,
              stream=stream, tc=self.tc, err=self._err)
         _native.call("tp_mlp_colsum", int(rows), N_H1, N_H1, _dptr(w["dz1"]), 1.0, _dptr(g["b1"]), _stream(stream))
-        return float(w["loss"][:rows].sum().item()) / max(count, 1.0)
+        with _on(stream):
+            return float(w["loss"][:rows].sum().item()) / max(count, 1.0)
 
     def check(self):
         """Raise if a tensor-core GEMM of this network reported a wait that ran
